@@ -184,8 +184,8 @@ def warmup_alignment(warmup, S):
 
 def launches_for(k, since_sort, S, per_step, nspecies=1, per_sort=6):
     """Our kernels launched by k steps: per_step per step (single handle on a
-    power-of-two grid: push, the three spectral-solve kernels, one
-    diagnostics fold; ensemble: push, convert, k-space, two folds); per sort
+    power-of-two grid: push and the three spectral-solve kernels; ensemble of
+    such grids: push and three solve kernels per grid size); per sort
     and species histogram, 3 scan kernels, the scatter and the anchor kernel.
     Returns (count, sorts, since_sort)."""
     sorts, after = schedule(k, since_sort, S)
@@ -523,7 +523,8 @@ def bench_ensemble(args):
     ens_value = R.whole_job_rate(total_all * steps, ms / 1000.0)
     nb1 = -(-sum(int(g) * int(g) + 1 for g in grids) // 4096)
     per_sort = 6 if nb1 <= 4096 else 8  # two-level scan above 4096 block sums
-    ens_launches, ens_sorts, _ = launches_for(steps, S, S, 5, per_sort=per_sort)
+    ens_launches, ens_sorts, _ = launches_for(steps, S, S, 1 + 3 * len(set(int(g) for g in grids)),
+                                              per_sort=per_sort)
     plain_ms = m["plain_ms"]
     plain_value = R.whole_job_rate(total_all * steps, plain_ms / 1000.0) if plain_ms else None
     adj = ensemble_adjoint_rate(P, R, cfgs, specs, total_all, args.adjoint_steps, args.every, pg) \
@@ -890,8 +891,8 @@ def main():
         if args.nx == NX:
             fp64 = fp64_check(P, cfg, spec, -A / N, A / N, 10)
 
-    _, _, since_after_warmup = launches_for(args.warmup + align, 0, SORT_EVERY, 5)
-    launches, sorts_timed, _ = launches_for(args.steps, since_after_warmup, SORT_EVERY, 5)
+    _, _, since_after_warmup = launches_for(args.warmup + align, 0, SORT_EVERY, 4)
+    launches, sorts_timed, _ = launches_for(args.steps, since_after_warmup, SORT_EVERY, 4)
     if rank == 0:
         out = {
             "metric": METRIC, "value": value, "unit": "particle-steps/s", "n_gpus": world,

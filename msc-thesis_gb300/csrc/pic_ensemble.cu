@@ -44,6 +44,8 @@ ens_push_kernel(PushArgs A, const SegBlock *__restrict__ blk, const EnsRun *__re
     extern __shared__ __align__(16) unsigned char smem[];
     const SegBlock b = blk[blockIdx.x];
     const EnsRun &R = runs[b.run];
+    pdl_wait();
+    pdl_trigger();
     PushGeo G;
     G.ex = A.geo.ex + 2 * R.goff;
     G.ey = G.ex + R.ncp;
@@ -189,7 +191,9 @@ __global__ void ens_advance_kernel(DevState *devs, double *hist, int cap, int ki
                                    const EnsRun *__restrict__ runs)
 {
     const int r = blockIdx.x;
-    advance_state(devs + r, hist + (size_t)r * 6 * cap, cap, kind, runs[r].fe_scale);
+    pdl_wait();
+    pdl_trigger();
+    advance_state(devs + r, hist + (size_t)r * 6 * cap, cap, kind, runs[r].fe_scale, 32);
 }
 
 }  // namespace pic
@@ -452,20 +456,15 @@ pic_status ens_launch_push(pic_ensemble *E, int src, int kind)
     const PushArgs A = ens_push_args(E, src);
     dim3 grid((unsigned)E->npush), block(256);
     const size_t sm = E->push_smem;
-    cudaStream_t st = E->stream;
-    PIC_TRY(allow_dynamic_smem((const void *)ens_push_kernel<true, true>, sm));
-    PIC_TRY(allow_dynamic_smem((const void *)ens_push_kernel<true, false>, sm));
-    PIC_TRY(allow_dynamic_smem((const void *)ens_push_kernel<false, true>, sm));
-    if (kind == 0)
-        ens_push_kernel<true, true><<<grid, block, sm, st>>>(A, E->push_blk, E->d_runs, E->anchor, 1.f, 1.f);
-    else if (kind == 1)
-        ens_push_kernel<true, false><<<grid, block, sm, st>>>(A, E->push_blk, E->d_runs, E->anchor, -0.5f, 0.f);
-    else if (kind == 2)
-        ens_push_kernel<false, true><<<grid, block, sm, st>>>(A, E->push_blk, E->d_runs, E->anchor, 0.f, 0.f);
-    else
-        ens_push_kernel<false, true><<<grid, block, sm, st>>>(A, E->push_blk, E->d_runs, E->anchor, 0.f, -1.f);
-    PIC_CUDA(cudaGetLastError());
-    return PIC_OK;
+    // kick and drift coefficients by kind
+    static const float KICK[4] = {1.f, -0.5f, 0.f, 0.f}, DRIFT[4] = {1.f, 0.f, 0.f, -1.f};
+    const void *k = kind == 0   ? (const void *)ens_push_kernel<true, true>
+                    : kind == 1 ? (const void *)ens_push_kernel<true, false>
+                                : (const void *)ens_push_kernel<false, true>;
+    float kick = KICK[kind], drift = DRIFT[kind];
+    PIC_TRY(allow_dynamic_smem(k, sm));
+    void *args[] = {(void *)&A, &E->push_blk, &E->d_runs, &E->anchor, &kick, &drift};
+    return launch_dependent(k, grid, block, sm, E->stream, args);
 }
 
 pic_status ens_advance(pic_ensemble *E, int kind)
@@ -476,15 +475,15 @@ pic_status ens_advance(pic_ensemble *E, int kind)
     return PIC_OK;
 }
 
-pic_status ens_poisson(pic_ensemble *E)
+pic_status ens_poisson(pic_ensemble *E, int adv)
 {
     cudaStream_t st = E->stream;
     if (E->spectral) {
         for (auto &G : E->groups)
             PIC_TRY(launch_spectral_runs(E->d_runs, G.first, G.count, G.nx, G.ny, E->rho_fix,
-                                         E->rho, E->rhohat, E->ehat, E->e, G.tw, E->dev, st));
-        PIC_CUDA(cudaMemsetAsync(E->rho_fix, 0, sizeof(unsigned long long) * (size_t)E->nnodes, st));
-        return ens_advance(E, ADV_FIELD);
+                                         E->rho, E->rhohat, E->ehat, E->e, G.tw, E->dev, E->hist,
+                                         E->hist_cap, adv, st));
+        return PIC_OK;
     }
     ens_convert_kernel<<<E->nnode_blk, 256, 0, st>>>(E->rho_fix, E->rho, E->node_blk, E->d_runs, E->dev);
     PIC_CUDA(cudaGetLastError());
@@ -499,7 +498,7 @@ pic_status ens_poisson(pic_ensemble *E)
         const EnsRun &R = E->runs[G.first];
         PIC_CUFFT(cufftExecC2R(G.c2r, (cufftComplex *)(E->ehat + R.khoff), E->e + 2 * R.goff));
     }
-    return ens_advance(E, ADV_FIELD);
+    return ens_advance(E, adv);
 }
 
 SortArgs ens_sort_args(pic_ensemble *E, const float *const *xin, float *const *xout)
@@ -563,8 +562,7 @@ pic_status ens_sort(pic_ensemble *E, const float *const *xin, float *const *xout
 pic_status ens_step_body(pic_ensemble *E, int src)
 {
     PIC_TRY(ens_launch_push(E, src, 0));
-    PIC_TRY(ens_advance(E, ADV_PUSH));
-    return ens_poisson(E);
+    return ens_poisson(E, ADV_PUSH | ADV_FIELD);
 }
 
 template <class F> pic_status ens_capture(pic_ensemble *E, cudaGraphExec_t *out, F &&body)

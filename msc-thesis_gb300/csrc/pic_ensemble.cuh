@@ -104,7 +104,8 @@ template <class T> pic_status ens_alloc(T **p, size_t n)
 // (x -= dt v) and deposit
 pic_status ens_launch_push(pic_ensemble *E, int src, int kind);
 pic_status ens_advance(pic_ensemble *E, int kind);
-pic_status ens_poisson(pic_ensemble *E);
+// solve of every run, densities cleared, diagnostics folds `adv`
+pic_status ens_poisson(pic_ensemble *E, int adv = ADV_FIELD);
 // sort every run from buffer 0 into buffer 1 (and the four extra per-particle
 // arrays xin -> xout when given), push-block anchors
 pic_status ens_sort(pic_ensemble *E, const float *const *xin = nullptr, float *const *xout = nullptr);

@@ -59,33 +59,47 @@ __device__ __forceinline__ KMode kspace_mode(float2 r, int mx, int my, int nx, i
     return K;
 }
 
-// Moves the accumulators of the finished stage into the history ring and
-// clears them; one warp, lane l folds slot l.  ADV_PUSH closes the particle
-// pass of step s (kinetic energy and momentum belong to step s) and advances
-// the step counter; ADV_FIELD records the field of the current step (after
-// the push fold when both bits are set).
-__device__ __forceinline__ void advance_state(DevState *d, double *hist, int cap, int kind,
-                                              double fe_scale)
+// Sum of an accumulator over its slots, which are cleared; threads
+// 0..lanes-1 call it (a power of two, at most 32).
+template <class T>
+__device__ __forceinline__ T fold_slots(T *acc, int lanes)
 {
-    const int l = threadIdx.x;  // 32 threads = ACC_SLOTS
-    long long s = d->step;
+    const unsigned mask = lanes >= 32 ? 0xffffffffu : (1u << lanes) - 1u;
+    T v = 0;
+    for (int l = threadIdx.x; l < ACC_SLOTS; l += lanes) {
+        v += acc[l];
+        acc[l] = 0;
+    }
+    for (int o = lanes / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
+    return v;
+}
+
+// Moves the accumulators of the finished stage into the history ring and
+// clears them; called by threads 0..lanes-1 of one block (lanes: a power of
+// two, at most 32).  ADV_PUSH closes the particle pass of step s (kinetic
+// energy and momentum belong to step s) and advances the step counter;
+// ADV_FIELD records the field of the current step (after the push fold when
+// both bits are set).
+__device__ __forceinline__ void advance_state(DevState *d, double *hist, int cap, int kind,
+                                              double fe_scale, int lanes)
+{
+    const int l = threadIdx.x;
+    const long long s = d->step;
     int k = (int)(s % cap);
     if (kind & ADV_PUSH) {
-        const double ke = warp_sum_d(d->ke[l]), px = warp_sum_d(d->px[l]), py = warp_sum_d(d->py[l]);
-        d->ke[l] = d->px[l] = d->py[l] = 0.0;
+        const double ke = fold_slots(d->ke, lanes), px = fold_slots(d->px, lanes);
+        const double py = fold_slots(d->py, lanes);
         if (l == 0) {
             hist[1 * (size_t)cap + k] = ke;
             hist[2 * (size_t)cap + k] = px;
             hist[3 * (size_t)cap + k] = py;
             d->step = s + 1;
         }
-        k = (int)(++s % cap);
+        k = (int)((s + 1) % cap);
     }
     if (kind & ADV_FIELD) {
-        const double fe = warp_sum_d(d->fe[l]);
-        const unsigned long long q = warp_sum_u64(d->q[l]);
-        d->fe[l] = 0.0;
-        d->q[l] = 0ull;
+        const double fe = fold_slots(d->fe, lanes);
+        const unsigned long long q = fold_slots(d->q, lanes);
         if (l == 0) {
             hist[0 * (size_t)cap + k] = fe * fe_scale;
             hist[4 * (size_t)cap + k] = (double)(long long)q;

@@ -257,19 +257,19 @@ static void update_mean(pic_handle *h)
 }
 
 // ---------------------------------------------------------------- stages
-// adv: the diagnostics folds to launch after the solve (ADV_FIELD, or
-// ADV_PUSH | ADV_FIELD when the particle pass left its fold to this launch)
+// adv: the diagnostics folds that ride on the solve (ADV_FIELD, or ADV_PUSH |
+// ADV_FIELD when the particle pass left its fold to it)
 pic_status record_poisson(pic_handle *h, int adv)
 {
     if (h->spectral) {
-        PIC_TRY(launch_spectral(h));
+        PIC_TRY(launch_spectral(h, adv));
     } else {
         PIC_TRY(launch_convert(h));
         PIC_CUFFT(cufftExecR2C(h->plan_r2c, h->rho, (cufftComplex *)h->rhohat));
-        PIC_TRY(launch_kspace(h, false, nullptr));
+        PIC_TRY(launch_kspace(h, false, nullptr, adv));
         PIC_CUFFT(cufftExecC2R(h->plan_c2r2, (cufftComplex *)h->ehat, h->e));
     }
-    PIC_TRY(launch_advance(h, adv));
+    h->rho_clear = true;
     return PIC_OK;
 }
 
@@ -293,14 +293,11 @@ pic_status record_push_all(pic_handle *h, int src, bool deposit, bool fold)
     return PIC_OK;
 }
 
-// One step.  Without MCC (whose pass starts from the folded counts) the
-// particle pass's fold rides on the field's: one launch fewer per step.
+// One step; the particle pass's fold rides on the field's.
 static pic_status record_step(pic_handle *h, int src)
 {
-    const bool merge = !h->mcc.on;
-    PIC_TRY(record_push_all(h, src, true, !merge));
-    PIC_TRY(record_poisson(h, merge ? (ADV_PUSH | ADV_FIELD) : ADV_FIELD));
-    return PIC_OK;
+    PIC_TRY(record_push_all(h, src, true, false));
+    return record_poisson(h, ADV_PUSH | ADV_FIELD);
 }
 
 // Sort every species; the DSMC species goes last so that the cell offsets it
@@ -356,10 +353,19 @@ static pic_status sort_now(pic_handle *h, bool import = false)
     return PIC_OK;
 }
 
+// The fixed-point density cleared for a deposit, unless the last solve left it so.
+static pic_status clear_rho(pic_handle *h)
+{
+    if (!h->rho_clear)
+        PIC_CUDA(cudaMemsetAsync(h->rho_fix, 0,
+                                 sizeof(unsigned long long) * (size_t)h->g.nx * h->g.ny, h->stream));
+    h->rho_clear = false;
+    return PIC_OK;
+}
+
 pic_status deposit_now(pic_handle *h)
 {
-    PIC_CUDA(cudaMemsetAsync(h->rho_fix, 0, sizeof(unsigned long long) * (size_t)h->g.nx * h->g.ny,
-                             h->stream));
+    PIC_TRY(clear_rho(h));
     for (int s = 0; s < h->cfg.nspecies; ++s)
         if (h->sp[s].cap) PIC_TRY(launch_deposit(h, s));
     return PIC_OK;
@@ -408,6 +414,7 @@ static pic_status build_graphs(pic_handle *h)
     if (h->graphs_valid) return PIC_OK;
     drop_graphs(h);
     const int S = h->cfg.sort_every;
+    const bool clear = h->rho_clear;  // capturing a solve runs none
     PIC_TRY(capture(h, &h->g_one, [&] { return record_step(h, 0); }));
     PIC_TRY(capture(h, &h->g_sortstep, [&] {
         PIC_TRY(record_sort_all(h));
@@ -419,6 +426,7 @@ static pic_status build_graphs(pic_handle *h)
         for (int k = 1; k < S; ++k) PIC_TRY(record_step(h, 0));
         return PIC_OK;
     }));
+    h->rho_clear = clear;
     h->graphs_valid = true;
     return PIC_OK;
 }
@@ -949,9 +957,7 @@ pic_status pic_gather_push(pic_handle *h, int deposit)
         set_error("pic_gather_push: no field yet");
         return PIC_ERR_STATE;
     }
-    if (deposit)
-        PIC_CUDA(cudaMemsetAsync(h->rho_fix, 0,
-                                 sizeof(unsigned long long) * (size_t)h->g.nx * h->g.ny, h->stream));
+    if (deposit) PIC_TRY(clear_rho(h));
     PIC_TRY(record_push_all(h, 0, deposit != 0));
     h->since_sort++;
     h->steps_host++;
@@ -987,6 +993,7 @@ pic_status pic_step(pic_handle *h, long long nsteps)
         }
     }
     h->steps_host += nsteps;
+    if (nsteps > 0) h->rho_clear = true;
     return PIC_OK;
 }
 
@@ -1107,6 +1114,7 @@ pic_status pic_get_rho_fixed(pic_handle *h, int64_t *out)
     PIC_TRY(deposit_now(h));
     PIC_CUDA(cudaMemcpyAsync(out, h->rho_fix, ncell * 8, cudaMemcpyDeviceToHost, h->stream));
     PIC_CUDA(cudaMemsetAsync(h->rho_fix, 0, ncell * 8, h->stream));
+    h->rho_clear = true;
     PIC_CUDA(cudaStreamSynchronize(h->stream));
     return PIC_OK;
 }

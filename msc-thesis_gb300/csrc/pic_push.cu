@@ -46,6 +46,8 @@ template <bool GATHER, bool DEPOSIT, bool AGG, bool MOVE = true>
 __global__ void __launch_bounds__(256, 4) push_kernel(PushArgs A)
 {
     extern __shared__ __align__(16) unsigned char smem[];
+    pdl_wait();
+    pdl_trigger();
     const long long n = *A.d_n;
     const long long base = (long long)blockIdx.x * A.chunk;
     if (base >= n) return;  // block-uniform
@@ -96,6 +98,25 @@ pic_status allow_dynamic_smem(const void *kernel, size_t bytes)
 {
     if (bytes > 48 * 1024)
         PIC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    return PIC_OK;
+}
+
+// The attribute holds for this launch alone; after work other than a kernel
+// (a copy, the start of a graph) it has no effect.
+pic_status launch_dependent(const void *kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                            void **args)
+{
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    PIC_CUDA(cudaLaunchKernelExC(&c, kernel, args));
     return PIC_OK;
 }
 
@@ -158,42 +179,19 @@ pic_status launch_push(pic_handle *h, int s, int src, bool deposit, float dt_sca
     PushArgs A = push_args(h, s, src, dt_scale);
     const bool charged = D.q != 0.0;
     const bool dep = deposit && D.q_int != 0;
-    dim3 grid((unsigned)B.nchunks), block(256);
-    if (h->cfg.push_variant == 3) {
-        // warp-summed deposit groups: measured 5% slower at 2048^2 x 32 ppc
-        // (1.144 vs 1.085 ms), so opt-in
-        const size_t sm = push_smem(g);
-        if (charged && dep) {
-            PIC_TRY(allow_dynamic_smem((const void *)push_kernel<true, true, true>, sm));
-            push_kernel<true, true, true><<<grid, block, sm, h->stream>>>(A);
-        } else if (charged) {
-            PIC_TRY(allow_dynamic_smem((const void *)push_kernel<true, false, false>, sm));
-            push_kernel<true, false, false><<<grid, block, sm, h->stream>>>(A);
-        } else if (dep) {
-            PIC_TRY(allow_dynamic_smem((const void *)push_kernel<false, true, true>, sm));
-            push_kernel<false, true, true><<<grid, block, sm, h->stream>>>(A);
-        } else {
-            PIC_TRY(allow_dynamic_smem((const void *)push_kernel<false, false, false>, sm));
-            push_kernel<false, false, false><<<grid, block, sm, h->stream>>>(A);
-        }
-    } else {
-        const size_t sm = push_smem(g);
-        if (charged && dep) {
-            PIC_TRY(allow_dynamic_smem((const void *)push_kernel<true, true, false>, sm));
-            push_kernel<true, true, false><<<grid, block, sm, h->stream>>>(A);
-        } else if (charged) {
-            PIC_TRY(allow_dynamic_smem((const void *)push_kernel<true, false, false>, sm));
-            push_kernel<true, false, false><<<grid, block, sm, h->stream>>>(A);
-        } else if (dep) {
-            PIC_TRY(allow_dynamic_smem((const void *)push_kernel<false, true, false>, sm));
-            push_kernel<false, true, false><<<grid, block, sm, h->stream>>>(A);
-        } else {
-            PIC_TRY(allow_dynamic_smem((const void *)push_kernel<false, false, false>, sm));
-            push_kernel<false, false, false><<<grid, block, sm, h->stream>>>(A);
-        }
-    }
-    PIC_CUDA(cudaGetLastError());
-    return PIC_OK;
+    // variant 3, warp-summed deposit groups: measured 5% slower at 2048^2 x 32
+    // ppc (1.144 vs 1.085 ms), so opt-in
+    const bool agg = h->cfg.push_variant == 3;
+    const void *k = charged ? (!dep  ? (const void *)push_kernel<true, false, false>
+                               : agg ? (const void *)push_kernel<true, true, true>
+                                     : (const void *)push_kernel<true, true, false>)
+                            : (!dep  ? (const void *)push_kernel<false, false, false>
+                               : agg ? (const void *)push_kernel<false, true, true>
+                                     : (const void *)push_kernel<false, true, false>);
+    const size_t sm = push_smem(g);
+    PIC_TRY(allow_dynamic_smem(k, sm));
+    void *args[] = {&A};
+    return launch_dependent(k, (unsigned)B.nchunks, 256, sm, h->stream, args);
 }
 
 // Deposit of buffer 0 where it stands: shared-memory windows at the chunk

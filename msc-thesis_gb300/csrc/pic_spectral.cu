@@ -44,7 +44,7 @@
 namespace pic {
 
 struct SpecArgs {
-    const unsigned long long *rho_fix;
+    unsigned long long *rho_fix;  // read by the forward rows, cleared by the columns
     float *rho;
     float2 *S;           // [nh][ny]: rows transformed along x
     float2 *Tx, *Ty;     // [nh][ny]: Ex~, Ey~ after the inverse along y
@@ -65,6 +65,10 @@ struct SpecArgs {
     int pairs, cols, rows;  // transforms (row pairs or rows), columns, rows per block
     int sa, sb, sc;         // buffer strides (float2) of the three kernels
     DevState *dev;
+    // diagnostics folds of the step (0: none), by one block of the inverse rows
+    double *hist;
+    int hist_cap, adv;
+    double fe_scale;
     // ensemble: blockIdx.y picks run first + blockIdx.y of this table, whose
     // grids sit at its offsets from the pointers above and whose constants
     // replace the ones above (nullptr: a single run)
@@ -92,6 +96,8 @@ __device__ __forceinline__ SpecArgs block_args(const SpecArgs &P)
         A.ky1 = R.ky1;
         A.inv_eps0_n = R.inv_eps0_n;
         A.dev = P.dev + r;
+        A.hist = P.hist + (size_t)r * 6 * P.hist_cap;
+        A.fe_scale = R.fe_scale;
     }
     return A;
 }
@@ -133,6 +139,8 @@ __global__ void __launch_bounds__(256) spec_rows_fwd_kernel(SpecArgs P)
     float2 *buf[1] = {smem + f * A.sa};
     float2 v[1][fft::E];
     unsigned long long qs = 0;
+    pdl_wait();
+    pdl_trigger();
     if (ADJ) {
         const size_t r0 = (size_t)(blockIdx.x * A.pairs + f) * NX;
 #pragma unroll
@@ -203,6 +211,15 @@ __global__ void __launch_bounds__(256, 2) spec_cols_kernel(SpecArgs P)
     const size_t col = (size_t)(on ? mx : 0) * NY;
     float fe = 0.f;
     float2 v[1][fft::E];
+    pdl_wait();
+    pdl_trigger();
+    if (!ADJ) {
+        // the density, converted by the forward rows, cleared for the next
+        // deposit (a memset of its own before; figures at pdl_wait)
+        const int n2 = (A.nx << LGY) >> 1, stride = gridDim.x * blockDim.x;
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n2; i += stride)
+            reinterpret_cast<ulonglong2 *>(A.rho_fix)[i] = make_ulonglong2(0ull, 0ull);
+    }
     // forward transform of column `src` along y, left in natural order in `bs`
     auto forward = [&](const float2 *src, float2 *bs) {
         float2 *buf[1] = {bs};
@@ -275,7 +292,10 @@ __global__ void __launch_bounds__(256, 2) spec_cols_kernel(SpecArgs P)
 }
 
 // LGX: log2 nx.  Block: `rows` transforms, nx/16 threads each: row y of Ex~
-// and Ey~ into Ex and Ey, or rows 2y and 2y + 1 of psi~ into psi.
+// and Ey~ into Ex and Ey, or rows 2y and 2y + 1 of psi~ into psi.  With
+// A.adv one block more than the rows need folds the step's diagnostics into
+// the history beside them (the push's, rows' and columns' sums are complete
+// here; a launch of its own before; figures at pdl_wait).
 template <int LGX>
 __global__ void __launch_bounds__(256) spec_rows_inv_kernel(SpecArgs P)
 {
@@ -285,6 +305,14 @@ __global__ void __launch_bounds__(256) spec_rows_inv_kernel(SpecArgs P)
     const int f = threadIdx.x / TP, t = threadIdx.x - f * TP;
     const int nr = A.rows;
     const int y0 = blockIdx.x * nr;
+    pdl_wait();
+    pdl_trigger();
+    if (A.adv && blockIdx.x == gridDim.x - 1) {
+        const int lanes = min((int)blockDim.x, 32);  // a power of two
+        if ((int)threadIdx.x < lanes)
+            advance_state(A.dev, A.hist, A.hist_cap, A.adv, A.fe_scale, lanes);
+        return;
+    }
     // (mode, row) with the row fastest: the block's rows of one mode are
     // adjacent in Tx and Ty.  nh nr = (8 + 16 / nx) times the block's
     // threads: at most 9 items per thread, all loads issued before the
@@ -384,7 +412,7 @@ pic_status spectral_twiddles(int nx, int ny, float2 **tw)
 
 // The three kernels over `batch` runs of one grid size (A.runs set) or one
 // run: the field solve, or with adj the adjoint solve (A.gx, A.gy -> psi in
-// A.ex).  The caller clears the fixed-point density afterwards.
+// A.ex).  The field solve leaves the fixed-point density cleared.
 static pic_status launch_kernels(SpecArgs &A, int batch, cudaStream_t st, bool adj = false)
 {
     const int nx = A.nx, ny = A.ny, nh = A.nh;
@@ -447,14 +475,14 @@ static pic_status launch_kernels(SpecArgs &A, int batch, cudaStream_t st, bool a
     PIC_TRY(allow_dynamic_smem(kc, mc));
     void *args[] = {&A};
     const unsigned nb = (unsigned)batch;
-    PIC_CUDA(cudaLaunchKernel(ka, dim3(na / A.pairs, nb), dim3(A.pairs * tpx), args, ma, st));
-    PIC_CUDA(cudaLaunchKernel(kb, dim3((nh + A.cols - 1) / A.cols, nb), dim3(A.cols * tpy), args,
-                              mb, st));
-    PIC_CUDA(cudaLaunchKernel(kc, dim3(nc / A.rows, nb), dim3(A.rows * tpx), args, mc, st));
-    return PIC_OK;
+    const unsigned fold = A.adv ? 1u : 0u;
+    PIC_TRY(launch_dependent(ka, dim3(na / A.pairs, nb), dim3(A.pairs * tpx), ma, st, args));
+    PIC_TRY(launch_dependent(kb, dim3((nh + A.cols - 1) / A.cols, nb), dim3(A.cols * tpy), mb, st,
+                             args));
+    return launch_dependent(kc, dim3(nc / A.rows + fold, nb), dim3(A.rows * tpx), mc, st, args);
 }
 
-pic_status launch_spectral(pic_handle *h)
+pic_status launch_spectral(pic_handle *h, int adv)
 {
     const Geometry &g = h->g;
     SpecArgs A;
@@ -478,16 +506,17 @@ pic_status launch_spectral(pic_handle *h)
     A.tmx = h->track_mx;
     A.tmy = h->track_my;
     A.dev = h->dev;
-    PIC_TRY(launch_kernels(A, 1, h->stream));
-    PIC_CUDA(cudaMemsetAsync(h->rho_fix, 0, sizeof(unsigned long long) * (size_t)g.nx * g.ny,
-                             h->stream));
-    return PIC_OK;
+    A.hist = h->hist;
+    A.hist_cap = h->hist_cap;
+    A.adv = adv;
+    A.fe_scale = 0.5 * h->cfg.eps0 * g.dx * g.dy * (double)g.nx * (double)g.ny;
+    return launch_kernels(A, 1, h->stream);
 }
 
 pic_status launch_spectral_runs(const EnsRun *runs, int first, int count, int nx, int ny,
-                                const unsigned long long *rho_fix, float *rho, float2 *rhohat,
+                                unsigned long long *rho_fix, float *rho, float2 *rhohat,
                                 float2 *ehat, float *e, const float2 *tw, DevState *devs,
-                                cudaStream_t st)
+                                double *hist, int hist_cap, int adv, cudaStream_t st)
 {
     SpecArgs A;
     memset(&A, 0, sizeof A);
@@ -502,6 +531,9 @@ pic_status launch_spectral_runs(const EnsRun *runs, int first, int count, int nx
     A.twx = tw;
     A.tmx = A.tmy = -1;
     A.dev = devs;
+    A.hist = hist;
+    A.hist_cap = hist_cap;
+    A.adv = adv;
     A.runs = runs;
     // a grid's y dimension holds at most 65535 runs
     for (int b = 0; b < count; b += 65535) {
