@@ -121,7 +121,8 @@ typedef struct pic_config {
     int sort_every;      /* steps between counting sorts (0: 20)              */
     int tile_w, tile_h;  /* sort tile in cells (0: chosen from the density)   */
     int chunk;           /* particles per push block, multiple of 4, at most
-                            32768 (0: 8192)                                   */
+                            32768 (0: chosen from the particle count, 1024
+                            to 13824)                                         */
     int halo;            /* shared-memory window halo in cells (0: 4, or less
                             where the window would exceed 56 KB; windows over
                             112 KB are refused)                               */

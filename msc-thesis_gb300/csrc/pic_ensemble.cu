@@ -254,6 +254,20 @@ void add_blocks(std::vector<SegBlock> &v, int run, long long start, long long le
         v.push_back(SegBlock{start + b, (int)std::min(per, len - b), run});
 }
 
+// sort tiles of about `chunk` particles and the push window over two of them
+void ens_tiles(EnsRun &R, const pic_config &c, int chunk, int halo)
+{
+    const double ppc = std::max(1.0, (double)c.species[0].capacity / ((double)c.nx * c.ny));
+    const int tcells = std::max(1, (int)std::lround(chunk / ppc));
+    R.tw = pick_divisor(c.nx, std::min(16, tcells));
+    R.th = pick_tile_h(c.ny, tcells, R.tw);
+    R.ntx = c.nx / R.tw;
+    R.nty = c.ny / R.th;
+    R.hx = R.hy = halo;
+    R.wcx = 2 * R.tw + 2 * R.hx;
+    R.wcy = R.th + 2 * R.hy;
+}
+
 pic_status ens_layout(pic_ensemble *E)
 {
     const int nr = E->nruns;
@@ -281,16 +295,10 @@ pic_status ens_layout(pic_ensemble *E)
         R.dx = c.Lx / c.nx;
         R.dy = c.Ly / c.ny;
         const long long ncell = (long long)c.nx * c.ny;
-        const double ppc = std::max(1.0, (double)D.capacity / (double)ncell);
-        const int tcells = std::max(1, (int)std::lround(E->chunk / ppc));
-        R.tw = pick_divisor(c.nx, std::min(16, tcells));
-        R.th = pick_tile_h(c.ny, tcells, R.tw);
-        R.ntx = c.nx / R.tw;
-        R.nty = c.ny / R.th;
-        R.hx = R.hy = E->halo;
-        R.wcx = 2 * R.tw + 2 * R.hx;
-        R.wcy = R.th + 2 * R.hy;
+        // a default chunk refuses what 8192 would (its tiles are never larger)
+        ens_tiles(R, c, E->cfg[0].chunk ? E->chunk : 8192, E->halo);
         if (window_smem(R) > WINDOW_SMEM_MAX) return ens_bad("shared-memory window too large for a run");
+        ens_tiles(R, c, E->chunk, E->halo);
         R.cap4 = (D.capacity + 3) & ~3ll;
         R.poff = poff;
         R.ncp = (ncell + 3) & ~3ll;
@@ -651,7 +659,13 @@ pic_status pic_ensemble_create(const pic_config *runs, int nruns, pic_ensemble *
     E->device = c0.device;
     E->nruns = nruns;
     E->cfg.assign(runs, runs + nruns);
-    E->chunk = c0.chunk ? c0.chunk : 8192;
+    E->chunk = c0.chunk;
+    if (!E->chunk) {  // one wave of blocks for small ensembles, at most 8192
+        long long total = 0;
+        for (int r = 0; r < nruns; ++r) total += runs[r].species[0].capacity;
+        const long long per = total / (4 * device_sms());
+        E->chunk = (int)std::max(1024ll, std::min(8192ll, (per + 3) & ~3ll));
+    }
     E->halo = c0.halo ? c0.halo : 2;
     E->sort_every = c0.sort_every ? c0.sort_every : 20;
     E->hist_cap = c0.history ? c0.history : 4096;

@@ -188,6 +188,32 @@ static pic_status validate(const pic_config *c, pic_handle *h)
     return PIC_OK;
 }
 
+// Particles per push block for n particles at ppc per cell where the caller
+// leaves it open.  Blocks of one size fill whole waves of the resident
+// blocks (four per SM): as few waves as keep a block at most 13824 particles
+// (its window stays small against them) and at most `limit` (about one and
+// a third of the particles of its tile, so that a block rarely reaches a
+// third tile), and at least 1024 (one pass of its threads).  us per step with
+// 8192 for all sizes before: 64^2 x 16 per cell 42.0 -> 21.9, 128^2 x 32 41.5
+// -> 26.3, 250 x 180 x 23 49.9 -> 36.3, 128^2 x 100 45.3 -> 35.2, 256^2 x 32
+// 53.2 -> 40.5, 512^2 x 32 109 -> 100, 1024^2 x 32 317 -> 308.
+static int push_chunk(long long n, double limit)
+{
+    const double per = std::ceil((double)std::max(1ll, n) / (4.0 * device_sms()));
+    const double waves = std::ceil(per / std::min(13824.0, std::max(1024.0, limit)));
+    return std::max(1024, ((int)std::ceil(per / waves) + 3) & ~3);
+}
+
+// Particles per push block of a species holding n.
+static void set_chunk(pic_handle *h, int s, long long n)
+{
+    const Geometry &g = h->g;
+    SpeciesBuf &B = h->sp[s];
+    const double tile = (double)g.tw * g.th * (double)n / ((double)g.nx * g.ny);
+    B.chunk = h->cfg.chunk ? h->cfg.chunk : push_chunk(n, 1.35 * tile);
+    B.nchunks = (B.cap + B.chunk - 1) / B.chunk;
+}
+
 static pic_status setup_geometry(pic_handle *h)
 {
     const pic_config &c = h->cfg;
@@ -199,35 +225,46 @@ static pic_status setup_geometry(pic_handle *h)
     g.Ly = c.Ly;
     g.dx = c.Lx / c.nx;
     g.dy = c.Ly / c.ny;
-    g.chunk = c.chunk ? c.chunk : 8192;
     // default halo: the particles' drift between sorts grows with the cadence
     // (2048^2 x 32 ppc, sort every 40: 1.203 ms per step with 4 cells against
     // 1.234 with 2, 1.216 with 3, 1.211 with 5 or 6, 1.300 with 8; sort every
     // 20: 1.100 ms with 3 against 1.106 with 4), less where the window would
     // not fit
     const int every = c.sort_every ? c.sort_every : 20;
-    g.halo = c.halo ? c.halo : (every <= 20 ? 3 : 4);
     long long maxcap = 0;
     for (int s = 0; s < c.nspecies; ++s) maxcap = std::max(maxcap, c.species[s].capacity);
     const double ppc = std::max(1.0, (double)maxcap / ((double)c.nx * c.ny));
-    const int tcells = std::max(1, (int)std::lround(g.chunk / ppc));
-    g.tw = c.tile_w ? c.tile_w : pick_divisor(c.nx, std::min(16, tcells));
-    g.th = c.tile_h ? c.tile_h : pick_tile_h(c.ny, tcells, g.tw);
-    g.ntx = c.nx / g.tw;
-    g.nty = c.ny / g.th;
-    auto window = [&] {
-        g.wcx = 2 * g.tw + 2 * g.halo;
-        g.wcy = g.th + 2 * g.halo;
-        return window_bytes(g.wcx, g.wcy) + 32;
+    // tiles of about one chunk of particles and their window, whose bytes it returns
+    auto lay = [&](int chunk) {
+        const int tcells = std::max(1, (int)std::lround(chunk / ppc));
+        g.halo = c.halo ? c.halo : (every <= 20 ? 3 : 4);
+        g.tw = c.tile_w ? c.tile_w : pick_divisor(c.nx, std::min(16, tcells));
+        g.th = c.tile_h ? c.tile_h : pick_tile_h(c.ny, tcells, g.tw);
+        g.ntx = c.nx / g.tw;
+        g.nty = c.ny / g.th;
+        auto window = [&] {
+            g.wcx = 2 * g.tw + 2 * g.halo;
+            g.wcy = g.th + 2 * g.halo;
+            return window_bytes(g.wcx, g.wcy) + 32;
+        };
+        size_t smem = window();
+        while (!c.halo && smem > WINDOW_SMEM_TARGET && g.halo > 1) {
+            --g.halo;
+            smem = window();
+        }
+        return smem;
     };
-    size_t smem = window();
-    while (!c.halo && smem > WINDOW_SMEM_TARGET && g.halo > 1) {
-        --g.halo;
-        smem = window();
-    }
-    if (smem > WINDOW_SMEM_MAX) {
+    if (lay(c.chunk ? c.chunk : 8192) > WINDOW_SMEM_MAX) {
         set_error("pic_create: shared-memory window too large; use smaller tiles or halo");
         return PIC_ERR_INVALID_ARG;
+    }
+    if (!c.chunk) {
+        // the chunk that fills the GPU, with a tile of at most 512 cells (16 x
+        // 32: its window fits four blocks per SM), unless its divisors of nx
+        // and ny make a worse window than 8192's
+        const Geometry base = g;
+        const size_t smem = lay(push_chunk(maxcap, 690.0 * ppc));
+        if (smem > WINDOW_SMEM_TARGET || g.halo < base.halo) g = base;
     }
     return PIC_OK;
 }
@@ -500,6 +537,9 @@ static pic_status set_count(pic_handle *h, int s, long long n)
     SpeciesBuf &B = h->sp[s];
     const long long old4 = (B.n + 3) & ~3ll;
     B.n = n;
+    const int chunk = B.chunk;
+    set_chunk(h, s, n);
+    if (B.chunk != chunk) drop_graphs(h);  // the push grid is baked into them
     const long long n4 = (n + 3) & ~3ll;
     PIC_CUDA(cudaMemcpyAsync(&h->dev->n[s], &B.n, sizeof(long long), cudaMemcpyHostToDevice,
                              h->stream));
@@ -668,9 +708,11 @@ pic_status pic_create(const pic_config *cfg, pic_handle **out)
             H_CUDA(cudaMemsetAsync(B.pid[b], 0, n * 4, h->stream));
             if (B.vz[b]) H_CUDA(cudaMemsetAsync(B.vz[b], 0, n * 4, h->stream));
         }
-        B.nchunks = (B.cap + g.chunk - 1) / g.chunk;
-        H_TRY(dalloc(&B.anchor, (size_t)B.nchunks));
-        H_CUDA(cudaMemsetAsync(B.anchor, 0xFF, (size_t)B.nchunks * 4, h->stream));
+        set_chunk(h, sp, B.cap);
+        // room for the smallest chunk a load can choose
+        const size_t na = (size_t)((B.cap + 1023) / std::min(B.chunk, 1024)) + 1;
+        H_TRY(dalloc(&B.anchor, na));
+        H_CUDA(cudaMemsetAsync(B.anchor, 0xFF, na * 4, h->stream));
     }
     H_TRY(dalloc(&h->rho_fix, ncell));
     H_TRY(dalloc(&h->rho, ncell));

@@ -134,6 +134,7 @@ struct SpeciesBuf {
     int32_t *anchor = nullptr;  // per push chunk: tile (tx | ty << 16) or -1
     long long cap = 0;          // allocated slots (multiple of 4)
     long long n = 0;            // host mirror of the count
+    int chunk = 0;              // particles per push block (push_chunk)
     long long nchunks = 0;      // push grid size for this species
     bool records_ready = false; // import keys and records already in the stage
     bool presorted = false;     // imported already sorted, range by range
@@ -195,7 +196,7 @@ struct Geometry {
     int nx, ny, nh;           // nh = nx/2 + 1 (half spectrum along x)
     double Lx, Ly, dx, dy;
     int tw, th, ntx, nty;     // sort tiles
-    int halo, chunk;
+    int halo;
     int wcx, wcy;             // cell window of a push block: (2 tw + 2 halo) x (th + 2 halo)
 };
 

@@ -154,7 +154,7 @@ static PushArgs push_args(pic_handle *h, int s, int src, float dt_scale)
     A.geo.hy = g.halo;
     A.geo.wcx = g.wcx;
     A.geo.wcy = g.wcy;
-    A.chunk = g.chunk;
+    A.chunk = B.chunk;
     const double dt = h->cfg.dt * dt_scale;
     const bool move = dt_scale > 0.0f;
     A.geo.qm_dt = (float)(D.q / D.m * dt);

@@ -240,7 +240,7 @@ pic_status launch_anchors(pic_handle *h, int s, int buf)
     A.tw = g.tw;
     A.th = g.th;
     A.ntx = g.ntx;
-    A.chunk = g.chunk;
+    A.chunk = B.chunk;
     PIC_CUDA(cudaMemsetAsync(B.anchor, 0xFF, sizeof(int32_t) * (size_t)B.nchunks, h->stream));
     sort_anchor_kernel<<<(unsigned)((B.nchunks + 255) / 256), 256, 0, h->stream>>>(A, B.nchunks);
     PIC_CUDA(cudaGetLastError());
@@ -296,7 +296,7 @@ static SortArgs sort_args(pic_handle *h, int s, int from = 0)
     A.tw = g.tw;
     A.th = g.th;
     A.ntx = g.ntx;
-    A.chunk = g.chunk;
+    A.chunk = B.chunk;
     A.err = &h->dev->err;
     A.nkeys = ncell + 1;  // cells + the bin of empty slots
     A.nslots = B.cap;
