@@ -29,7 +29,7 @@ __global__ void import_keys_kernel(const int32_t *__restrict__ cell, long long n
 {
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        keys[i] = (uint32_t)particle_key(G, err, cell[i]);
+        keys[i] = import_key(G, err, cell[i]);
         idx[i] = (uint32_t)i;
     }
 }
@@ -42,7 +42,7 @@ __global__ void import_keys_ens_kernel(const int32_t *__restrict__ cell,
 {
     const SegBlock b = blk[blockIdx.x];
     const EnsRun &R = runs[b.run];
-    const KeyGeo G = key_geo(R.nx, R.ny, R.tw, R.th, R.ntx, R.key_off);
+    const KeyGeo G = key_geo(R.nx, R.ny, R.tw, R.th, R.ntx, R.key_off, 1);
     for (long long i = b.base + threadIdx.x; i < b.base + b.count; i += blockDim.x) {
         keys[i] = (uint32_t)particle_key(G, err, cell[i]);
         idx[i] = (uint32_t)i;
@@ -78,7 +78,7 @@ __global__ void import_pack_kernel(Fields F, long long n, KeyGeo G, unsigned *er
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         const uint32_t c = F.in[0][i];
-        keys[i] = (uint32_t)particle_key(G, err, (int)c);
+        keys[i] = import_key(G, err, (int)c);
         idx[i] = (uint32_t)i;
         rec[2 * i] = make_uint4(c, F.in[1][i], F.in[2][i], F.in[3][i]);
         rec[2 * i + 1] = make_uint4(F.in[4][i], F.in[5][i], F.nf > 6 ? F.in[6][i] : 0u, 0u);
@@ -160,14 +160,13 @@ pic_status import_sort(pic_handle *h, int s, bool *in_buffer0)
         set_error("import sort: more than 2^31 slots");
         return PIC_ERR_INVALID_ARG;
     }
-    const Geometry &g = h->g;
     const bool ready = B.records_ready;  // keys, slots and records written by the conversion
     B.records_ready = false;
     const bool packed = ready || stage_fits(h, (size_t)n * 48);
     if (!ready) PIC_TRY(ensure_stage(h, (size_t)n * (packed ? 48 : 16)));
     uint32_t *scratch = (uint32_t *)h->stage;
     uint4 *rec = reinterpret_cast<uint4 *>(scratch + 4 * n);
-    const KeyGeo G = key_geo(g.nx, g.ny, g.tw, g.th, g.ntx, 0);
+    const KeyGeo G = import_geo(h, s);
     Fields F;
     memset(&F, 0, sizeof F);
     const void *in[7] = {B.cell[0], B.ox[0], B.oy[0], B.vx[0], B.vy[0], B.pid[0], B.vz[0]};
@@ -188,7 +187,7 @@ pic_status import_sort(pic_handle *h, int s, bool *in_buffer0)
     }
     PIC_CUDA(cudaGetLastError());
     const uint32_t *idx = nullptr;
-    PIC_TRY(radix_pairs(scratch, n, key_bits((long long)g.nx * g.ny + 1), &h->cub_temp,
+    PIC_TRY(radix_pairs(scratch, n, key_bits(import_keys(G)), &h->cub_temp,
                         &h->cub_temp_bytes, h->stream, &idx));
     if (packed)
         import_unpack_kernel<<<grid_for(n, 256), 256, 0, h->stream>>>(F, rec, idx, n);
@@ -227,8 +226,7 @@ pic_status import_records_in_parts(pic_handle *h, int s, long long n, const doub
         return PIC_ERR_INVALID_ARG;
     }
     PIC_TRY(ensure_copy_stream(h));
-    const Geometry &g = h->g;
-    const int bits = key_bits((long long)g.nx * g.ny + 1);
+    const int bits = key_bits(import_keys(import_geo(h, s)));
     uint32_t *scratch = (uint32_t *)h->stage;
     const uint4 *rec = reinterpret_cast<const uint4 *>(scratch + 4 * cap);
     long long bnd[IMPORT_PARTS + 1];

@@ -146,13 +146,13 @@ __global__ void from_global_records_kernel(InitArgs A, KeyGeo G, long long lo, l
             locate(x[i], A.Lx, A.inv_dx, A.nx, cx, ox);
             locate(y[i], A.Ly, A.inv_dy, A.ny, cy, oy);
             const int c = cx | (cy << 16);
-            keys[i] = (uint32_t)particle_key(G, err, c);
+            keys[i] = import_key(G, err, c);
             rec[2 * i] = make_uint4((uint32_t)c, __float_as_uint(ox), __float_as_uint(oy),
                                     __float_as_uint((float)vx[i]));
             rec[2 * i + 1] = make_uint4(__float_as_uint((float)vy[i]), (uint32_t)i,
                                         vz ? __float_as_uint((float)vz[i]) : 0u, 0u);
         } else {
-            keys[i] = (uint32_t)particle_key(G, err, -1);
+            keys[i] = import_key(G, err, -1);
             rec[2 * i] = make_uint4(0xFFFFFFFFu, 0u, 0u, 0u);
             rec[2 * i + 1] = make_uint4(0u, 0xFFFFFFFFu, 0u, 0u);
         }
@@ -443,8 +443,7 @@ pic_status launch_from_global_records_range(pic_handle *h, int s, long long n, l
     if (!cap || hi <= lo) return PIC_OK;
     InitArgs A = base_args(h, s);
     A.n = n;
-    const Geometry &g = h->g;
-    const KeyGeo G = key_geo(g.nx, g.ny, g.tw, g.th, g.ntx, 0);
+    const KeyGeo G = import_geo(h, s);
     uint32_t *scratch = (uint32_t *)h->stage;
     int grid = grid_for(hi - lo, 256);
     if (max_blocks > 0) grid = std::min(grid, max_blocks);

@@ -92,6 +92,8 @@ __device__ __forceinline__ int sort_key(int c, const KeyGeo &G)
     return G.rows ? row : row * G.tw + (cx - tx * G.tw);
 }
 
+KeyGeo import_geo(const pic_handle *h, int s);  // keys of an import of species s
+
 __device__ __forceinline__ KeyGeo single_geo(const SortArgs &A)
 {
     return key_geo(A.nx, A.ny, A.tw, A.th, A.ntx, 0, A.rows);
@@ -164,6 +166,19 @@ __device__ __forceinline__ int particle_key(const KeyGeo &G, unsigned int *err, 
         return empty;
     }
     return G.key_off + sort_key(c, G);
+}
+
+// Keys of the import's radix sort: the counting sort's, but with the empty
+// slots right after the last key in use (fewer key bits for tile rows).
+__host__ __device__ __forceinline__ long long import_keys(const KeyGeo &G)
+{
+    return (long long)G.nx * G.ny / (G.rows ? G.tw : 1) + 1;
+}
+
+__device__ __forceinline__ uint32_t import_key(const KeyGeo &G, unsigned int *err, int c)
+{
+    const int k = particle_key(G, err, c);
+    return k == G.nx * G.ny ? (uint32_t)(import_keys(G) - 1) : (uint32_t)k;
 }
 
 // first key of the shared-memory window of a block over particles
