@@ -37,7 +37,7 @@ namespace pic {
 
 // ------------------------------------------------------------------ kernels
 template <bool GATHER, bool DEPOSIT>
-__global__ void __launch_bounds__(256, 4)
+__global__ void __launch_bounds__(512, 2)
 ens_push_kernel(PushArgs A, const SegBlock *__restrict__ blk, const EnsRun *__restrict__ runs,
                 const int32_t *__restrict__ anchor, float kick, float drift)
 {
@@ -360,28 +360,80 @@ pic_status ens_layout(pic_ensemble *E)
     return PIC_OK;
 }
 
-// Window halos from the fastest particles of each run's load: the halo
-// along an axis covers half the drift of a sort period (the mean
-// displacement at which a particle is pushed), at least the configured halo,
-// as far as a window of WINDOW_SMEM_TARGET bytes allows.
-void ens_windows(pic_ensemble *E, const pic_init_spec *specs)
+// Tiles, push blocks and window halos of every run for its load.
+//
+// Narrow windows (four 256-thread blocks per SM): halos cover half the drift
+// of the fastest particles over a sort period (the mean displacement at which
+// a particle is pushed), at least the configured halo, as far as a window of
+// WINDOW_SMEM_TARGET bytes allows.
+//
+// Wide windows (two 512-thread blocks per SM, windows up to WINDOW_SMEM_MAX):
+// blocks of up to MAX_CHUNK particles over tiles of up to 512 cells, with
+// halos of the whole drift along both axes.  Beams that cross many cells
+// between sorts leave a narrow window, and once the two-stream instability
+// has saturated their energy is thermal along both axes: at 512^2 a particle
+// then moves 0.57 cells a step each way, 11 in 20 steps.  A particle outside
+// its block's window costs eight global loads and four global atomics.  16
+// runs of up to 512^2 x 256 (209 M particles, a sort every 20 steps), us per
+// step at t < 4, t < 24 and t < 32: narrow 1734, 2676, 3458; wide 1571, 1733,
+// 1802 (blocks of at most 16384: 1684, 1859, 1941; tiles of at most 256 cells:
+// 1599, 1759, 1830; halos of half the drift: 1687, 1803, 1899).  They need
+// particles to fill their blocks (8 runs of up to 256^2 x 64, 10 M particles:
+// 103 us narrow, 110 wide) and fast ones; so they are taken when three
+// quarters of at least 12 M particles belong to runs of 32 or more per cell
+// that drift four cells or more between sorts, and then for every run (the
+// other runs on narrow windows: 1656 us per step instead of 1571).  A block of
+// a dense run then holds just its tile's particles; sized to whole waves
+// instead, blocks straddle two tiles: 1635 us.
+struct RunDrift {
+    double ppc, x, y;  // particles per cell; cells crossed in a sort period
+    bool fast() const { return ppc >= 32.0 && std::max(x, y) >= 4.0; }
+};
+
+static RunDrift run_drift(const pic_ensemble *E, int s, const pic_init_spec &S)
 {
+    const EnsRun &R = E->runs[s];
+    double ux = std::fabs(S.vdrift[0]) + std::fabs(S.beam_v) + 4.0 * std::fabs(S.vth[0]);
+    for (int b = 0; b < 2; ++b) ux += std::hypot(S.beam_u[b][0], S.beam_u[b][1]);
+    const double uy = std::fabs(S.vdrift[1]) + 4.0 * std::fabs(S.vth[1]);
+    const double t = E->sort_every * E->cfg[E->run_of[s]].dt;
+    return RunDrift{(double)S.n / ((double)R.nx * R.ny), ux * t / R.dx, uy * t / R.dy};
+}
+
+void ens_windows(pic_ensemble *E, const pic_init_spec *specs, bool allow_wide)
+{
+    long long total = 0, fast = 0;
+    for (int s = 0; s < E->nruns; ++s) {
+        const pic_init_spec &S = specs[E->run_of[s]];
+        total += S.n;
+        if (run_drift(E, s, S).fast()) fast += S.n;
+    }
+    const bool wide = allow_wide && total >= 12000000 && 4 * fast >= 3 * total;
+    E->push_threads = wide ? 512 : 256;
     E->push_smem = 0;
+    E->per.assign(E->nruns, E->chunk);
     for (int s = 0; s < E->nruns; ++s) {
         EnsRun &R = E->runs[s];
         const int r = E->run_of[s];
-        const pic_init_spec &S = specs[r];
-        const double dt = E->cfg[r].dt;
-        double ux = std::fabs(S.vdrift[0]) + std::fabs(S.beam_v) + 4.0 * std::fabs(S.vth[0]);
-        for (int b = 0; b < 2; ++b) ux += std::hypot(S.beam_u[b][0], S.beam_u[b][1]);
-        const double uy = std::fabs(S.vdrift[1]) + 4.0 * std::fabs(S.vth[1]);
-        const double half = 0.5 * E->sort_every * dt;
-        R.hx = std::max(E->halo, std::min(24, (int)std::ceil(ux * half / R.dx)));
-        R.hy = std::max(E->halo, std::min(24, (int)std::ceil(uy * half / R.dy)));
+        const RunDrift D = run_drift(E, s, specs[r]);
+        double hx = 0.5 * D.x, hy = 0.5 * D.y;
+        if (wide) {
+            hx = D.x;
+            hy = std::max(D.x, D.y);
+            ens_tiles(R, E->cfg[r], std::max(1, (int)std::min((double)MAX_CHUNK, 512.0 * D.ppc)), E->halo);
+            const double n = std::min((double)MAX_CHUNK, 1.35 * D.ppc * R.tw * R.th);
+            E->per[s] = std::max(1024, (int)n & ~3);
+        } else {
+            ens_tiles(R, E->cfg[r], E->chunk, E->halo);
+        }
+        const int most = wide ? 32 : 24;
+        const size_t budget = wide ? WINDOW_SMEM_MAX : WINDOW_SMEM_TARGET;
+        R.hx = std::max(E->halo, (int)std::min((double)most, std::ceil(hx)));
+        R.hy = std::max(E->halo, (int)std::min((double)most, std::ceil(hy)));
         for (;;) {
             R.wcx = 2 * R.tw + 2 * R.hx;
             R.wcy = R.th + 2 * R.hy;
-            if (window_smem(R) <= WINDOW_SMEM_TARGET || (R.hx <= E->halo && R.hy <= E->halo)) break;
+            if (window_smem(R) <= budget || (R.hx <= E->halo && R.hy <= E->halo)) break;
             if (R.hx >= R.hy && R.hx > E->halo)
                 --R.hx;
             else
@@ -398,7 +450,7 @@ pic_status ens_push_table(pic_ensemble *E, const std::vector<long long> &n_slot)
     for (int s = 0; s < E->nruns; ++s) {
         EnsRun &R = E->runs[s];
         R.n = n_slot[s];
-        add_blocks(pb, s, R.poff, (R.n + 3) & ~3ll, E->chunk);
+        add_blocks(pb, s, R.poff, (R.n + 3) & ~3ll, E->per.empty() ? E->chunk : E->per[s]);
     }
     if (E->push_blk) cudaFree(E->push_blk);
     if (E->anchor) cudaFree(E->anchor);
@@ -462,7 +514,7 @@ pic_status ens_launch_push(pic_ensemble *E, int src, int kind)
 {
     if (!E->npush) return PIC_OK;
     const PushArgs A = ens_push_args(E, src);
-    dim3 grid((unsigned)E->npush), block(256);
+    dim3 grid((unsigned)E->npush), block(E->push_threads);
     const size_t sm = E->push_smem;
     // kick and drift coefficients by kind
     static const float KICK[4] = {1.f, -0.5f, 0.f, 0.f}, DRIFT[4] = {1.f, 0.f, 0.f, -1.f};
@@ -767,6 +819,13 @@ pic_status pic_ensemble_synchronize(pic_ensemble *e)
 
 pic_status pic_ensemble_init(pic_ensemble *e, const pic_init_spec *specs)
 {
+    return pic::ens_init(e, specs, true);
+}
+
+}  // extern "C"
+
+pic_status pic::ens_init(pic_ensemble *e, const pic_init_spec *specs, bool wide)
+{
     PIC_TRY(ens_need(e, -1));
     if (!specs) return PIC_ERR_INVALID_ARG;
     std::vector<long long> n_slot(e->nruns);
@@ -785,7 +844,7 @@ pic_status pic_ensemble_init(pic_ensemble *e, const pic_init_spec *specs)
     PIC_CUDA(cudaStreamSynchronize(st));
     const size_t ns = (size_t)e->nslots;
     for (int b = 0; b < 2; ++b) PIC_CUDA(cudaMemsetAsync(e->cell[b], 0xFF, ns * 4, st));
-    ens_windows(e, specs);
+    ens_windows(e, specs, wide);
     PIC_TRY(ens_push_table(e, n_slot));
     std::vector<DevState> z(e->nruns);
     memset(z.data(), 0, sizeof(DevState) * z.size());
@@ -846,6 +905,8 @@ pic_status pic_ensemble_init(pic_ensemble *e, const pic_init_spec *specs)
     e->ready = true;
     return PIC_OK;
 }
+
+extern "C" {
 
 pic_status pic_ensemble_step(pic_ensemble *e, long long nsteps)
 {

@@ -67,6 +67,8 @@ struct pic_ensemble {
     int npush = 0, nsort = 0, nnode_blk = 0, nmode_blk = 0, nhist = 0;
     int32_t *anchor = nullptr;
     size_t push_smem = 0;
+    int push_threads = 256;  // 512 with wide windows (ens_windows)
+    std::vector<int> per;    // particles per push block of each run (slot order)
     // diagnostics
     pic::DevState *dev = nullptr;
     double *hist = nullptr;
@@ -110,6 +112,8 @@ pic_status ens_poisson(pic_ensemble *E, int adv = ADV_FIELD);
 // arrays xin -> xout when given), push-block anchors
 pic_status ens_sort(pic_ensemble *E, const float *const *xin = nullptr, float *const *xout = nullptr);
 pic_status ens_graphs(pic_ensemble *E);
+// pic_ensemble_init; wide: push windows may be wide (see ens_windows)
+pic_status ens_init(pic_ensemble *E, const pic_init_spec *specs, bool wide);
 // pic_import.cu: every run, arbitrary order in buffer 0 -> key order in
 // buffer 1; scratch holds 4 words per slot (12 with packed records), CUB
 // temporary storage grows in temp

@@ -490,7 +490,7 @@ pic_status ens_adjoint(pic_ensemble *E, const pic_init_spec *specs, long long ns
         set_error("pic_ensemble_adjoint: needs specs, nsteps >= 1 and every >= 1");
         return PIC_ERR_INVALID_ARG;
     }
-    PIC_TRY(pic_ensemble_init(E, specs));
+    PIC_TRY(ens_init(E, specs, false));
     cudaStream_t st = E->stream;
     const int nr = E->nruns;
     const size_t ns = (size_t)E->nslots;
