@@ -58,3 +58,28 @@ def test_compat_larger_case_vs_restatement():
                              x, y, vx, vy, 30)
     for k in ("x", "y", "vx", "vy"):
         np.testing.assert_allclose(out[k], ref[k], rtol=0, atol=1e-9, err_msg=k)
+
+
+@pytest.mark.parametrize("nx,ny", [(8, 8), (8, 1024), (1024, 8), (16, 64), (64, 32), (128, 16),
+                                   (12, 10), (2, 3), (16, 20), (9, 32)])
+def test_compat_grid_sizes_vs_restatement(nx, ny):
+    """The own power-of-two transforms (one and several per block, with and
+    without a radix-2 pass) and the cuFFT path, from particles in the domain,
+    on its edges and slightly outside it."""
+    rng = np.random.default_rng(nx * 1000 + ny)
+    kw = dict(xDim=7, yDim=12, nx=nx, ny=ny, npx=37, npy=11, dt=0.01, tmax=1.0, charge=-30.0,
+              mass=7.0)
+    n = 37 * 11
+    x, y = rng.uniform(0, 7, n), rng.uniform(0, 12, n)
+    x[:6] = [0.0, 7.0, -0.0, 7.0 / nx, -0.01 / nx, 7.0]
+    y[:6] = [12.0, 0.0, 12.0, 12.0 / ny, 12.0, -0.01 / ny]
+    vx, vy = rng.normal(0, 3.0, n), rng.normal(0, 3.0, n)
+    ref = O.compat_run(O.ref_params(**kw), x, y, vx, vy, 12)
+    out = P.compat_run_steps(P.ref_params(**kw), x, y, vx, vy, 12)
+    # FP64 with another summation and transform order: the bounds of the
+    # golden cases above
+    for k in ("x", "y", "vx", "vy"):
+        np.testing.assert_allclose(out[k], ref[k], rtol=0, atol=1e-9, err_msg=k)
+    for k in ("rho", "phi", "ex", "ey"):
+        scale = max(np.abs(ref[k]).max(), 1e-300)
+        np.testing.assert_allclose(out[k], ref[k], rtol=0, atol=1e-10 * scale, err_msg=k)
