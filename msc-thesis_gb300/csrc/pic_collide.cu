@@ -12,9 +12,6 @@
 // reproducible for a given particle or cell whatever the storage order.
 #include <cuda_runtime.h>
 
-#include <algorithm>
-#include <cstring>
-
 #include "pic_internal.cuh"
 
 namespace pic {
@@ -48,23 +45,21 @@ struct MccArgs {
     int32_t *ecell;
     float *eox, *eoy, *evx, *evy, *evz;
     uint32_t *epid;
-    long long n0;            // electrons at the start of the pass
+    long long *d_ne;
     long long ecap;
     int32_t *icell;
     float *iox, *ioy, *ivx, *ivy, *ivz;
     uint32_t *ipid;
-    long long ni0;           // ions at the start of the pass
+    long long *d_ni;
     long long icap;
     int has_ion;
     const float *tab;   // [energy | elastic | excitation | ionisation] x ntab
     int ntab;
     float ln_emin, inv_dln;
     float half_me_over_e;  // E[eV] = half_me_over_e * |v|^2
-    float ng, nu_max, two_m_over_M;
-    uint32_t cand_below;  // candidate when the draw's top 24 bits are below (u01f < P_null)
+    float ng, nu_max, p_null, two_m_over_M;
     float e_exc, e_ion, vth_ion;
     uint32_t k0, k1;
-    int e, i;             // electron and ion species
     DevState *dev;
 };
 
@@ -95,10 +90,8 @@ __device__ __forceinline__ void mcc_sigmas(const MccArgs &A, const float *tab, f
 }
 
 constexpr int MCC_THREADS = 256;
-constexpr int MCC_BLOCKS_PER_SM = 4;
-constexpr int MCC_PER_LANE = 8;
-constexpr int MCC_CHUNK = 32 * MCC_PER_LANE;  // electrons a warp tests at a time
-constexpr int MCC_QUEUE = MCC_CHUNK + 32;     // a warp's candidates: a chunk's and up to 31 carried over
+constexpr int MCC_PER_THREAD = 8;
+constexpr int MCC_CHUNK = MCC_THREADS * MCC_PER_THREAD;  // electrons tested per block pass
 
 // Collision of candidate electron i (r: its first draw of this pass):
 // real (elastic, excitation, ionisation with ion birth) or null.
@@ -151,9 +144,9 @@ __device__ __forceinline__ void mcc_collide(const MccArgs &A, const float *s_tab
             // reserve the ion slot, then the electron slot; a reservation past
             // the capacity is given back, so the successful slots stay
             // contiguous from the old count
-            const long long ji = A.ni0 + (long long)atomicAdd(&A.dev->born[1], 1ull);
+            const long long ji = (long long)atomicAdd((unsigned long long *)A.d_ni, 1ull);
             long long je = A.ecap;
-            if (ji < A.icap) je = A.n0 + (long long)atomicAdd(&A.dev->born[0], 1ull);
+            if (ji < A.icap) je = (long long)atomicAdd((unsigned long long *)A.d_ne, 1ull);
             if (ji < A.icap && je < A.ecap) {
                 A.ecell[je] = A.ecell[i];
                 A.eox[je] = A.eox[i];
@@ -178,9 +171,9 @@ __device__ __forceinline__ void mcc_collide(const MccArgs &A, const float *s_tab
                 // no room: give back what was reserved and report; an ion slot
                 // whose electron did not fit stays empty (cell -1)
                 if (ji >= A.icap) {
-                    atomicAdd(&A.dev->born[1], (unsigned long long)-1ll);
+                    atomicAdd((unsigned long long *)A.d_ni, (unsigned long long)-1ll);
                 } else {
-                    atomicAdd(&A.dev->born[0], (unsigned long long)-1ll);
+                    atomicAdd((unsigned long long *)A.d_ne, (unsigned long long)-1ll);
                     A.icell[ji] = -1;
                     A.ipid[ji] = (uint32_t)ji;
                 }
@@ -196,94 +189,76 @@ __device__ __forceinline__ void mcc_collide(const MccArgs &A, const float *s_tab
     A.evz[i] = vz;
 }
 
-// One null-collision pass over the electrons present at its start (births
-// are counted apart and added to the species' counts by the last block).
-// Each warp works on its own, without block barriers: it tests MCC_CHUNK
-// electrons at a time (one Philox draw per electron, keyed by particle id and
-// pass; the ids of its next chunk are loaded meanwhile), queues the
-// candidates (fraction P_null, a few percent) in shared memory and collides
-// them 32 at a time, so that the costly collision path runs in full warps
-// and one warp's collisions overlap the other warps' draws.  Bound by the
-// Philox arithmetic (about 60 issue slots per electron, 32 us for 16.8 M);
-// whether a slot is live is looked up for candidates only.  512^2 x 64 per
-// cell: 79 us against 117 us with a block-wide queue (a barrier before and
-// after each chunk's collisions, which half the threads sat out).
-__global__ void __launch_bounds__(MCC_THREADS, MCC_BLOCKS_PER_SM) mcc_kernel(MccArgs A)
+// One null-collision pass over the electrons present at its start.  Each
+// block takes MCC_CHUNK electrons at a time: first every electron draws its
+// candidate test (one Philox draw keyed by particle id and pass) and the
+// candidates (fraction P_null, a few percent) are queued in shared memory,
+// then the block's threads work through the queue together, so the costly
+// collision path runs in full warps instead of one lane per warp.  A thread
+// loads the cells and ids of all its electrons of a chunk before the first
+// draw, so that their DRAM reads overlap.
+__global__ void __launch_bounds__(MCC_THREADS) mcc_kernel(MccArgs A)
 {
-    extern __shared__ float s_tab[];  // 4 ntab table floats, then a candidate queue per warp
+    extern __shared__ float s_tab[];  // 4 ntab table floats, then the candidate queue
+    int *s_q = reinterpret_cast<int *>(s_tab + 4 * A.ntab);
     for (int i = threadIdx.x; i < 4 * A.ntab; i += blockDim.x) s_tab[i] = A.tab[i];
+    __shared__ unsigned long long s_cnt[4];
+    __shared__ unsigned s_nq;
+    if (threadIdx.x < 4) s_cnt[threadIdx.x] = 0ull;
     __syncthreads();
-    pdl_wait();
-    pdl_trigger();
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    uint32_t *q = reinterpret_cast<uint32_t *>(s_tab + 4 * A.ntab) + MCC_QUEUE * (threadIdx.x >> 5);
-    A.n0 = min(A.dev->n[A.e], A.ecap);
-    A.ni0 = A.has_ion ? A.dev->n[A.i] : 0;
-    const unsigned long long pass = A.dev->mcc_pass + 1ull;
+    // the count at the start of the pass: electrons born in this pass are not
+    // candidates (blocks that start late would otherwise see them)
+    const long long n = min(A.dev->mcc_n0, A.ecap);
+    const unsigned long long pass = A.dev->mcc_pass;
     unsigned c_el = 0, c_exc = 0, c_ion = 0, c_null = 0;
     bool overflow = false;
-    const uint32_t n = (uint32_t)A.n0;  // capacities are below 2^31
-    const uint32_t stride = gridDim.x * (MCC_THREADS / 32) * MCC_CHUNK;
-    uint32_t c0 = (blockIdx.x * (MCC_THREADS / 32) + (threadIdx.x >> 5)) * MCC_CHUNK;
-    uint32_t pid[MCC_PER_LANE];
-    auto load = [&](uint32_t base) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    for (long long c0 = (long long)blockIdx.x * MCC_CHUNK; c0 < n;
+         c0 += (long long)gridDim.x * MCC_CHUNK) {
+        if (threadIdx.x == 0) s_nq = 0u;
+        __syncthreads();
+        int cellv[MCC_PER_THREAD];
+        uint32_t pidv[MCC_PER_THREAD];
 #pragma unroll
-        for (int j = 0; j < MCC_PER_LANE; ++j) {
-            const uint32_t i = base + j * 32 + lane;
-            pid[j] = i < n ? A.epid[i] : 0u;
+        for (int j = 0; j < MCC_PER_THREAD; ++j) {
+            const long long i = c0 + threadIdx.x + j * MCC_THREADS;
+            cellv[j] = i < n ? A.ecell[i] : -1;
+            pidv[j] = i < n ? A.epid[i] : 0u;
         }
-    };
-    auto collide = [&](uint32_t i) {
-        if (A.ecell[i] < 0) return;  // an empty slot
-        const uint32_t id = A.epid[i];
-        const U4 r = philox4x32_10(U4{id, (uint32_t)pass, 0u, STREAM_MCC}, A.k0, A.k1);
-        mcc_collide(A, s_tab, i, id, pass, r, c_el, c_exc, c_ion, c_null, overflow);
-    };
-    int nq = 0;  // queued candidates (warp-uniform)
-    if (c0 < n) load(c0);
-    for (; c0 < n; c0 += stride) {
-        unsigned cand = 0u;
 #pragma unroll
-        for (int j = 0; j < MCC_PER_LANE; ++j) {
-            const U4 r = philox4x32_10(U4{pid[j], (uint32_t)pass, 0u, STREAM_MCC}, A.k0, A.k1);
-            if ((r.x >> 8) < A.cand_below && c0 + j * 32 + lane < n) cand |= 1u << j;
+        for (int j = 0; j < MCC_PER_THREAD; ++j) {  // warp-uniform trip count
+            const int k = threadIdx.x + j * MCC_THREADS;
+            bool cand = false;
+            if (cellv[j] >= 0) {
+                const U4 r = philox4x32_10(U4{pidv[j], (uint32_t)pass, 0u, STREAM_MCC}, A.k0, A.k1);
+                cand = u01f(r.x) < A.p_null;
+            }
+            const unsigned m = __ballot_sync(full, cand);
+            if (m) {
+                unsigned base = 0u;
+                if (lane == 0) base = atomicAdd(&s_nq, (unsigned)__popc(m));
+                base = __shfl_sync(full, base, 0);
+                if (cand) s_q[base + __popc(m & ((1u << lane) - 1u))] = k;
+            }
         }
-        if (n - c0 > stride) load(c0 + stride);
-#pragma unroll
-        for (int j = 0; j < MCC_PER_LANE; ++j) {
-            const bool mine = (cand >> j) & 1u;
-            const unsigned m = __ballot_sync(full, mine);
-            if (mine) q[nq + __popc(m & ((1u << lane) - 1u))] = c0 + j * 32 + lane;
-            nq += __popc(m);
+        __syncthreads();
+        const int nq = (int)s_nq;
+        for (int j = threadIdx.x; j < nq; j += blockDim.x) {
+            const long long i = c0 + s_q[j];
+            const uint32_t pid = A.epid[i];
+            const U4 r = philox4x32_10(U4{pid, (uint32_t)pass, 0u, STREAM_MCC}, A.k0, A.k1);
+            mcc_collide(A, s_tab, i, pid, pass, r, c_el, c_exc, c_ion, c_null, overflow);
         }
-        __syncwarp();
-        while (nq >= 32) {
-            nq -= 32;
-            collide(q[nq + lane]);
-        }
-        __syncwarp();  // the queue is written again by the next chunk
+        __syncthreads();  // the queue is reused by the next chunk
     }
-    if (lane < nq) collide(q[lane]);
-    c_el = __reduce_add_sync(full, c_el);
-    c_exc = __reduce_add_sync(full, c_exc);
-    c_ion = __reduce_add_sync(full, c_ion);
-    c_null = __reduce_add_sync(full, c_null);
-    if (lane < 4) {
-        const unsigned c = lane == 0 ? c_el : lane == 1 ? c_exc : lane == 2 ? c_ion : c_null;
-        if (c) atomicAdd(&A.dev->coll[lane][acc_slot()], (unsigned long long)c);
-    }
+    atomicAdd(&s_cnt[0], (unsigned long long)c_el);
+    atomicAdd(&s_cnt[1], (unsigned long long)c_exc);
+    atomicAdd(&s_cnt[2], (unsigned long long)c_ion);
+    atomicAdd(&s_cnt[3], (unsigned long long)c_null);
     const int any_over = __syncthreads_or(overflow ? 1 : 0);
-    if (threadIdx.x == 0) {
-        if (any_over) atomicOr(&A.dev->err, (unsigned)PIC_DEVERR_CAPACITY);
-        __threadfence();  // this block's births before its ticket
-        if (atomicInc(&A.dev->ticket, gridDim.x - 1) == gridDim.x - 1) {
-            __threadfence();
-            A.dev->n[A.e] += (long long)atomicExch(&A.dev->born[0], 0ull);
-            if (A.has_ion) A.dev->n[A.i] += (long long)atomicExch(&A.dev->born[1], 0ull);
-            A.dev->mcc_pass = pass;
-        }
-    }
+    if (threadIdx.x < 4) atomicAdd(&A.dev->coll[threadIdx.x][acc_slot()], s_cnt[threadIdx.x]);
+    if (threadIdx.x == 0 && any_over) atomicOr(&A.dev->err, (unsigned)PIC_DEVERR_CAPACITY);
 }
 
 // ---------------------------------------------------------------- DSMC
@@ -365,22 +340,14 @@ __global__ void __launch_bounds__(256) ntc_kernel(NtcArgs A)
 
 __global__ void bump_kernel(unsigned long long *counter) { *counter += 1ull; }
 
-// ---------------------------------------------------------------- launchers
-// The number of 24-bit draws k with u01f(k << 8) < p (u01f is monotone): an
-// electron is a candidate when its draw's top 24 bits are below it.
-uint32_t mcc_candidates_below(float p)
+// opens an MCC pass: new pass number and the electron count it works on
+__global__ void mcc_prepare_kernel(DevState *d, int e)
 {
-    uint32_t lo = 0, hi = 1u << 24;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi) / 2;
-        if (u01f(mid << 8) < p)
-            lo = mid + 1;
-        else
-            hi = mid;
-    }
-    return lo;
+    d->mcc_pass += 1ull;
+    d->mcc_n0 = d->n[e];
 }
 
+// ---------------------------------------------------------------- launchers
 pic_status launch_mcc(pic_handle *h)
 {
     const MccState &M = h->mcc;
@@ -394,6 +361,7 @@ pic_status launch_mcc(pic_handle *h)
     A.evy = E.vy[0];
     A.evz = E.vz[0];
     A.epid = E.pid[0];
+    A.d_ne = &h->dev->n[M.e];
     A.ecap = E.cap;
     if (M.i >= 0) {
         SpeciesBuf &I = h->sp[M.i];
@@ -404,6 +372,7 @@ pic_status launch_mcc(pic_handle *h)
         A.ivy = I.vy[0];
         A.ivz = I.vz[0];
         A.ipid = I.pid[0];
+        A.d_ni = &h->dev->n[M.i];
         A.icap = I.cap;
         A.has_ion = 1;
     }
@@ -414,9 +383,7 @@ pic_status launch_mcc(pic_handle *h)
     A.half_me_over_e = M.half_me_over_e;
     A.ng = M.ng;
     A.nu_max = M.nu_max;
-    A.cand_below = M.cand_below;
-    A.e = M.e;
-    A.i = M.i;
+    A.p_null = M.p_null;
     A.two_m_over_M = M.two_m_over_M;
     A.e_exc = M.e_exc;
     A.e_ion = M.e_ion;
@@ -424,13 +391,12 @@ pic_status launch_mcc(pic_handle *h)
     A.k0 = (uint32_t)M.seed;
     A.k1 = (uint32_t)(M.seed >> 32);
     A.dev = h->dev;
-    void *args[] = {&A};
-    const long long warps = (E.cap + MCC_CHUNK - 1) / MCC_CHUNK, per = MCC_THREADS / 32;
-    const long long most = (long long)MCC_BLOCKS_PER_SM * device_sms();
-    const unsigned blocks = (unsigned)std::max(1ll, std::min((warps + per - 1) / per, most));
-    const size_t smem = 4 * M.ntab * sizeof(float) + (MCC_THREADS / 32) * MCC_QUEUE * sizeof(uint32_t);
-    PIC_TRY(allow_dynamic_smem((const void *)mcc_kernel, smem));
-    return launch_dependent((const void *)mcc_kernel, blocks, MCC_THREADS, smem, h->stream, args);
+    mcc_prepare_kernel<<<1, 1, 0, h->stream>>>(h->dev, M.e);
+    PIC_CUDA(cudaGetLastError());
+    mcc_kernel<<<grid_for(E.cap, MCC_CHUNK), MCC_THREADS,
+                 4 * M.ntab * sizeof(float) + MCC_CHUNK * sizeof(int), h->stream>>>(A);
+    PIC_CUDA(cudaGetLastError());
+    return PIC_OK;
 }
 
 // DSMC pass on species D.s, which must have just been sorted (buffer 1, offsets)

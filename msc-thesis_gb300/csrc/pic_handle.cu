@@ -1221,7 +1221,7 @@ extern "C" pic_status pic_set_mcc(pic_handle *h, const pic_mcc_params *p)
     M.half_me_over_e = (float)(0.5 * p->electron_mass / p->unit_charge);
     M.ng = (float)p->neutral_density;
     M.nu_max = (float)nu_max;
-    M.cand_below = mcc_candidates_below((float)(1.0 - std::exp(-nu_max * c.dt)));
+    M.p_null = (float)(1.0 - std::exp(-nu_max * c.dt));
     M.two_m_over_M = (float)(2.0 * p->electron_mass / p->ion_mass);
     M.e_exc = (float)p->e_exc_eV;
     M.e_ion = (float)p->e_ion_eV;

@@ -167,7 +167,7 @@ struct DevState {
     unsigned int err;         // PIC_DEVERR_* bits
     unsigned int ticket;      // blocks of the k-space kernel that are done (wraps to 0)
     unsigned long long mcc_pass, dsmc_pass;  // collision pass counters (Philox counters)
-    unsigned long long born[2];  // electrons and ions born in the current MCC pass
+    long long mcc_n0;         // electron count at the start of the current MCC pass
 };
 __device__ __forceinline__ int acc_slot() { return (int)(blockIdx.x & (ACC_SLOTS - 1)); }
 
@@ -177,8 +177,7 @@ struct MccState {
     int e = 0, i = -1;        // electron / ion species
     float *tab = nullptr;     // device [energy | elastic | excitation | ionisation] x ntab
     int ntab = 0;
-    float ln_emin = 0, inv_dln = 0, half_me_over_e = 0, ng = 0, nu_max = 0;
-    uint32_t cand_below = 0;  // see mcc_candidates_below
+    float ln_emin = 0, inv_dln = 0, half_me_over_e = 0, ng = 0, nu_max = 0, p_null = 0;
     float two_m_over_M = 0, e_exc = 0, e_ion = 0, vth_ion = 0;
     unsigned long long seed = 0;
 };
@@ -306,7 +305,6 @@ pic_status launch_key_scan(const uint32_t *count, uint32_t *offset, uint32_t *cu
 // pic_collide.cu
 pic_status launch_mcc(pic_handle *h);
 pic_status launch_ntc(pic_handle *h);
-uint32_t mcc_candidates_below(float p_null);
 // pic_init.cu
 pic_status launch_init(pic_handle *h, int s, const pic_init_spec *spec, int lat_nx, int lat_ny);
 pic_status launch_from_global(pic_handle *h, int s, long long n, const double *x_dev,
