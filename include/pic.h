@@ -258,7 +258,7 @@ pic_status pic_set_mcc(pic_handle *h, const pic_mcc_params *p);
 
 /* Neutral-neutral DSMC with Bird's no-time-counter scheme (Bird, Molecular
  * Gas Dynamics and the Direct Simulation of Gas Flows, 1994), hard spheres:
- * per cell of the cell-sorted array, N = 1/2 n (n-1) F_N (sigma g)_max dt_c
+ * per cell, N = 1/2 n (n-1) F_N (sigma g)_max dt_c
  * / V_c candidate pairs (fraction by randomised rounding), each accepted
  * with probability sigma g / (sigma g)_max, isotropic scattering in the
  * centre-of-mass frame.  (sigma g)_max is kept per cell and raised when

@@ -12,7 +12,7 @@
 // reproducible for a given particle or cell whatever the storage order.
 #include <cuda_runtime.h>
 
-#include "pic_internal.cuh"
+#include "pic_sort_dev.cuh"
 
 namespace pic {
 
@@ -197,6 +197,9 @@ __device__ __forceinline__ void mcc_collide(const MccArgs &A, const float *s_tab
 // collision path runs in full warps instead of one lane per warp.  A thread
 // loads the cells and ids of all its electrons of a chunk before the first
 // draw, so that their DRAM reads overlap.
+// (By warps with queues of their own, without block barriers, the pass took 79
+// instead of 117 us; but births take slots, ids and with them random streams
+// in the order in which the blocks come to them, which that changed.)
 __global__ void __launch_bounds__(MCC_THREADS) mcc_kernel(MccArgs A)
 {
     extern __shared__ float s_tab[];  // 4 ntab table floats, then the candidate queue
@@ -262,47 +265,155 @@ __global__ void __launch_bounds__(MCC_THREADS) mcc_kernel(MccArgs A)
 }
 
 // ---------------------------------------------------------------- DSMC
+// The scheme draws a few pairs per cell and step, so it needs lists of the
+// cells that collide, not a sorted array: three passes
+//   count   per cell: its candidate pairs of this step; a cell that has any
+//           reserves room for its particles in the list
+//   list    every particle of such a cell enters its slot number
+//   collide per cell: the pairs, drawn from its part of the list
+// (Sorting the species every step instead, at 512^2 x 50 per cell: 154 us for
+// the scatter, 11 us for the scans, and a push from the sorted buffer back
+// that moves ids and vz too, 113 us; these passes take 5 + 22 + 7 us and the
+// push in place 81 us.)
 struct NtcArgs {
-    float *vx, *vy, *vz;      // the species' sorted buffer
-    const uint32_t *offset;   // per key: particles [offset[k], offset[k+1])
+    const int32_t *cell;
+    float *vx, *vy, *vz;
+    const uint32_t *count;    // per key: particles of the cell (kept current by the pushes)
+    uint32_t *pairs;          // per key: candidate pairs of this pass
+    uint32_t *start;          // per key with pairs: first entry of its list
+    uint32_t *cursor;         // per key: next free entry, or NTC_NONE without pairs
+    uint32_t *list;           // slot numbers
     float *sgmax;             // per key (sigma g)_max
-    long long nkeys;
-    long long nslots;         // slots of the sorted buffer (bound of the offsets)
+    const long long *d_n;
+    uint32_t nkeys;
+    uint32_t nslots;          // slots of the species (bound of the list)
+    KeyGeo geo;
     float sigma;              // pi d^2
     float coef;               // F_N dt_c / (2 V_c)
     uint32_t k0, k1;
     DevState *dev;
 };
+constexpr uint32_t NTC_NONE = 0xFFFFFFFFu;
 
-__global__ void __launch_bounds__(256) ntc_kernel(NtcArgs A)
+__global__ void __launch_bounds__(256) ntc_count_kernel(NtcArgs A)
 {
-    __shared__ unsigned long long s_cnt[2];
-    if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0ull;
-    __syncthreads();
+    pdl_wait();
+    pdl_trigger();
+    const unsigned long long pass = A.dev->dsmc_pass;
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const uint32_t stride = gridDim.x * blockDim.x;
+    // a warp's cells together (one reservation for all of them)
+    for (uint32_t k0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); k0 < A.nkeys; k0 += stride) {
+        const uint32_t key = k0 + lane;
+        const uint32_t n = key < A.nkeys ? A.count[key] : 0u;
+        uint32_t nc = 0u;
+        if (n >= 2) {
+            const float want = A.coef * (float)n * (float)(n - 1) * A.sgmax[key];
+            const U4 r0 = philox4x32_10(U4{key, (uint32_t)pass, 0u, STREAM_DSMC}, A.k0, A.k1);
+            const float fl = floorf(want);
+            nc = (uint32_t)fl + (u01f(r0.x) < want - fl ? 1u : 0u);
+        }
+        uint32_t at = NTC_NONE;
+        if (__any_sync(full, nc != 0u)) {
+            const uint32_t mine = nc ? n : 0u;
+            uint32_t sum = mine;  // inclusive over the lanes
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(full, sum, o);
+                if (lane >= o) sum += t;
+            }
+            uint32_t base = 0u;
+            if (lane == 31) base = atomicAdd(&A.dev->ntc_listed, sum);
+            base = __shfl_sync(full, base, 31);
+            if (nc) {
+                at = base + sum - mine;
+                if (n > A.nslots || at > A.nslots - n) {  // counts that do not fit the slots
+                    atomicOr(&A.dev->err, (unsigned)PIC_DEVERR_SORT);
+                    nc = 0u;
+                    at = NTC_NONE;
+                }
+            }
+        }
+        if (key >= A.nkeys) continue;
+        A.pairs[key] = nc;
+        A.cursor[key] = at;
+        if (nc) A.start[key] = at;
+    }
+}
+
+// Quads of four consecutive particles, NTC_QUADS of them loaded at a time; the
+// particles of a run in one cell enter together (one atomic).
+constexpr int NTC_QUADS = 4;
+
+__global__ void __launch_bounds__(256) ntc_list_kernel(NtcArgs A)
+{
+    pdl_wait();
+    pdl_trigger();
+    const uint32_t n = (uint32_t)*A.d_n;  // capacities are below 2^31
+    const uint32_t step = 4u * blockDim.x;
+    for (uint32_t q0 = blockIdx.x * NTC_QUADS * step + 4u * threadIdx.x; q0 < n;
+         q0 += gridDim.x * NTC_QUADS * step) {
+        int4 c4[NTC_QUADS];
+#pragma unroll
+        for (int u = 0; u < NTC_QUADS; ++u) {
+            const uint32_t q = q0 + u * step;
+            c4[u] = q < n ? *reinterpret_cast<const int4 *>(A.cell + q) : make_int4(-1, -1, -1, -1);
+        }
+#pragma unroll
+        for (int u = 0; u < NTC_QUADS; ++u) {
+            const uint32_t q = q0 + u * step;
+            const int c[4] = {c4[u].x, q + 1 < n ? c4[u].y : -1, q + 2 < n ? c4[u].z : -1,
+                              q + 3 < n ? c4[u].w : -1};
+            uint32_t slot = 0u;  // list entry of the current run's first particle
+            bool listed = false;
+            int first = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (j == 0 || c[j] != c[j - 1]) {
+                    first = j;
+                    listed = false;
+                    if (c[j] >= 0 && (c[j] & 0xFFFF) < A.geo.nx && (c[j] >> 16) < A.geo.ny) {
+                        const int key = cell_key(c[j], A.geo);
+                        if (A.cursor[key] != NTC_NONE) {
+                            uint32_t len = 1u;
+#pragma unroll
+                            for (int e = j + 1; e < 4; ++e)
+                                if (len == (uint32_t)(e - j) && c[e] == c[j]) ++len;
+                            slot = atomicAdd(A.cursor + key, len);
+                            listed = true;
+                        }
+                    }
+                }
+                const uint32_t o = slot + (uint32_t)(j - first);
+                if (listed && o < A.nslots) A.list[o] = q + j;
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(256) ntc_collide_kernel(NtcArgs A)
+{
+    pdl_wait();
+    pdl_trigger();
     const unsigned long long pass = A.dev->dsmc_pass;
     unsigned ncoll = 0, ncand = 0;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long key = (long long)blockIdx.x * blockDim.x + threadIdx.x; key < A.nkeys;
-         key += stride) {
-        const uint32_t o0 = A.offset[key], o1 = A.offset[key + 1];
-        if (o1 < o0 || (long long)o1 > A.nslots) {  // offsets that do not fit the slots
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t key = blockIdx.x * blockDim.x + threadIdx.x; key < A.nkeys; key += stride) {
+        const uint32_t nc = A.pairs[key];
+        if (!nc) continue;
+        const uint32_t o0 = A.start[key], n = A.count[key];
+        if (A.cursor[key] != o0 + n) {  // the list does not hold the cell's count
             atomicOr(&A.dev->err, (unsigned)PIC_DEVERR_SORT);
             continue;
         }
-        const uint32_t n = o1 - o0;
-        if (n < 2) continue;
         float sgm = A.sgmax[key];
-        const float want = A.coef * (float)n * (float)(n - 1) * sgm;
-        const U4 r0 = philox4x32_10(U4{(uint32_t)key, (uint32_t)pass, 0u, STREAM_DSMC}, A.k0, A.k1);
-        const float fl = floorf(want);
-        const uint32_t nc = (uint32_t)fl + (u01f(r0.x) < want - fl ? 1u : 0u);
         for (uint32_t c = 0; c < nc; ++c) {
-            const U4 r = philox4x32_10(U4{(uint32_t)key, (uint32_t)pass, 2u * c + 1u, STREAM_DSMC},
-                                       A.k0, A.k1);
+            const U4 r = philox4x32_10(U4{key, (uint32_t)pass, 2u * c + 1u, STREAM_DSMC}, A.k0, A.k1);
             uint32_t a = min((uint32_t)(u01f(r.x) * (float)n), n - 1);
             uint32_t b = min((uint32_t)(u01f(r.y) * (float)(n - 1)), n - 2);
             if (b >= a) ++b;
-            const uint32_t i = o0 + a, j = o0 + b;
+            const uint32_t i = A.list[o0 + a], j = A.list[o0 + b];
             const float gx = A.vx[i] - A.vx[j], gy = A.vy[i] - A.vy[j], gz = A.vz[i] - A.vz[j];
             const float g = sqrtf(gx * gx + gy * gy + gz * gz);
             const float sg = A.sigma * g;
@@ -310,8 +421,7 @@ __global__ void __launch_bounds__(256) ntc_kernel(NtcArgs A)
             ++ncand;
             if (u01f(r.z) * sgm >= sg) continue;
             // hard spheres: isotropic post-collision relative velocity in the CM frame
-            const U4 r2 = philox4x32_10(U4{(uint32_t)key, (uint32_t)pass, 2u * c + 2u, STREAM_DSMC},
-                                        A.k0, A.k1);
+            const U4 r2 = philox4x32_10(U4{key, (uint32_t)pass, 2u * c + 2u, STREAM_DSMC}, A.k0, A.k1);
             const float cx = 2.f * u01f(r.w) - 1.f;
             const float sx = sqrtf(fmaxf(0.f, 1.f - cx * cx));
             float sp, cp;
@@ -329,16 +439,22 @@ __global__ void __launch_bounds__(256) ntc_kernel(NtcArgs A)
         }
         A.sgmax[key] = sgm;
     }
-    atomicAdd(&s_cnt[0], (unsigned long long)ncoll);
-    atomicAdd(&s_cnt[1], (unsigned long long)ncand);
+    const unsigned full = 0xffffffffu;
+    ncoll = __reduce_add_sync(full, ncoll);
+    ncand = __reduce_add_sync(full, ncand);
+    if ((threadIdx.x & 31) == 0 && ncand) {
+        atomicAdd(&A.dev->coll[4][acc_slot()], (unsigned long long)ncoll);
+        atomicAdd(&A.dev->coll[5][acc_slot()], (unsigned long long)ncand);
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
-        atomicAdd(&A.dev->coll[4][acc_slot()], s_cnt[0]);
-        atomicAdd(&A.dev->coll[5][acc_slot()], s_cnt[1]);
+        // every block has read the pass number before its ticket
+        if (atomicInc(&A.dev->ticket, gridDim.x - 1) == gridDim.x - 1) {
+            A.dev->dsmc_pass = pass + 1ull;
+            A.dev->ntc_listed = 0u;
+        }
     }
 }
-
-__global__ void bump_kernel(unsigned long long *counter) { *counter += 1ull; }
 
 // opens an MCC pass: new pass number and the electron count it works on
 __global__ void mcc_prepare_kernel(DevState *d, int e)
@@ -399,29 +515,39 @@ pic_status launch_mcc(pic_handle *h)
     return PIC_OK;
 }
 
-// DSMC pass on species D.s, which must have just been sorted (buffer 1, offsets)
-pic_status launch_ntc(pic_handle *h)
+// DSMC pass on species D.s in buffer `from`, whose counts are current; the
+// list takes the place of the other buffer's ids.
+pic_status launch_ntc(pic_handle *h, int from)
 {
     const DsmcState &D = h->dsmc;
     SpeciesBuf &B = h->sp[D.s];
+    const Geometry &g = h->g;
     NtcArgs A;
-    A.vx = B.vx[1];
-    A.vy = B.vy[1];
-    A.vz = B.vz[1];
-    A.offset = h->offset;
+    A.cell = B.cell[from];
+    A.vx = B.vx[from];
+    A.vy = B.vy[from];
+    A.vz = B.vz[from];
+    A.count = D.count;
+    A.pairs = h->count;
+    A.start = h->offset;
+    A.cursor = h->cursor;
+    A.list = B.pid[1 - from];
     A.sgmax = D.sgmax;
-    A.nkeys = (long long)h->g.nx * h->g.ny;
-    A.nslots = B.cap;
+    A.d_n = &h->dev->n[D.s];
+    A.nkeys = (uint32_t)(g.nx * g.ny);
+    A.nslots = (uint32_t)B.cap;
+    A.geo = key_geo(g.nx, g.ny, g.tw, g.th, g.ntx, 0);
     A.sigma = D.sigma;
     A.coef = D.coef;
     A.k0 = (uint32_t)D.seed;
     A.k1 = (uint32_t)(D.seed >> 32);
     A.dev = h->dev;
-    ntc_kernel<<<grid_for(A.nkeys, 256), 256, 0, h->stream>>>(A);
-    PIC_CUDA(cudaGetLastError());
-    bump_kernel<<<1, 1, 0, h->stream>>>(&h->dev->dsmc_pass);
-    PIC_CUDA(cudaGetLastError());
-    return PIC_OK;
+    void *args[] = {&A};
+    const int gk = grid_for(A.nkeys, 256);
+    PIC_TRY(launch_dependent((const void *)ntc_count_kernel, gk, 256, 0, h->stream, args));
+    PIC_TRY(launch_dependent((const void *)ntc_list_kernel, grid_for((B.cap + 4 * NTC_QUADS - 1) / (4 * NTC_QUADS), 256), 256, 0,
+                             h->stream, args));
+    return launch_dependent((const void *)ntc_collide_kernel, gk, 256, 0, h->stream, args);
 }
 
 }  // namespace pic

@@ -124,7 +124,9 @@ __device__ __forceinline__ void compat_place(const CompatDev &D, long long k, do
 // Gather, lagged kick-drift-kick and the deposit of the new position for the
 // next step, in one pass: the weights computed for the deposit are those of
 // the next gather (32 bytes kept per particle instead of 24 FP64 operations).
-// @COMPAT@
+// 128^2, 1.6 M particles: 220 us against 377 us for a push and 194 us for a
+// deposit that each computed cells and weights with general divisions; 64
+// FP64 operations per particle, 168 us at the pipe's rate.
 template <bool DEPOSIT>
 __global__ void compat_push_kernel(CompatDev D)
 {

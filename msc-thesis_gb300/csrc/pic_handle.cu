@@ -311,19 +311,13 @@ pic_status record_poisson(pic_handle *h, int adv)
 }
 
 // Particle pass of one step.  src = 1: every species was just sorted into
-// buffer 1.  A DSMC species is sorted every step and collides on its sorted
-// buffer before its push moves it back; MCC follows the push.
+// buffer 1.  A DSMC species collides before its push; MCC follows the push.
 pic_status record_push_all(pic_handle *h, int src, bool deposit, bool fold)
 {
     for (int s = 0; s < h->cfg.nspecies; ++s) {
         if (!h->sp[s].cap) continue;
-        int from = src;
-        if (h->dsmc.on && s == h->dsmc.s) {
-            if (!src) PIC_TRY(launch_sort(h, s, true));  // counts kept by its last push
-            PIC_TRY(launch_ntc(h));
-            from = 1;
-        }
-        PIC_TRY(launch_push(h, s, from, deposit, 1.0f));
+        if (h->dsmc.on && s == h->dsmc.s) PIC_TRY(launch_ntc(h, src));
+        PIC_TRY(launch_push(h, s, src, deposit, 1.0f));
     }
     if (fold) PIC_TRY(launch_advance(h, ADV_PUSH));
     if (h->mcc.on) PIC_TRY(launch_mcc(h));
@@ -337,13 +331,10 @@ static pic_status record_step(pic_handle *h, int src)
     return record_poisson(h, ADV_PUSH | ADV_FIELD);
 }
 
-// Sort every species; the DSMC species goes last so that the cell offsets it
-// collides on are the ones left in the shared sort buffers.
 static pic_status record_sort_all(pic_handle *h)
 {
     for (int s = 0; s < h->cfg.nspecies; ++s)
-        if (h->sp[s].cap && !(h->dsmc.on && s == h->dsmc.s)) PIC_TRY(launch_sort(h, s));
-    if (h->dsmc.on && h->sp[h->dsmc.s].cap) PIC_TRY(launch_sort(h, h->dsmc.s));
+        if (h->sp[s].cap) PIC_TRY(launch_sort(h, s));
     return PIC_OK;
 }
 
@@ -1275,7 +1266,7 @@ extern "C" pic_status pic_collide(pic_handle *h, int kind)
             return PIC_ERR_STATE;
         }
         PIC_TRY(launch_sort(h, h->dsmc.s, true));
-        PIC_TRY(launch_ntc(h));
+        PIC_TRY(launch_ntc(h, 1));
         return copy_back(h, h->dsmc.s);
     }
     set_error("pic_collide: unknown collision kind");

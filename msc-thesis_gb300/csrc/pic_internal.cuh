@@ -166,6 +166,7 @@ struct DevState {
     long long n[PIC_MAX_SPECIES];
     unsigned int err;         // PIC_DEVERR_* bits
     unsigned int ticket;      // blocks of the k-space kernel that are done (wraps to 0)
+    unsigned int ntc_listed, pad;  // particles listed in the current DSMC pass
     unsigned long long mcc_pass, dsmc_pass;  // collision pass counters (Philox counters)
     long long mcc_n0;         // electron count at the start of the current MCC pass
 };
@@ -304,7 +305,7 @@ pic_status launch_key_scan(const uint32_t *count, uint32_t *offset, uint32_t *cu
                            const long long *d_total, cudaStream_t st);
 // pic_collide.cu
 pic_status launch_mcc(pic_handle *h);
-pic_status launch_ntc(pic_handle *h);
+pic_status launch_ntc(pic_handle *h, int from);
 // pic_init.cu
 pic_status launch_init(pic_handle *h, int s, const pic_init_spec *spec, int lat_nx, int lat_ny);
 pic_status launch_from_global(pic_handle *h, int s, long long n, const double *x_dev,
