@@ -19,6 +19,7 @@
 #include <cufft.h>
 
 #include <algorithm>
+#include <cstring>
 #include <vector>
 
 #include "pic_adjoint_dev.cuh"
@@ -27,56 +28,33 @@ namespace pic {
 
 struct AdjArgs {
     const int32_t *cell;
-    const float *ox, *oy;      // positions of the step (ring slot)
-    const float *ex, *ey;      // field of the step
-    float *ax, *ay, *avx, *avy;  // adjoint state (storage order)
-    float *gx, *gy;            // scatter target planes
-    const float *psi;          // S^T g
+    const float *ox, *oy;        // positions of the step
+    float *ax, *ay;              // adjoint positions (storage order)
+    const float *psi;            // S^T g
     long long n;
     int nx, ny;
     float inv_dx, inv_dy;
-    float C;                   // kick coefficient times q/m
-    float drift_dt;            // dt for the drift adjoint (0: none)
     float q_over_dA;
 };
 
-// drift adjoint, kick local term and scatter of mu
-__global__ void __launch_bounds__(256) adj_kick_scatter_kernel(AdjArgs A)
+// Drift adjoint, kick local term and scatter of mu, one push chunk per block
+// (adj_kick_block; 128^2 x 32 per cell: 16 us against 21 us with eight global
+// float adds per particle).
+__global__ void __launch_bounds__(256, 3)
+adj_kick_kernel(KickArgs A, KickGeo K, const int32_t *__restrict__ anchor, int chunk, long long n4)
 {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < A.n; i += stride) {
-        const Cic w = cic_of(A.cell[i], A.ox[i], A.oy[i], A.nx, A.ny);
-        if (!w.ok) continue;
-        float ax = A.ax[i], ay = A.ay[i];
-        float avx = A.avx[i], avy = A.avy[i];
-        avx = fmaf(A.drift_dt, ax, avx);
-        avy = fmaf(A.drift_dt, ay, avy);
-        const float mx = A.C * avx, my = A.C * avy;
-        const float gx = 1.f - w.fx, gy = 1.f - w.fy;
-        const float w00 = gx * gy, w10 = w.fx * gy, w01 = gx * w.fy, w11 = w.fx * w.fy;
-        atomicAdd(A.gx + w.i00, w00 * mx);
-        atomicAdd(A.gy + w.i00, w00 * my);
-        atomicAdd(A.gx + w.i10, w10 * mx);
-        atomicAdd(A.gy + w.i10, w10 * my);
-        atomicAdd(A.gx + w.i01, w01 * mx);
-        atomicAdd(A.gy + w.i01, w01 * my);
-        atomicAdd(A.gx + w.i11, w11 * mx);
-        atomicAdd(A.gy + w.i11, w11 * my);
-        const float s00 = A.ex[w.i00] * mx + A.ey[w.i00] * my;
-        const float s10 = A.ex[w.i10] * mx + A.ey[w.i10] * my;
-        const float s01 = A.ex[w.i01] * mx + A.ey[w.i01] * my;
-        const float s11 = A.ex[w.i11] * mx + A.ey[w.i11] * my;
-        const float2 l = grad_dot(w, s00, s10, s01, s11, A.inv_dx, A.inv_dy);
-        A.ax[i] = ax + l.x;
-        A.ay[i] = ay + l.y;
-        A.avx[i] = avx;
-        A.avy[i] = avy;
-    }
+    extern __shared__ __align__(16) unsigned char smem[];
+    pdl_wait();
+    pdl_trigger();
+    const long long base = (long long)blockIdx.x * chunk;
+    adj_kick_block<false>(A, K, smem, base, min(base + (long long)chunk, n4), anchor[blockIdx.x]);
 }
 
 // adjoint of the deposit: a_x += (q/dA) sum_m psi_m grad w_m
 __global__ void __launch_bounds__(256) adj_gather_kernel(AdjArgs A)
 {
+    pdl_wait();
+    pdl_trigger();
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < A.n; i += stride) {
         const Cic w = cic_of(A.cell[i], A.ox[i], A.oy[i], A.nx, A.ny);
@@ -127,22 +105,26 @@ __global__ void to_id_order_kernel(const float *a, const float *b, const uint32_
 // ---------------------------------------------------------------- driver
 namespace {
 
+// An adjoint run's device memory: one block, carved up by a layout that is
+// run twice (sizes, then addresses).  Up to ADJ_STAGE_MAX bytes lie in the
+// handle's stage, which later runs find in place; more is allocated for the
+// call alone.
+constexpr size_t ADJ_STAGE_MAX = 256ull << 20;
+
 struct AdjWork {
-    pic_handle *h;
-    std::vector<void *> allocs;
+    char *base = nullptr, *own = nullptr;
+    size_t used = 0;
     cufftHandle r2c2 = 0;
     ~AdjWork()
     {
-        for (void *p : allocs) cudaFree(p);
+        if (own) cudaFree(own);
         if (r2c2) cufftDestroy(r2c2);
     }
-    template <class T> pic_status alloc(T **p, size_t n)
+    template <class T> T *take(size_t n)
     {
-        void *q = nullptr;
-        PIC_CUDA(cudaMalloc(&q, (n ? n : 1) * sizeof(T)));
-        allocs.push_back(q);
-        *p = (T *)q;
-        return PIC_OK;
+        char *p = base + used;
+        used += (n * sizeof(T) + 255) & ~(size_t)255;
+        return reinterpret_cast<T *>(p);
     }
 };
 
@@ -151,34 +133,25 @@ struct Snap {  // particle state of species 0 (storage order)
     float *ox, *oy, *vx, *vy;
 };
 
-pic_status snap_alloc(AdjWork &W, Snap &S, size_t n)
+Snap take_snap(AdjWork &W, size_t n)
 {
-    PIC_TRY(W.alloc(&S.cell, n));
-    PIC_TRY(W.alloc(&S.ox, n));
-    PIC_TRY(W.alloc(&S.oy, n));
-    PIC_TRY(W.alloc(&S.vx, n));
-    PIC_TRY(W.alloc(&S.vy, n));
-    return PIC_OK;
+    Snap S;
+    S.cell = W.take<int32_t>(n);
+    S.ox = W.take<float>(n);
+    S.oy = W.take<float>(n);
+    S.vx = W.take<float>(n);
+    S.vy = W.take<float>(n);
+    return S;
 }
 
 pic_status snap_copy(pic_handle *h, Snap &S, bool save, size_t n)
 {
     SpeciesBuf &B = h->sp[0];
-    const cudaMemcpyKind k = cudaMemcpyDeviceToDevice;
-    cudaStream_t st = h->stream;
-    if (save) {
-        PIC_CUDA(cudaMemcpyAsync(S.cell, B.cell[0], n * 4, k, st));
-        PIC_CUDA(cudaMemcpyAsync(S.ox, B.ox[0], n * 4, k, st));
-        PIC_CUDA(cudaMemcpyAsync(S.oy, B.oy[0], n * 4, k, st));
-        PIC_CUDA(cudaMemcpyAsync(S.vx, B.vx[0], n * 4, k, st));
-        PIC_CUDA(cudaMemcpyAsync(S.vy, B.vy[0], n * 4, k, st));
-    } else {
-        PIC_CUDA(cudaMemcpyAsync(B.cell[0], S.cell, n * 4, k, st));
-        PIC_CUDA(cudaMemcpyAsync(B.ox[0], S.ox, n * 4, k, st));
-        PIC_CUDA(cudaMemcpyAsync(B.oy[0], S.oy, n * 4, k, st));
-        PIC_CUDA(cudaMemcpyAsync(B.vx[0], S.vx, n * 4, k, st));
-        PIC_CUDA(cudaMemcpyAsync(B.vy[0], S.vy, n * 4, k, st));
-    }
+    void *live[5] = {B.cell[0], B.ox[0], B.oy[0], B.vx[0], B.vy[0]};
+    void *kept[5] = {S.cell, S.ox, S.oy, S.vx, S.vy};
+    for (int k = 0; k < 5; ++k)
+        PIC_CUDA(cudaMemcpyAsync(save ? kept[k] : live[k], save ? live[k] : kept[k], n * 4,
+                                 cudaMemcpyDeviceToDevice, h->stream));
     return PIC_OK;
 }
 
@@ -200,89 +173,132 @@ pic_status adjoint_run(pic_handle *h, const pic_init_spec *spec, long long nstep
         return PIC_ERR_STATE;
     }
     const Geometry &g = h->g;
-    const size_t np = (size_t)h->sp[0].cap;
-    const long long n = h->sp[0].n;
+    SpeciesBuf &B = h->sp[0];
+    cudaStream_t st = h->stream;
+    const size_t np = (size_t)B.cap;
+    const long long n = B.n;
     const size_t ncell = (size_t)g.nx * g.ny, nk = (size_t)g.ny * g.nh;
     const double qm = c.species[0].q / c.species[0].m, dt = c.dt;
     const int K = (int)std::min<long long>(every, nsteps);
     const int nseg = (int)((nsteps + K - 1) / K);
     AdjWork W;
-    W.h = h;
-    std::vector<Snap> ck(nseg);
-    for (auto &S : ck) PIC_TRY(snap_alloc(W, S, np));
-    Snap fin;
-    PIC_TRY(snap_alloc(W, fin, np));
-    // ring of one segment: positions and fields per step
-    int32_t *rc = nullptr;
-    float *rox = nullptr, *roy = nullptr, *re = nullptr;
-    PIC_TRY(W.alloc(&rc, np * K));
-    PIC_TRY(W.alloc(&rox, np * K));
-    PIC_TRY(W.alloc(&roy, np * K));
-    PIC_TRY(W.alloc(&re, 2 * ncell * K));
-    float *ax = nullptr, *ay = nullptr, *avx = nullptr, *avy = nullptr, *gpl = nullptr, *psi = nullptr;
+    std::vector<Snap> ck(nseg - 1);  // state at the start of every segment but the last
+    Snap fin = {};                   // the final state (several segments)
+    std::vector<StepSlot> ring(K);   // positions and field of a segment's steps
+    KickArgs A = {};
+    float *gpl = nullptr, *psi = nullptr;
     float2 *gh = nullptr, *ph = nullptr;
-    PIC_TRY(W.alloc(&ax, np));
-    PIC_TRY(W.alloc(&ay, np));
-    PIC_TRY(W.alloc(&avx, np));
-    PIC_TRY(W.alloc(&avy, np));
-    PIC_TRY(W.alloc(&gpl, 2 * ncell));
-    PIC_TRY(W.alloc(&psi, ncell));
-    PIC_TRY(W.alloc(&gh, 2 * nk));
-    PIC_TRY(W.alloc(&ph, nk));
-    int dims[2] = {g.ny, g.nx};
-    PIC_CUFFT(cufftPlanMany(&W.r2c2, 2, dims, nullptr, 1, (int)ncell, nullptr, 1, (int)nk,
-                            CUFFT_R2C, 2));
-    PIC_CUFFT(cufftSetStream(W.r2c2, h->stream));
-    cudaStream_t st = h->stream;
-    SpeciesBuf &B = h->sp[0];
+    double *buf = nullptr;           // the gradients in id order
+    DevState *saved = nullptr;
+    auto layout = [&]() {
+        W.used = 0;
+        for (auto &S : ck) S = take_snap(W, np);
+        if (nseg > 1) fin = take_snap(W, np);
+        for (auto &S : ring) {
+            S.cell = W.take<int32_t>(np);
+            S.ox = W.take<float>(np);
+            S.oy = W.take<float>(np);
+            S.e = W.take<float>(2 * ncell);
+        }
+        A.ax = W.take<float>(np);
+        A.ay = W.take<float>(np);
+        A.avx = W.take<float>(np);
+        A.avy = W.take<float>(np);
+        gpl = W.take<float>(2 * ncell);
+        psi = W.take<float>(ncell);
+        gh = W.take<float2>(2 * nk);
+        ph = W.take<float2>(nk);
+        buf = W.take<double>(4 * (size_t)n);
+        saved = W.take<DevState>(1);
+    };
+    layout();
+    if (W.used <= ADJ_STAGE_MAX) {
+        PIC_TRY(ensure_stage(h, W.used));
+        W.base = (char *)h->stage;
+    } else {
+        PIC_CUDA(cudaMalloc(&W.own, W.used));
+        W.base = W.own;
+    }
+    layout();
+    if (!h->spectral) {
+        int dims[2] = {g.ny, g.nx};
+        PIC_CUFFT(cufftPlanMany(&W.r2c2, 2, dims, nullptr, 1, (int)ncell, nullptr, 1, (int)nk,
+                                CUFFT_R2C, 2));
+        PIC_CUFFT(cufftSetStream(W.r2c2, st));
+    }
+    const StepSlot live = {B.cell[0], B.ox[0], B.oy[0], h->e};
 
-    // ---- forward: prime, checkpoints every K steps, no re-sorting
+    // The live state and field into ring slot 0, then `steps` pushes, each
+    // from its slot to the next (the last one of the final segment back into
+    // the live arrays): nothing is copied for the ring but its first slot.
+    // (128^2 x 32 per cell, 40 steps every 10, through the torch binding: 11.0
+    // ms with every slot copied, the last segment run twice, forty-odd
+    // allocations and a cuFFT plan per call; 4.7 ms now.)
+    auto fill_ring = [&](int steps, bool last, int adv) -> pic_status {
+        PIC_CUDA(cudaMemcpyAsync(ring[0].cell, live.cell, np * 4, cudaMemcpyDeviceToDevice, st));
+        PIC_CUDA(cudaMemcpyAsync(ring[0].ox, live.ox, np * 4, cudaMemcpyDeviceToDevice, st));
+        PIC_CUDA(cudaMemcpyAsync(ring[0].oy, live.oy, np * 4, cudaMemcpyDeviceToDevice, st));
+        PIC_CUDA(cudaMemcpyAsync(ring[0].e, live.e, 2 * ncell * 4, cudaMemcpyDeviceToDevice, st));
+        for (int s = 0; s < steps; ++s) {
+            const StepSlot &to = last && s == steps - 1 ? live : ring[s + 1];
+            PIC_TRY(launch_push_slot(h, ring[s], to));
+            PIC_TRY(record_poisson(h, adv, to.e));
+        }
+        return PIC_OK;
+    };
+
+    // ---- forward: prime, checkpoints every K steps, the last segment into
+    // the ring, no re-sorting
     PIC_TRY(pic_prime_leapfrog(h));
-    for (int m = 0; m < nseg; ++m) {
+    if (!h->rho_clear) PIC_CUDA(cudaMemsetAsync(h->rho_fix, 0, ncell * 8, st));
+    for (int m = 0; m + 1 < nseg; ++m) {
         PIC_TRY(snap_copy(h, ck[m], true, np));
-        const long long s0 = (long long)m * K, s1 = std::min<long long>(nsteps, s0 + K);
-        for (long long s = s0; s < s1; ++s) {
-            PIC_CUDA(cudaMemsetAsync(h->rho_fix, 0, ncell * 8, st));
-            PIC_TRY(record_push_all(h, 0, true));
-            PIC_TRY(record_poisson(h));
+        for (int s = 0; s < K; ++s) {
+            PIC_TRY(record_push_all(h, 0, true, false));
+            PIC_TRY(record_poisson(h, ADV_PUSH | ADV_FIELD));
         }
     }
-    PIC_TRY(snap_copy(h, fin, true, np));
-    PIC_CUDA(cudaStreamSynchronize(st));
+    PIC_TRY(fill_ring((int)(nsteps - (long long)(nseg - 1) * K), true, ADV_PUSH | ADV_FIELD));
+    if (nseg > 1) PIC_TRY(snap_copy(h, fin, true, np));
     h->steps_host += nsteps;
     h->since_sort += (int)std::min<long long>(nsteps, 1 << 30);
-    pic_diag d;
-    PIC_TRY(pic_diagnostics(h, &d));
-    const double J = d.field_energy;
-    // the recompute passes below advance the step counter and the history;
-    // the device state of step nsteps is put back at the end
-    DevState saved;
-    PIC_CUDA(cudaMemcpy(&saved, h->dev, sizeof(DevState), cudaMemcpyDeviceToHost));
-    const size_t hist_bytes = 6 * (size_t)h->hist_cap * sizeof(double);
-    double *hist_saved;
-    PIC_TRY(W.alloc(&hist_saved, 6 * (size_t)h->hist_cap));
-    PIC_CUDA(cudaMemcpyAsync(hist_saved, h->hist, hist_bytes, cudaMemcpyDeviceToDevice, st));
+    // the diagnostics of step nsteps are kept apart from the passes below,
+    // which fold nothing into the history
+    PIC_CUDA(cudaMemcpyAsync(saved, h->dev, sizeof(DevState), cudaMemcpyDeviceToDevice, st));
 
-    AdjArgs A;
-    A.n = n;
-    A.nx = g.nx;
-    A.ny = g.ny;
-    A.inv_dx = (float)(1.0 / g.dx);
-    A.inv_dy = (float)(1.0 / g.dy);
-    A.q_over_dA = (float)(c.species[0].q / (g.dx * g.dy));
-    A.ax = ax;
-    A.ay = ay;
-    A.avx = avx;
-    A.avy = avy;
-    A.gx = gpl;
-    A.gy = gpl + ncell;
-    A.psi = psi;
+    AdjArgs G;
+    G.n = n;
+    G.nx = g.nx;
+    G.ny = g.ny;
+    G.inv_dx = (float)(1.0 / g.dx);
+    G.inv_dy = (float)(1.0 / g.dy);
+    G.q_over_dA = (float)(c.species[0].q / (g.dx * g.dy));
+    G.ax = A.ax;
+    G.ay = A.ay;
+    G.psi = psi;
+    KickGeo Q;
+    memset(&Q, 0, sizeof Q);
+    Q.G.nx = g.nx;
+    Q.G.ny = g.ny;
+    Q.G.tw = g.tw;
+    Q.G.th = g.th;
+    Q.G.hx = Q.G.hy = g.halo;
+    Q.G.wcx = g.wcx;
+    Q.G.wcy = g.wcy;
+    Q.gx = gpl;
+    Q.gy = gpl + ncell;
+    Q.inv_dx = G.inv_dx;
+    Q.inv_dy = G.inv_dy;
+    long long n4 = (n + 3) & ~3ll;
+    const unsigned nblk = (unsigned)((n4 + B.chunk - 1) / B.chunk);
+    const size_t kick_smem = kick_bytes(g.wcx, g.wcy);
     const int gp = grid_for(n, 256), gg = grid_for((long long)nk, 256);
     const float kx1 = (float)(2.0 * 3.14159265358979323846 / g.Lx);
     const float ky1 = (float)(2.0 * 3.14159265358979323846 / g.Ly);
     const float inv_eps0_n = (float)(1.0 / (c.eps0 * (double)ncell));
-    // psi = S^T g and a_x += (q/dA) sum psi grad w at the positions in A
-    auto solve_and_gather = [&]() -> pic_status {
+    // psi = S^T g (which leaves g clear) and a_x += (q/dA) sum psi grad w at
+    // the positions of a slot
+    auto solve_and_gather = [&](const StepSlot &S) -> pic_status {
         if (h->spectral) {
             PIC_TRY(launch_spectral_adjoint(h, gpl, gpl + ncell, gh, ph, psi));
         } else {
@@ -290,110 +306,106 @@ pic_status adjoint_run(pic_handle *h, const pic_init_spec *spec, long long nstep
             adj_kspace_kernel<<<gg, 256, 0, st>>>(gh, ph, g.nx, g.ny, g.nh, kx1, ky1, inv_eps0_n);
             PIC_CUDA(cudaGetLastError());
             PIC_CUFFT(cufftExecC2R(h->plan_c2r1, (cufftComplex *)ph, psi));
+            PIC_CUDA(cudaMemsetAsync(gpl, 0, 2 * ncell * 4, st));
         }
-        adj_gather_kernel<<<gp, 256, 0, st>>>(A);
-        PIC_CUDA(cudaGetLastError());
-        return PIC_OK;
+        G.cell = S.cell;
+        G.ox = S.ox;
+        G.oy = S.oy;
+        void *args[] = {&G};
+        return launch_dependent((const void *)adj_gather_kernel, gp, 256, 0, st, args);
     };
-    auto kick = [&](float C, float drift) -> pic_status {
-        A.C = (float)(C * qm);
-        A.drift_dt = drift;
-        PIC_CUDA(cudaMemsetAsync(gpl, 0, 2 * ncell * 4, st));
-        adj_kick_scatter_kernel<<<gp, 256, 0, st>>>(A);
-        PIC_CUDA(cudaGetLastError());
-        return solve_and_gather();
+    auto kick = [&](const StepSlot &S, float C, float drift) -> pic_status {
+        A.cell = S.cell;
+        A.ox = S.ox;
+        A.oy = S.oy;
+        Q.G.ex = S.e;
+        Q.G.ey = S.e + ncell;
+        Q.muc = (float)(C * qm);
+        Q.ddt = drift;
+        if (nblk) {
+            PIC_TRY(allow_dynamic_smem((const void *)adj_kick_kernel, kick_smem));
+            void *args[] = {&A, &Q, &B.anchor, &B.chunk, &n4};
+            PIC_TRY(launch_dependent((const void *)adj_kick_kernel, nblk, 256, kick_smem, st, args));
+        }
+        return solve_and_gather(S);
     };
 
     // ---- terminal condition: a_x = grad J(x_N)
-    PIC_CUDA(cudaMemsetAsync(ax, 0, np * 4, st));
-    PIC_CUDA(cudaMemsetAsync(ay, 0, np * 4, st));
-    PIC_CUDA(cudaMemsetAsync(avx, 0, np * 4, st));
-    PIC_CUDA(cudaMemsetAsync(avy, 0, np * 4, st));
+    PIC_CUDA(cudaMemsetAsync(A.ax, 0, np * 4, st));
+    PIC_CUDA(cudaMemsetAsync(A.ay, 0, np * 4, st));
+    PIC_CUDA(cudaMemsetAsync(A.avx, 0, np * 4, st));
+    PIC_CUDA(cudaMemsetAsync(A.avy, 0, np * 4, st));
     scale_planes_kernel<<<grid_for((long long)ncell, 256), 256, 0, st>>>(
         h->e, h->e + ncell, (float)(c.eps0 * g.dx * g.dy), gpl, gpl + ncell, (long long)ncell);
     PIC_CUDA(cudaGetLastError());
-    A.cell = B.cell[0];
-    A.ox = B.ox[0];
-    A.oy = B.oy[0];
-    PIC_TRY(solve_and_gather());
+    PIC_TRY(solve_and_gather(live));
 
-    // ---- backward over the segments, recomputing each into the ring
+    // ---- backward over the segments, recomputing each but the last into the ring
     for (int m = nseg - 1; m >= 0; --m) {
-        const long long s0 = (long long)m * K, s1 = std::min<long long>(nsteps, s0 + K);
-        PIC_TRY(snap_copy(h, ck[m], false, np));
-        PIC_TRY(deposit_now(h));
-        PIC_TRY(record_poisson(h));
-        for (long long s = s0; s < s1; ++s) {
-            const size_t r = (size_t)(s - s0);
-            PIC_CUDA(cudaMemcpyAsync(rc + r * np, B.cell[0], np * 4, cudaMemcpyDeviceToDevice, st));
-            PIC_CUDA(cudaMemcpyAsync(rox + r * np, B.ox[0], np * 4, cudaMemcpyDeviceToDevice, st));
-            PIC_CUDA(cudaMemcpyAsync(roy + r * np, B.oy[0], np * 4, cudaMemcpyDeviceToDevice, st));
-            PIC_CUDA(cudaMemcpyAsync(re + r * 2 * ncell, h->e, 2 * ncell * 4, cudaMemcpyDeviceToDevice, st));
-            if (s + 1 < s1) {
-                PIC_CUDA(cudaMemsetAsync(h->rho_fix, 0, ncell * 8, st));
-                PIC_TRY(record_push_all(h, 0, true));
-                PIC_TRY(record_poisson(h));
-            }
+        const int steps = (int)(std::min<long long>(nsteps, (long long)(m + 1) * K) - (long long)m * K);
+        if (m < nseg - 1) {
+            PIC_TRY(snap_copy(h, ck[m], false, np));
+            PIC_TRY(deposit_now(h));
+            PIC_TRY(record_poisson(h, 0));
+            PIC_TRY(fill_ring(steps - 1, false, 0));
         }
-        for (long long s = s1 - 1; s >= s0; --s) {
-            const size_t r = (size_t)(s - s0);
-            A.cell = rc + r * np;
-            A.ox = rox + r * np;
-            A.oy = roy + r * np;
-            A.ex = re + r * 2 * ncell;
-            A.ey = A.ex + ncell;
-            PIC_TRY(kick((float)dt, (float)dt));
-        }
+        for (int s = steps - 1; s >= 0; --s) PIC_TRY(kick(ring[s], (float)dt, (float)dt));
     }
     // ---- the priming kick v(-1/2) = v0 - (q/m) F(x0) dt/2 (ring slot 0 of segment 0)
-    A.cell = rc;
-    A.ox = rox;
-    A.oy = roy;
-    A.ex = re;
-    A.ey = re + ncell;
-    PIC_TRY(kick((float)(-0.5 * dt), 0.f));
+    PIC_TRY(kick(ring[0], (float)(-0.5 * dt), 0.f));
 
     // ---- outputs in id order
-    double *buf;
-    PIC_TRY(W.alloc(&buf, 4 * (size_t)n));
-    to_id_order_kernel<<<gp, 256, 0, st>>>(ax, ay, B.pid[0], n, buf, buf + n);
-    to_id_order_kernel<<<gp, 256, 0, st>>>(avx, avy, B.pid[0], n, buf + 2 * n, buf + 3 * n);
+    to_id_order_kernel<<<gp, 256, 0, st>>>(A.ax, A.ay, B.pid[0], n, buf, buf + n);
+    to_id_order_kernel<<<gp, 256, 0, st>>>(A.avx, A.avy, B.pid[0], n, buf + 2 * n, buf + 3 * n);
     PIC_CUDA(cudaGetLastError());
-    std::vector<double> hb(4 * (size_t)n);
-    PIC_CUDA(cudaMemcpyAsync(hb.data(), buf, hb.size() * 8, cudaMemcpyDeviceToHost, st));
-    PIC_CUDA(cudaStreamSynchronize(st));
-    if (gx0) std::copy(hb.begin(), hb.begin() + n, gx0);
-    if (gy0) std::copy(hb.begin() + n, hb.begin() + 2 * n, gy0);
-    if (gvx0) std::copy(hb.begin() + 2 * n, hb.begin() + 3 * n, gvx0);
-    if (gvy0) std::copy(hb.begin() + 3 * n, hb.begin() + 4 * n, gvy0);
+    // the load's derivatives need dJ/dx0, dJ/dy0 and dJ/dvx0 on the host
+    std::vector<double> own;
+    double *dst[4] = {gx0, gy0, gvx0, gvy0};
+    if (out && spec) {
+        int missing = 0;
+        for (int k = 0; k < 3; ++k) missing += dst[k] ? 0 : 1;
+        own.resize((size_t)missing * n);
+        double *p = own.data();
+        for (int k = 0; k < 3; ++k)
+            if (!dst[k]) {
+                dst[k] = p;
+                p += n;
+            }
+    }
+    for (int k = 0; k < 4; ++k)
+        if (dst[k])
+            PIC_CUDA(cudaMemcpyAsync(dst[k], buf + k * n, (size_t)n * 8, cudaMemcpyDeviceToHost, st));
+    std::vector<double> dA;
+    if (out && spec) {
+        dA.resize(2 * (size_t)n);
+        int lx = 0, ly = 0;
+        if (spec->layout == PIC_LOAD_LATTICE) PIC_TRY(lattice_dims(h, n, &lx, &ly));
+        PIC_TRY(launch_init_dA(h, spec, lx, ly, buf, buf + n));
+        PIC_CUDA(cudaMemcpyAsync(dA.data(), buf, dA.size() * 8, cudaMemcpyDeviceToHost, st));
+    }
+    // ---- leave the handle at step nsteps
+    if (nseg > 1) {
+        PIC_TRY(snap_copy(h, fin, false, np));
+        PIC_TRY(deposit_now(h));
+        PIC_TRY(record_poisson(h, 0));
+    }
+    PIC_CUDA(cudaMemcpyAsync(h->dev, saved, sizeof(DevState), cudaMemcpyDeviceToDevice, st));
+    pic_diag d;
+    PIC_TRY(pic_diagnostics(h, &d));  // waits for all of it
     if (out) {
-        out->J = J;
+        out->J = d.field_energy;
         out->dJ_dbeam_v = 0.0;
         out->dJ_damp = 0.0;
         if (spec) {
-            double sb = 0.0;
-            for (long long i = 0; i < n; ++i) sb += (i & 1) ? -hb[2 * n + i] : hb[2 * n + i];
-            out->dJ_dbeam_v = sb;  // vx carries +-beam_v by id parity
-            std::vector<double> dA(2 * (size_t)n);
-            double *dAd;
-            PIC_TRY(W.alloc(&dAd, 2 * (size_t)n));
-            int lx = 0, ly = 0;
-            if (spec->layout == PIC_LOAD_LATTICE) PIC_TRY(lattice_dims(h, n, &lx, &ly));
-            PIC_TRY(launch_init_dA(h, spec, lx, ly, dAd, dAd + n));
-            PIC_CUDA(cudaMemcpyAsync(dA.data(), dAd, dA.size() * 8, cudaMemcpyDeviceToHost, st));
-            PIC_CUDA(cudaStreamSynchronize(st));
-            double sa = 0.0;
-            for (long long i = 0; i < n; ++i) sa += hb[i] * dA[i] + hb[n + i] * dA[n + i];
+            double sb = 0.0, sa = 0.0;
+            for (long long i = 0; i < n; ++i) {
+                sb += (i & 1) ? -dst[2][i] : dst[2][i];  // vx carries +-beam_v by id parity
+                sa += dst[0][i] * dA[i] + dst[1][i] * dA[n + i];
+            }
+            out->dJ_dbeam_v = sb;
             out->dJ_damp = sa;
         }
     }
-    // ---- leave the handle at step nsteps
-    PIC_TRY(snap_copy(h, fin, false, np));
-    PIC_TRY(deposit_now(h));
-    PIC_TRY(record_poisson(h));
-    PIC_CUDA(cudaMemcpyAsync(h->dev, &saved, sizeof(DevState), cudaMemcpyHostToDevice, st));
-    PIC_CUDA(cudaMemcpyAsync(h->hist, hist_saved, hist_bytes, cudaMemcpyDeviceToDevice, st));
-    PIC_CUDA(cudaStreamSynchronize(st));
     return PIC_OK;
 }
 

@@ -233,6 +233,10 @@ void ens_free(pic_ensemble *E)
         if (G.c2r1) cufftDestroy(G.c2r1);
         if (G.tw) cudaFree(G.tw);
     }
+    for (int b = 0; b < 2; ++b) {
+        if (E->bounce[b]) cudaFreeHost(E->bounce[b]);
+        if (E->bounced[b]) cudaEventDestroy(E->bounced[b]);
+    }
     if (E->g_one) cudaGraphExecDestroy(E->g_one);
     if (E->g_period) cudaGraphExecDestroy(E->g_period);
     if (E->g_sortstep) cudaGraphExecDestroy(E->g_sortstep);

@@ -87,6 +87,10 @@ struct pic_ensemble {
     cudaGraphExec_t g_one = nullptr, g_period = nullptr, g_sortstep = nullptr;
     int since_sort = 0;
     bool ready = false;
+    // page-locked buffers of the gradients' export
+    static constexpr size_t BOUNCE = 4u << 20;
+    void *bounce[2] = {nullptr, nullptr};
+    cudaEvent_t bounced[2] = {nullptr, nullptr};
     // export staging
     double *stage = nullptr;
     size_t stage_n = 0;

@@ -65,79 +65,7 @@ __device__ __forceinline__ PushGeo adj_geo(const EnsRun &R, const float *e)
     return G;
 }
 
-// Sums v[0..7] over each maximal run of consecutive lanes with the same key
-// (particles are cell-sorted, so a warp holds few runs); true on the run's
-// first lane, which then holds the run's totals.  Every lane of the warp
-// must call it; key -1 marks a lane without a particle.  Lane i adds the
-// partial of lane i + o only while i + o is before the next run start.
-__device__ __forceinline__ bool warp_run_sum8(int key, float (&v)[8])
-{
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int prev = __shfl_up_sync(full, key, 1);
-    const bool head = lane == 0 || key != prev;
-    const unsigned heads = __ballot_sync(full, head);
-    const unsigned after = heads & (0xfffffffeu << lane);
-    const int seg_end = after ? __ffs(after) - 1 : 32;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const float t = __shfl_down_sync(full, v[k], o);
-            if (lane + o < seg_end) v[k] += t;
-        }
-    }
-    return head;
-}
-
-__device__ __forceinline__ void red_cell(float *gx, float *gy, int c, int nx, int ny, const float (&v)[8])
-{
-    const Cic w = cic_of(c, 0.f, 0.f, nx, ny);
-    atomicAdd(gx + w.i00, v[0]);
-    atomicAdd(gy + w.i00, v[1]);
-    atomicAdd(gx + w.i10, v[2]);
-    atomicAdd(gy + w.i10, v[3]);
-    atomicAdd(gx + w.i01, v[4]);
-    atomicAdd(gy + w.i01, v[5]);
-    atomicAdd(gx + w.i11, v[6]);
-    atomicAdd(gy + w.i11, v[7]);
-}
-
-// the same eight sums into the block's window (shared-memory float adds)
-// when the cell lies in it, else straight to the grid
-__device__ __forceinline__ void red_cell_win(const Window &W, int wcx, int wcy, float *gx, float *gy,
-                                             int c, int nx, int ny, const float (&v)[8])
-{
-    int dxl = (c & 0xFFFF) - W.wx0, dyl = (c >> 16) - W.wy0;
-    if (dxl < 0) dxl += nx;
-    if (dyl < 0) dyl += ny;
-    if (W.on && dxl < wcx && dyl < wcy) {
-        float *sx = reinterpret_cast<float *>(W.sLo), *sy = reinterpret_cast<float *>(W.sHi);
-        const int l = dyl * W.nwx + dxl;
-        atomicAdd(sx + l, v[0]);
-        atomicAdd(sy + l, v[1]);
-        atomicAdd(sx + l + 1, v[2]);
-        atomicAdd(sy + l + 1, v[3]);
-        atomicAdd(sx + l + W.nwx, v[4]);
-        atomicAdd(sy + l + W.nwx, v[5]);
-        atomicAdd(sx + l + W.nwx + 1, v[6]);
-        atomicAdd(sy + l + W.nwx + 1, v[7]);
-    } else {
-        red_cell(gx, gy, c, nx, ny, v);
-    }
-}
-
-// Drift adjoint, kick transpose (scatter of mu and local term) and, with
-// UNKICK, the reversal of the kick.  One push block of particles per CTA;
-// each lane owns four consecutive particles (128-bit loads), E comes from
-// the block's shared-memory window (global loads outside it).  Scatter
-// contributions are summed in registers over a lane's particles in one
-// cell, then over the warp's lanes in one cell (warp_run_sum8); the run's
-// first lane adds them to the block's window (the deposit window's two
-// planes, here as float x and y sums), which is flushed to the grid at the
-// end.  Cells outside the window go to the grid directly.  Window adds
-// without the warp sums measured 8% slower, global reductions without
-// the window 4% slower.
+// one push block of particles per CTA (adj_kick_block)
 template <bool UNKICK>
 __global__ void __launch_bounds__(256, 3)
 ens_adj_kick_kernel(EnsAdjArgs A, const SegBlock *__restrict__ blk, const EnsRun *__restrict__ runs,
@@ -146,117 +74,19 @@ ens_adj_kick_kernel(EnsAdjArgs A, const SegBlock *__restrict__ blk, const EnsRun
     extern __shared__ __align__(16) unsigned char smem[];
     const SegBlock b = blk[blockIdx.x];
     const EnsRun &R = runs[b.run];
-    const PushGeo G = adj_geo(R, A.e);
-    const Window W = setup_window(G, smem, anchor[blockIdx.x]);
-    load_window<true, false>(G, W);
-    if (W.on)
-        for (int i = threadIdx.x; i < W.nw; i += blockDim.x) W.sLo[i] = W.sHi[i] = 0u;
-    __syncthreads();
-    float *ggx = A.g + 2 * R.goff, *ggy = ggx + R.ncp;
-    const float qmdt = R.qm_dt, muc = cscale * R.qm_dt, ddt = dscale * R.dt;
-    const int nx = R.nx, ny = R.ny;
-    const long long end = b.base + b.count;  // a multiple of 4 from base
-    const long long lane4 = 4ll * (threadIdx.x & 31);
-    for (long long qw = b.base + 4ll * (threadIdx.x & ~31u); qw < end; qw += 4ll * blockDim.x) {
-        const long long q = qw + lane4;
-        const bool live = q < end;
-        int cc[4] = {-1, -1, -1, -1};
-        float ox[4], oy[4], ax[4], ay[4], avx[4], avy[4], vx[4], vy[4];
-        if (live) {
-            const int4 c4 = *reinterpret_cast<const int4 *>(A.cell + q);
-            const float4 a4 = *reinterpret_cast<const float4 *>(A.ox + q);
-            const float4 b4 = *reinterpret_cast<const float4 *>(A.oy + q);
-            const float4 x4 = *reinterpret_cast<const float4 *>(A.ax + q);
-            const float4 y4 = *reinterpret_cast<const float4 *>(A.ay + q);
-            const float4 u4 = *reinterpret_cast<const float4 *>(A.avx + q);
-            const float4 w4 = *reinterpret_cast<const float4 *>(A.avy + q);
-            cc[0] = c4.x, cc[1] = c4.y, cc[2] = c4.z, cc[3] = c4.w;
-            ox[0] = a4.x, ox[1] = a4.y, ox[2] = a4.z, ox[3] = a4.w;
-            oy[0] = b4.x, oy[1] = b4.y, oy[2] = b4.z, oy[3] = b4.w;
-            ax[0] = x4.x, ax[1] = x4.y, ax[2] = x4.z, ax[3] = x4.w;
-            ay[0] = y4.x, ay[1] = y4.y, ay[2] = y4.z, ay[3] = y4.w;
-            avx[0] = u4.x, avx[1] = u4.y, avx[2] = u4.z, avx[3] = u4.w;
-            avy[0] = w4.x, avy[1] = w4.y, avy[2] = w4.z, avy[3] = w4.w;
-            if (UNKICK) {
-                const float4 p4 = *reinterpret_cast<const float4 *>(A.vx + q);
-                const float4 r4 = *reinterpret_cast<const float4 *>(A.vy + q);
-                vx[0] = p4.x, vx[1] = p4.y, vx[2] = p4.z, vx[3] = p4.w;
-                vy[0] = r4.x, vy[1] = r4.y, vy[2] = r4.z, vy[3] = r4.w;
-            }
-        }
-        int gkey = -1;
-        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int c = cc[j];
-            const int cx = c & 0xFFFF, cy = c >> 16;
-            if (c < 0 || cx >= nx || cy >= ny) continue;
-            const float avxj = fmaf(ddt, ax[j], avx[j]), avyj = fmaf(ddt, ay[j], avy[j]);
-            const float mx = muc * avxj, my = muc * avyj;
-            const float gx = 1.f - ox[j], gy = 1.f - oy[j];
-            const float w00 = gx * gy, w10 = ox[j] * gy, w01 = gx * oy[j], w11 = ox[j] * oy[j];
-            float2 e00, e10, e01, e11;
-            int dxl = cx - W.wx0, dyl = cy - W.wy0;
-            if (dxl < 0) dxl += nx;
-            if (dyl < 0) dyl += ny;
-            if (W.on && dxl < G.wcx && dyl < G.wcy) {
-                const int l = dyl * W.nwx + dxl;
-                e00 = W.sE[l];
-                e10 = W.sE[l + 1];
-                e01 = W.sE[l + W.nwx];
-                e11 = W.sE[l + W.nwx + 1];
-            } else {
-                const Cic w = cic_of(c, 0.f, 0.f, nx, ny);
-                e00 = make_float2(G.ex[w.i00], G.ey[w.i00]);
-                e10 = make_float2(G.ex[w.i10], G.ey[w.i10]);
-                e01 = make_float2(G.ex[w.i01], G.ey[w.i01]);
-                e11 = make_float2(G.ex[w.i11], G.ey[w.i11]);
-            }
-            const float v[8] = {w00 * mx, w00 * my, w10 * mx, w10 * my,
-                                w01 * mx, w01 * my, w11 * mx, w11 * my};
-            if (gkey < 0) gkey = c;
-            if (c == gkey) {
-#pragma unroll
-                for (int k = 0; k < 8; ++k) acc[k] += v[k];
-            } else {
-                red_cell_win(W, G.wcx, G.wcy, ggx, ggy, c, nx, ny, v);
-            }
-            const float s00 = e00.x * mx + e00.y * my, s10 = e10.x * mx + e10.y * my;
-            const float s01 = e01.x * mx + e01.y * my, s11 = e11.x * mx + e11.y * my;
-            ax[j] += (gy * (s10 - s00) + oy[j] * (s11 - s01)) * R.inv_dx;
-            ay[j] += (gx * (s01 - s00) + ox[j] * (s11 - s10)) * R.inv_dy;
-            avx[j] = avxj;
-            avy[j] = avyj;
-            if (UNKICK) {  // the push's gather, then the kick taken back
-                const float Ex = gy * fmaf(gx, e00.x, ox[j] * e10.x) + oy[j] * fmaf(gx, e01.x, ox[j] * e11.x);
-                const float Ey = gy * fmaf(gx, e00.y, ox[j] * e10.y) + oy[j] * fmaf(gx, e01.y, ox[j] * e11.y);
-                vx[j] = fmaf(-qmdt, Ex, vx[j]);
-                vy[j] = fmaf(-qmdt, Ey, vy[j]);
-            }
-        }
-        if (warp_run_sum8(gkey, acc) && gkey >= 0) red_cell_win(W, G.wcx, G.wcy, ggx, ggy, gkey, nx, ny, acc);
-        if (live) {
-            *reinterpret_cast<float4 *>(A.ax + q) = make_float4(ax[0], ax[1], ax[2], ax[3]);
-            *reinterpret_cast<float4 *>(A.ay + q) = make_float4(ay[0], ay[1], ay[2], ay[3]);
-            *reinterpret_cast<float4 *>(A.avx + q) = make_float4(avx[0], avx[1], avx[2], avx[3]);
-            *reinterpret_cast<float4 *>(A.avy + q) = make_float4(avy[0], avy[1], avy[2], avy[3]);
-            if (UNKICK) {
-                *reinterpret_cast<float4 *>(A.vx + q) = make_float4(vx[0], vx[1], vx[2], vx[3]);
-                *reinterpret_cast<float4 *>(A.vy + q) = make_float4(vy[0], vy[1], vy[2], vy[3]);
-            }
-        }
-    }
-    if (!W.on) return;
-    __syncthreads();
-    const float *sx = reinterpret_cast<const float *>(W.sLo), *sy = reinterpret_cast<const float *>(W.sHi);
-    WindowWalk w(W);
-    for (int i = threadIdx.x; i < W.nw; i += blockDim.x, w.next(W)) {
-        const float fx = sx[i], fy = sy[i];
-        if (fx == 0.f && fy == 0.f) continue;
-        const size_t o = w.node(W, nx, ny);
-        if (fx != 0.f) atomicAdd(ggx + o, fx);
-        if (fy != 0.f) atomicAdd(ggy + o, fy);
-    }
+    pdl_wait();
+    pdl_trigger();
+    KickGeo K;
+    K.G = adj_geo(R, A.e);
+    K.gx = A.g + 2 * R.goff;
+    K.gy = K.gx + R.ncp;
+    K.qm_dt = R.qm_dt;
+    K.muc = cscale * R.qm_dt;
+    K.ddt = dscale * R.dt;
+    K.inv_dx = R.inv_dx;
+    K.inv_dy = R.inv_dy;
+    const KickArgs P = {A.cell, A.ox, A.oy, A.vx, A.vy, A.ax, A.ay, A.avx, A.avy};
+    adj_kick_block<UNKICK>(P, K, smem, b.base, b.base + b.count, anchor[blockIdx.x]);
 }
 
 // adjoint of the deposit: a_x += (q/dA) sum_m psi_m grad w_m (four
@@ -266,6 +96,8 @@ ens_adj_gather_kernel(EnsAdjArgs A, const SegBlock *__restrict__ blk, const EnsR
 {
     const SegBlock b = blk[blockIdx.x];
     const EnsRun &R = runs[b.run];
+    pdl_wait();
+    pdl_trigger();
     const float *psi = A.psi + R.goff;
     const long long end = b.base + b.count;
     for (long long q = b.base + 4ll * threadIdx.x; q < end; q += 4ll * blockDim.x) {
@@ -481,6 +313,36 @@ pic_status adj_plans(pic_ensemble *E)
     return PIC_OK;
 }
 
+// Device array to pageable host memory through two page-locked buffers, the
+// copy out of one beside the transfer into the other.  Into memory that the
+// caller has never touched (a fresh array) the driver's own copy faults page
+// by page: 330 MB of gradients took 140 ms, 38 ms through a vector that stayed
+// touched, 32 ms this way.
+pic_status export_array(pic_ensemble *E, const double *src, size_t n, double *dst)
+{
+    constexpr size_t PART = pic_ensemble::BOUNCE / sizeof(double);
+    if (!E->bounce[0])
+        for (int b = 0; b < 2; ++b) {
+            PIC_CUDA(cudaMallocHost(&E->bounce[b], pic_ensemble::BOUNCE));
+            PIC_CUDA(cudaEventCreateWithFlags(&E->bounced[b], cudaEventDisableTiming));
+        }
+    const size_t parts = (n + PART - 1) / PART;
+    for (size_t k = 0; k <= parts; ++k) {
+        if (k < parts) {
+            const size_t m = std::min(PART, n - k * PART);
+            PIC_CUDA(cudaMemcpyAsync(E->bounce[k & 1], src + k * PART, m * sizeof(double),
+                                     cudaMemcpyDeviceToHost, E->stream));
+            PIC_CUDA(cudaEventRecord(E->bounced[k & 1], E->stream));
+        }
+        if (k > 0) {
+            const size_t m = std::min(PART, n - (k - 1) * PART);
+            PIC_CUDA(cudaEventSynchronize(E->bounced[(k - 1) & 1]));
+            memcpy(dst + (k - 1) * PART, E->bounce[(k - 1) & 1], m * sizeof(double));
+        }
+    }
+    return PIC_OK;
+}
+
 }  // namespace
 
 pic_status ens_adjoint(pic_ensemble *E, const pic_init_spec *specs, long long nsteps, int every,
@@ -504,6 +366,8 @@ pic_status ens_adjoint(pic_ensemble *E, const pic_init_spec *specs, long long ns
     PIC_TRY(B.dalloc(&g, 2 * (size_t)E->nnodes));
     PIC_TRY(B.dalloc(&ghat, (size_t)E->nmodes));
     PIC_TRY(adj_plans(E));
+    size_t kick_smem = 0;
+    for (const EnsRun &R : E->runs) kick_smem = std::max(kick_smem, kick_bytes(R.wcx, R.wcy));
     std::vector<Ckpt> ck((size_t)nseg);  // ck[m-1]: state at step m K; ck[nseg-1]: final state
     int on_host = 0;
     for (auto &C : ck) PIC_TRY(ck_alloc(B, C, ns, &on_host));
@@ -552,22 +416,19 @@ pic_status ens_adjoint(pic_ensemble *E, const pic_init_spec *specs, long long ns
             PIC_CUFFT(cufftExecC2R(G.c2r1, (cufftComplex *)(E->rhohat + R.khoff), E->rho + R.goff));
         }
         set_arrays();
-        ens_adj_gather_kernel<<<E->npush, 256, 0, st>>>(A, E->push_blk, E->d_runs);
-        PIC_CUDA(cudaGetLastError());
+        void *args[] = {&A, &E->push_blk, &E->d_runs};
+        if (E->npush)
+            PIC_TRY(launch_dependent((const void *)ens_adj_gather_kernel, (unsigned)E->npush, 256, 0, st, args));
         return PIC_OK;
     };
     auto kick = [&](bool unkick, float cscale, float dscale) -> pic_status {
         PIC_CUDA(cudaMemsetAsync(g, 0, sizeof(float) * 2 * (size_t)E->nnodes, st));
         set_arrays();
-        PIC_TRY(allow_dynamic_smem((const void *)ens_adj_kick_kernel<true>, E->push_smem));
-        PIC_TRY(allow_dynamic_smem((const void *)ens_adj_kick_kernel<false>, E->push_smem));
-        if (unkick)
-            ens_adj_kick_kernel<true><<<E->npush, 256, E->push_smem, st>>>(A, E->push_blk, E->d_runs,
-                                                                       E->anchor, cscale, dscale);
-        else
-            ens_adj_kick_kernel<false><<<E->npush, 256, E->push_smem, st>>>(A, E->push_blk, E->d_runs,
-                                                                        E->anchor, cscale, dscale);
-        PIC_CUDA(cudaGetLastError());
+        const void *k = unkick ? (const void *)ens_adj_kick_kernel<true>
+                               : (const void *)ens_adj_kick_kernel<false>;
+        PIC_TRY(allow_dynamic_smem(k, kick_smem));
+        void *args[] = {&A, &E->push_blk, &E->d_runs, &E->anchor, &cscale, &dscale};
+        if (E->npush) PIC_TRY(launch_dependent(k, (unsigned)E->npush, 256, kick_smem, st, args));
         return solve_gather();
     };
     auto quad = [&](int b) {
@@ -630,7 +491,6 @@ pic_status ens_adjoint(pic_ensemble *E, const pic_init_spec *specs, long long ns
     PIC_TRY(B.dalloc(&dA, 2 * (size_t)nmax));
     std::vector<long long> first(nr, 0);
     for (int r = 1; r < nr; ++r) first[r] = first[r - 1] + specs[r - 1].n;
-    std::vector<double> host;
     for (int r = 0; r < nr; ++r) {
         const int sidx = E->slot_of[r];
         const EnsRun &R = E->runs[sidx];
@@ -653,12 +513,9 @@ pic_status ens_adjoint(pic_ensemble *E, const pic_init_spec *specs, long long ns
             amp_kind ? dA : nullptr, amp_kind ? dA + R.n : nullptr, d_acc + 2 * r);
         PIC_CUDA(cudaGetLastError());
         if (want && R.n) {
-            host.resize(4 * (size_t)R.n);
-            PIC_CUDA(cudaMemcpyAsync(host.data(), stage, host.size() * 8, cudaMemcpyDeviceToHost, st));
-            PIC_CUDA(cudaStreamSynchronize(st));
             double *dst[4] = {gx0, gy0, gvx0, gvy0};
             for (int k = 0; k < 4; ++k)
-                if (dst[k]) std::copy(host.begin() + k * R.n, host.begin() + (k + 1) * R.n, dst[k] + first[r]);
+                if (dst[k]) PIC_TRY(export_array(E, stage + k * R.n, (size_t)R.n, dst[k] + first[r]));
         }
     }
     PIC_CUDA(cudaMemcpyAsync(acc.data(), d_acc, 16 * (size_t)nr, cudaMemcpyDeviceToHost, st));

@@ -296,15 +296,15 @@ static void update_mean(pic_handle *h)
 // ---------------------------------------------------------------- stages
 // adv: the diagnostics folds that ride on the solve (ADV_FIELD, or ADV_PUSH |
 // ADV_FIELD when the particle pass left its fold to it)
-pic_status record_poisson(pic_handle *h, int adv)
+pic_status record_poisson(pic_handle *h, int adv, float *e)
 {
     if (h->spectral) {
-        PIC_TRY(launch_spectral(h, adv));
+        PIC_TRY(launch_spectral(h, adv, e));
     } else {
         PIC_TRY(launch_convert(h));
         PIC_CUFFT(cufftExecR2C(h->plan_r2c, h->rho, (cufftComplex *)h->rhohat));
         PIC_TRY(launch_kspace(h, false, nullptr, adv));
-        PIC_CUFFT(cufftExecC2R(h->plan_c2r2, (cufftComplex *)h->ehat, h->e));
+        PIC_CUFFT(cufftExecC2R(h->plan_c2r2, (cufftComplex *)h->ehat, e ? e : h->e));
     }
     h->rho_clear = true;
     return PIC_OK;

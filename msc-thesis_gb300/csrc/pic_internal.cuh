@@ -257,6 +257,15 @@ namespace pic {
 // ------------------------------------------------------------------ launchers
 // pic_push.cu
 pic_status launch_push(pic_handle *h, int s, int src, bool deposit, float dt_scale);
+// positions and field of one step of species 0, kept by the adjoint
+struct StepSlot {
+    int32_t *cell;
+    float *ox, *oy;
+    float *e;  // Ex plane, then Ey
+};
+// one push with deposit of species 0 from the positions and field of `in` to
+// the positions of `out`; velocities in place
+pic_status launch_push_slot(pic_handle *h, const StepSlot &in, const StepSlot &out);
 // lets `kernel` take `bytes` of dynamic shared memory (above the default 48 KB)
 pic_status allow_dynamic_smem(const void *kernel, size_t bytes);
 pic_status launch_deposit(pic_handle *h, int s);
@@ -272,11 +281,12 @@ bool spectral_size_ok(int nx, int ny);
 bool spectral_wanted(int nx, int ny);
 pic_status spectral_twiddles(int nx, int ny, float2 **tw);  // cudaMalloc'd tables
 // convert + solve, rho_fix cleared, diagnostics folds `adv` (0: none)
-pic_status launch_spectral(pic_handle *h, int adv);
+// (e: field planes to write, nullptr: the handle's)
+pic_status launch_spectral(pic_handle *h, int adv, float *e = nullptr);
 // the adjoint solve psi = S^T g (gx, gy -> psi) on a handle with h->spectral;
-// gh (2 ny nh) and ph (ny nh) are scratch
-pic_status launch_spectral_adjoint(pic_handle *h, const float *gx, const float *gy, float2 *gh,
-                                   float2 *ph, float *psi);
+// gx and gy are cleared; gh (2 ny nh) and ph (ny nh) are scratch
+pic_status launch_spectral_adjoint(pic_handle *h, float *gx, float *gy, float2 *gh, float2 *ph,
+                                   float *psi);
 struct EnsRun;
 // convert + solve of runs [first, first + count) of an ensemble's run table
 // (one grid size; grids at each run's offsets), rho_fix cleared, the folds
@@ -356,7 +366,8 @@ int device_sms();  // multiprocessors of the current device (cached; 152 if unkn
 unsigned sort_grid(long long chunks, int per_sm);  // sort blocks: at most the resident ones
 
 // pic_handle.cu stages used by other host files
-pic_status record_poisson(pic_handle *h, int adv = ADV_FIELD);
+// (e: field planes to write, nullptr: the handle's)
+pic_status record_poisson(pic_handle *h, int adv = ADV_FIELD, float *e = nullptr);
 pic_status record_push_all(pic_handle *h, int src, bool deposit, bool fold = true);
 pic_status deposit_now(pic_handle *h);
 pic_status refresh(pic_handle *h);

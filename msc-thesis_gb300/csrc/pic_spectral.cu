@@ -59,7 +59,7 @@ struct SpecArgs {
     // spectra in S and Sy, psi^ after the inverse along y in Tx; the inverse
     // rows take rows y ys and y ys + yo of Tx and Ty into ex and ey (ys = 1,
     // yo = 0 for the field; 2 and 1 for psi, two rows per transform)
-    const float *gx, *gy;
+    float *gx, *gy;  // cleared by the columns
     float2 *Sy;
     int ys, yo;
     int pairs, cols, rows;  // transforms (row pairs or rows), columns, rows per block
@@ -87,9 +87,9 @@ __device__ __forceinline__ SpecArgs block_args(const SpecArgs &P)
         A.rho = P.rho + R.goff;
         A.S = P.S + R.khoff;
         A.Tx = P.Tx + R.khoff;
-        A.Ty = P.Tx + R.khoff + R.nk;
+        A.Ty = A.Tx + R.nk;
         A.ex = P.ex + 2 * R.goff;
-        A.ey = P.ex + 2 * R.goff + R.ncp;
+        A.ey = A.ex + R.ncp;
         A.mean_fix = R.mean_fix;
         A.scale = R.rho_scale;
         A.kx1 = R.kx1;
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(256) spec_rows_fwd_kernel(SpecArgs P)
         const size_t r0 = (size_t)(blockIdx.x * A.pairs + f) * NX;
 #pragma unroll
         for (int k = 0; k < fft::E; ++k)
-            v[0][k] = make_float2(__ldg(A.gx + r0 + t + k * TP), __ldg(A.gy + r0 + t + k * TP));
+            v[0][k] = make_float2(A.gx[r0 + t + k * TP], A.gy[r0 + t + k * TP]);
     } else {
         // all loads first (the density is read-only here), then the
         // conversions and the float density's stores
@@ -219,6 +219,13 @@ __global__ void __launch_bounds__(256, 2) spec_cols_kernel(SpecArgs P)
         const int n2 = (A.nx << LGY) >> 1, stride = gridDim.x * blockDim.x;
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n2; i += stride)
             reinterpret_cast<ulonglong2 *>(A.rho_fix)[i] = make_ulonglong2(0ull, 0ull);
+    } else {
+        // the scatter planes, transformed by the forward rows, likewise
+        const int n4 = (A.nx << LGY) >> 2, stride = gridDim.x * blockDim.x;
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride) {
+            reinterpret_cast<float4 *>(A.gx)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            reinterpret_cast<float4 *>(A.gy)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
     }
     // forward transform of column `src` along y, left in natural order in `bs`
     auto forward = [&](const float2 *src, float2 *bs) {
@@ -482,7 +489,7 @@ static pic_status launch_kernels(SpecArgs &A, int batch, cudaStream_t st, bool a
     return launch_dependent(kc, dim3(nc / A.rows + fold, nb), dim3(A.rows * tpx), mc, st, args);
 }
 
-pic_status launch_spectral(pic_handle *h, int adv)
+pic_status launch_spectral(pic_handle *h, int adv, float *e)
 {
     const Geometry &g = h->g;
     SpecArgs A;
@@ -492,8 +499,8 @@ pic_status launch_spectral(pic_handle *h, int adv)
     A.S = h->rhohat;
     A.Tx = h->ehat;
     A.Ty = h->ehat + (size_t)g.nh * g.ny;
-    A.ex = h->e;
-    A.ey = h->e + (size_t)g.nx * g.ny;
+    A.ex = e ? e : h->e;
+    A.ey = A.ex + (size_t)g.nx * g.ny;
     A.nx = g.nx;
     A.ny = g.ny;
     A.nh = g.nh;
@@ -545,8 +552,8 @@ pic_status launch_spectral_runs(const EnsRun *runs, int first, int count, int nx
 
 // psi = S^T g on a power-of-two handle: gx, gy (ncell each) -> psi; gh
 // (2 ny nh) and ph (ny nh) are scratch
-pic_status launch_spectral_adjoint(pic_handle *h, const float *gx, const float *gy, float2 *gh,
-                                   float2 *ph, float *psi)
+pic_status launch_spectral_adjoint(pic_handle *h, float *gx, float *gy, float2 *gh, float2 *ph,
+                                   float *psi)
 {
     const Geometry &g = h->g;
     SpecArgs A;
