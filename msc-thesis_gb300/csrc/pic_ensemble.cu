@@ -543,11 +543,10 @@ pic_status ens_poisson(pic_ensemble *E, int adv)
 {
     cudaStream_t st = E->stream;
     if (E->spectral) {
-        for (auto &G : E->groups)
-            PIC_TRY(launch_spectral_runs(E->d_runs, G.first, G.count, G.nx, G.ny, E->rho_fix,
-                                         E->rho, E->rhohat, E->ehat, E->e, G.tw, E->dev, E->hist,
-                                         E->hist_cap, adv, st));
-        return PIC_OK;
+        std::vector<SpecGroup> groups;
+        for (auto &G : E->groups) groups.push_back(SpecGroup{G.nx, G.ny, G.first, G.count, G.tw});
+        return launch_spectral_runs(E->d_runs, groups.data(), (int)groups.size(), E->rho_fix, E->rho,
+                                    E->rhohat, E->ehat, E->e, E->dev, E->hist, E->hist_cap, adv, st);
     }
     ens_convert_kernel<<<E->nnode_blk, 256, 0, st>>>(E->rho_fix, E->rho, E->node_blk, E->d_runs, E->dev);
     PIC_CUDA(cudaGetLastError());

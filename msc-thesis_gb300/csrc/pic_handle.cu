@@ -314,10 +314,15 @@ pic_status record_poisson(pic_handle *h, int adv, float *e)
 // buffer 1.  A DSMC species collides before its push; MCC follows the push.
 pic_status record_push_all(pic_handle *h, int src, bool deposit, bool fold)
 {
+    bool pushed = false;  // the last launch was another species' push
     for (int s = 0; s < h->cfg.nspecies; ++s) {
         if (!h->sp[s].cap) continue;
-        if (h->dsmc.on && s == h->dsmc.s) PIC_TRY(launch_ntc(h, src));
-        PIC_TRY(launch_push(h, s, src, deposit, 1.0f));
+        if (h->dsmc.on && s == h->dsmc.s) {
+            PIC_TRY(launch_ntc(h, src));
+            pushed = false;
+        }
+        PIC_TRY(launch_push(h, s, src, deposit, 1.0f, pushed));
+        pushed = true;
     }
     if (fold) PIC_TRY(launch_advance(h, ADV_PUSH));
     if (h->mcc.on) PIC_TRY(launch_mcc(h));

@@ -118,6 +118,15 @@ enum : uint32_t {
 // solve's kernels (four kernels a step instead of five and a memset), 128^2 x
 // 100 per cell went from 52.7 to 48.6 us a step, a step called stage by stage
 // on 64^2 x 16 from 80.7 to 60.2 us, 2048^2 x 32 from 1.216 to 1.208 ms.
+//
+// Kernels of one stage that do not depend on each other (the pushes of several
+// species, a solve stage of several grid sizes) overlap: all but the first
+// are "late", they do not wait at their start but at their end.  The first
+// one triggers after its own wait, so what came before the stage is complete
+// when a late kernel starts; the wait at the end keeps the rule above.  A
+// late kernel has not passed a wait that would discard stale lines of the
+// first-level cache, so it loads what earlier kernels wrote from L2
+// (ld.global.cg).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger()
 {
@@ -256,7 +265,8 @@ namespace pic {
 
 // ------------------------------------------------------------------ launchers
 // pic_push.cu
-pic_status launch_push(pic_handle *h, int s, int src, bool deposit, float dt_scale);
+// (late: right after another species' push, with which it may overlap)
+pic_status launch_push(pic_handle *h, int s, int src, bool deposit, float dt_scale, bool late = false);
 // positions and field of one step of species 0, kept by the adjoint
 struct StepSlot {
     int32_t *cell;
@@ -289,12 +299,16 @@ pic_status launch_spectral_adjoint(pic_handle *h, float *gx, float *gy, float2 *
                                    float *psi);
 struct EnsRun;
 // convert + solve of runs [first, first + count) of an ensemble's run table
-// (one grid size; grids at each run's offsets), rho_fix cleared, the folds
-// `adv` of each run into its history ring
-pic_status launch_spectral_runs(const EnsRun *runs, int first, int count, int nx, int ny,
+// for every group (one grid size each; grids at each run's offsets), rho_fix
+// cleared, the folds `adv` of each run into its history ring
+struct SpecGroup {
+    int nx, ny, first, count;
+    const float2 *tw;
+};
+pic_status launch_spectral_runs(const EnsRun *runs, const SpecGroup *groups, int ngroups,
                                 unsigned long long *rho_fix, float *rho, float2 *rhohat,
-                                float2 *ehat, float *e, const float2 *tw, DevState *devs,
-                                double *hist, int hist_cap, int adv, cudaStream_t st);
+                                float2 *ehat, float *e, DevState *devs, double *hist, int hist_cap,
+                                int adv, cudaStream_t st);
 // pic_sort.cu
 pic_status launch_sort(pic_handle *h, int s, bool counts_kept = false, int from = 0);
 pic_status launch_recount(pic_handle *h, int s);

@@ -125,6 +125,14 @@ __device__ __forceinline__ Window setup_window(const PushGeo &A, unsigned char *
     return W;
 }
 
+// A value that an earlier kernel of the chain wrote: a late kernel (see
+// pdl_wait) reads it from L2.
+template <bool LATE, class T>
+__device__ __forceinline__ T ld(const T *p)
+{
+    return LATE ? __ldcg(p) : *p;
+}
+
 // Walks the window's nodes i = threadIdx.x, threadIdx.x + blockDim.x, ...
 // with their grid node (gx, gy), advanced incrementally (the divisions run
 // once per thread, not once per node).
@@ -156,7 +164,7 @@ struct WindowWalk {
     }
 };
 
-template <bool GATHER, bool DEPOSIT>
+template <bool GATHER, bool DEPOSIT, bool LATE = false>
 __device__ __forceinline__ void load_window(const PushGeo &A, const Window &W)
 {
     if (!W.on) return;
@@ -164,7 +172,7 @@ __device__ __forceinline__ void load_window(const PushGeo &A, const Window &W)
         WindowWalk w(W);
         for (int i = threadIdx.x; i < W.nw; i += blockDim.x, w.next(W)) {
             const size_t g = w.node(W, A.nx, A.ny);
-            W.sE[i] = make_float2(A.ex[g], A.ey[g]);
+            W.sE[i] = make_float2(ld<LATE>(A.ex + g), ld<LATE>(A.ey + g));
         }
     }
     if (DEPOSIT) {  // 8-byte stores (the moments start on 8 bytes)
@@ -385,7 +393,7 @@ __device__ __forceinline__ int wrap_cell(int v, int n)
 // window coordinates and fixed-point offsets to `deposit`.  One branch for
 // all that a drift makes rare (an offset rounded up to 1, a cell across the
 // boundary).
-template <bool GATHER, bool DEPOSIT, bool MOVE, class F>
+template <bool GATHER, bool DEPOSIT, bool MOVE, bool LATE, class F>
 __device__ __forceinline__ void push_one(const PushGeo &A, const Window &W, int &cell, float &x,
                                          float &y, float &u, float &v, float &ke, float &px,
                                          float &py, F &&deposit)
@@ -410,10 +418,10 @@ __device__ __forceinline__ void push_one(const PushGeo &A, const Window &W, int 
             const int cy1 = (cy + 1 == ny) ? 0 : cy + 1;
             const int i00 = cy * nx + cx, i10 = cy * nx + cx1;
             const int i01 = cy1 * nx + cx, i11 = cy1 * nx + cx1;
-            e00 = make_float2(A.ex[i00], A.ey[i00]);
-            e10 = make_float2(A.ex[i10], A.ey[i10]);
-            e01 = make_float2(A.ex[i01], A.ey[i01]);
-            e11 = make_float2(A.ex[i11], A.ey[i11]);
+            e00 = make_float2(ld<LATE>(A.ex + i00), ld<LATE>(A.ey + i00));
+            e10 = make_float2(ld<LATE>(A.ex + i10), ld<LATE>(A.ey + i10));
+            e01 = make_float2(ld<LATE>(A.ex + i01), ld<LATE>(A.ey + i01));
+            e11 = make_float2(ld<LATE>(A.ex + i11), ld<LATE>(A.ey + i11));
         }
         const float Ex = gy * fmaf(gx, e00.x, ox * e10.x) + oy * fmaf(gx, e01.x, ox * e11.x);
         const float Ey = gy * fmaf(gx, e00.y, ox * e10.y) + oy * fmaf(gx, e01.y, ox * e11.y);
@@ -468,14 +476,14 @@ __device__ __forceinline__ void push_one(const PushGeo &A, const Window &W, int 
 // per step (chunk 16384; with the slow slots out of line and one address per
 // quad and per deposit); collected per quad as before 1.077, with spills up to
 // 1.211.
-template <bool GATHER, bool DEPOSIT, bool MOVE>
+template <bool GATHER, bool DEPOSIT, bool MOVE, bool LATE>
 __device__ __forceinline__ void push_four(const PushGeo &A, const Window &W, int (&cc)[4],
                                           float (&xo)[4], float (&yo)[4], float (&xv)[4],
                                           float (&yv)[4], float &ke, float &px, float &py)
 {
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-        push_one<GATHER, DEPOSIT, MOVE>(A, W, cc[j], xo[j], yo[j], xv[j], yv[j], ke, px, py,
+        push_one<GATHER, DEPOSIT, MOVE, LATE>(A, W, cc[j], xo[j], yo[j], xv[j], yv[j], ke, px, py,
                                         [&](int cx, int cy, int dxl, int dyl, unsigned fx, unsigned fy) {
             deposit_group(A, W, cx, cy, dxl, dyl, 1u, fx, fy, (unsigned long long)fx * fy);
         });
@@ -484,7 +492,7 @@ __device__ __forceinline__ void push_four(const PushGeo &A, const Window &W, int
 // Four slots of which some are empty or corrupt (the array's last quad): the
 // live ones one at a time through push_one, from local memory, so that the
 // code that nearly every quad runs stays small.
-template <bool GATHER, bool DEPOSIT, bool MOVE>
+template <bool GATHER, bool DEPOSIT, bool MOVE, bool LATE>
 __device__ __forceinline__ void push_slots(const PushGeo &A, const Window &W, int (&cc)[4],
                                            float (&xo)[4], float (&yo)[4], float (&xv)[4],
                                            float (&yv)[4], float &ke, float &px, float &py, bool &bad)
@@ -504,7 +512,7 @@ __device__ __forceinline__ void push_slots(const PushGeo &A, const Window &W, in
             atomicOr(&A.dev->err, (unsigned)PIC_DEVERR_CELL);
             continue;
         }
-        push_one<GATHER, DEPOSIT, MOVE>(A, W, c[j], p[0][j], p[1][j], p[2][j], p[3][j], ke, px, py,
+        push_one<GATHER, DEPOSIT, MOVE, LATE>(A, W, c[j], p[0][j], p[1][j], p[2][j], p[3][j], ke, px, py,
                                         [&](int cx, int cy, int dxl, int dyl, unsigned fx, unsigned fy) {
             deposit_group(A, W, cx, cy, dxl, dyl, 1u, fx, fy, (unsigned long long)fx * fy);
         });
@@ -524,6 +532,7 @@ __device__ __forceinline__ T &at(P *p, unsigned o)
     return *reinterpret_cast<T *>(reinterpret_cast<char *>(const_cast<std::remove_const_t<P> *>(p)) + o);
 }
 
+template <bool LATE>
 __device__ __forceinline__ void store_quad(const PushArgs &A, long long base, unsigned o,
                                            const int (&cc)[4], const float (&xo)[4],
                                            const float (&yo)[4], const float (&xv)[4],
@@ -534,8 +543,8 @@ __device__ __forceinline__ void store_quad(const PushArgs &A, long long base, un
     at<float4>(A.oyout + base, o) = make_float4(yo[0], yo[1], yo[2], yo[3]);
     at<float4>(A.vxout + base, o) = make_float4(xv[0], xv[1], xv[2], xv[3]);
     at<float4>(A.vyout + base, o) = make_float4(yv[0], yv[1], yv[2], yv[3]);
-    if (A.pidin) at<uint4>(A.pidout + base, o) = at<uint4>(A.pidin + base, o);
-    if (A.vzin) at<float4>(A.vzout + base, o) = at<float4>(A.vzin + base, o);
+    if (A.pidin) at<uint4>(A.pidout + base, o) = ld<LATE>(&at<uint4>(A.pidin + base, o));
+    if (A.vzin) at<float4>(A.vzout + base, o) = ld<LATE>(&at<float4>(A.vzin + base, o));
 }
 
 // end of a block: diagnostics reduction, error flags, window flush
@@ -601,13 +610,13 @@ __device__ __forceinline__ void finish_block(const PushGeo &A, const Window &W, 
 // Thread t owns the quads base + 4t + 4k blockDim.x; the loop runs while any
 // lane of the warp has a quad, so that the warp stays converged for AGG.
 // !MOVE: a deposit of the particles in place; nothing is stored.
-template <bool GATHER, bool DEPOSIT, bool AGG, bool MOVE = true>
+template <bool GATHER, bool DEPOSIT, bool AGG, bool MOVE = true, bool LATE = false>
 __device__ __forceinline__ void push_block(const PushArgs &A, const PushGeo &G, unsigned char *smem,
                                            long long base, long long end, int anc)
 {
     const Window W = setup_window(G, smem, anc);
     double *sAcc = reinterpret_cast<double *>(smem + window_bytes(G.wcx, G.wcy));
-    load_window<GATHER, DEPOSIT>(G, W);
+    load_window<GATHER, DEPOSIT, LATE>(G, W);
     if (threadIdx.x < 3) sAcc[threadIdx.x] = 0.0;
     __syncthreads();
 
@@ -631,20 +640,20 @@ __device__ __forceinline__ void push_block(const PushArgs &A, const PushGeo &G, 
             asm volatile("prefetch.global.L2 [%0];" ::"l"(&at<char>(A.vxin + base, on)));
             asm volatile("prefetch.global.L2 [%0];" ::"l"(&at<char>(A.vyin + base, on)));
         }
-        // plain (coherent) loads: with an in-place pass the same addresses are stored below
+        // coherent loads (with an in-place pass the same addresses are stored below)
         int cc[4] = {-1, -1, -1, -1};
         float xo[4] = {0.f, 0.f, 0.f, 0.f}, yo[4] = {0.f, 0.f, 0.f, 0.f};
         float xv[4] = {0.f, 0.f, 0.f, 0.f}, yv[4] = {0.f, 0.f, 0.f, 0.f};
         if (live) {
-            const int4 c4 = at<int4>(A.cin + base, o);
-            const float4 a4 = at<float4>(A.oxin + base, o);
-            const float4 b4 = at<float4>(A.oyin + base, o);
+            const int4 c4 = ld<LATE>(&at<int4>(A.cin + base, o));
+            const float4 a4 = ld<LATE>(&at<float4>(A.oxin + base, o));
+            const float4 b4 = ld<LATE>(&at<float4>(A.oyin + base, o));
             cc[0] = c4.x, cc[1] = c4.y, cc[2] = c4.z, cc[3] = c4.w;
             xo[0] = a4.x, xo[1] = a4.y, xo[2] = a4.z, xo[3] = a4.w;
             yo[0] = b4.x, yo[1] = b4.y, yo[2] = b4.z, yo[3] = b4.w;
             if (MOVE) {
-                const float4 u4 = at<float4>(A.vxin + base, o);
-                const float4 v4 = at<float4>(A.vyin + base, o);
+                const float4 u4 = ld<LATE>(&at<float4>(A.vxin + base, o));
+                const float4 v4 = ld<LATE>(&at<float4>(A.vyin + base, o));
                 xv[0] = u4.x, xv[1] = u4.y, xv[2] = u4.z, xv[3] = u4.w;
                 yv[0] = v4.x, yv[1] = v4.y, yv[2] = v4.z, yv[3] = v4.w;
             }
@@ -657,11 +666,11 @@ __device__ __forceinline__ void push_block(const PushArgs &A, const PushGeo &G, 
             for (int j = 0; j < 4; ++j)
                 whole = whole && (cc[j] & 0xFFFF) < G.nx && (unsigned)(cc[j] >> 16) < (unsigned)G.ny;
             if (whole)
-                push_four<GATHER, DEPOSIT, MOVE>(G, W, cc, xo, yo, xv, yv, ke, px, py);
+                push_four<GATHER, DEPOSIT, MOVE, LATE>(G, W, cc, xo, yo, xv, yv, ke, px, py);
             else if (live)
-                push_slots<GATHER, DEPOSIT, MOVE>(G, W, cc, xo, yo, xv, yv, ke, px, py, bad);
+                push_slots<GATHER, DEPOSIT, MOVE, LATE>(G, W, cc, xo, yo, xv, yv, ke, px, py, bad);
         }
-        if (MOVE && live) store_quad(A, base, o, cc, xo, yo, xv, yv);
+        if (MOVE && live) store_quad<LATE>(A, base, o, cc, xo, yo, xv, yv);
     }
     // a non-finite (or overflowing) velocity makes the sum of squares non-finite
     if (MOVE) bad |= !(fabsf(ke) <= 3.0e38f);
