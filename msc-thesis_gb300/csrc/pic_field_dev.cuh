@@ -59,53 +59,63 @@ __device__ __forceinline__ KMode kspace_mode(float2 r, int mx, int my, int nx, i
     return K;
 }
 
-// Sum of an accumulator over its slots, which are cleared; threads
-// 0..lanes-1 call it (a power of two, at most 32).
-template <class T>
-__device__ __forceinline__ T fold_slots(T *acc, int lanes)
-{
-    const unsigned mask = lanes >= 32 ? 0xffffffffu : (1u << lanes) - 1u;
-    T v = 0;
-    for (int l = threadIdx.x; l < ACC_SLOTS; l += lanes) {
-        v += acc[l];
-        acc[l] = 0;
-    }
-    for (int o = lanes / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
-    return v;
-}
-
 // Moves the accumulators of the finished stage into the history ring and
 // clears them; called by threads 0..lanes-1 of one block (lanes: a power of
 // two, at most 32).  ADV_PUSH closes the particle pass of step s (kinetic
 // energy and momentum belong to step s) and advances the step counter;
 // ADV_FIELD records the field of the current step (after the push fold when
-// both bits are set).
+// both bits are set).  fe, q: this lane's share of sums that are not in the
+// accumulators; amp: the tracked mode, where it is not in d.  Loads come
+// before the first store, so that their latencies overlap: one after the other
+// they were 2.5 us of a small grid's step (figures in pic_spectral_small.cu).
 __device__ __forceinline__ void advance_state(DevState *d, double *hist, int cap, int kind,
-                                              double fe_scale, int lanes)
+                                              double fe_scale, int lanes, double fe = 0.0,
+                                              unsigned long long q = 0, const double *amp = nullptr)
 {
-    const int l = threadIdx.x;
+    const int l = threadIdx.x & 31;
+    const unsigned mask = lanes >= 32 ? 0xffffffffu : (1u << lanes) - 1u;
     const long long s = d->step;
-    int k = (int)(s % cap);
-    if (kind & ADV_PUSH) {
-        const double ke = fold_slots(d->ke, lanes), px = fold_slots(d->px, lanes);
-        const double py = fold_slots(d->py, lanes);
-        if (l == 0) {
-            hist[1 * (size_t)cap + k] = ke;
-            hist[2 * (size_t)cap + k] = px;
-            hist[3 * (size_t)cap + k] = py;
-            d->step = s + 1;
+    const double mode = amp ? *amp : d->mode_amp;
+    double ke = 0.0, px = 0.0, py = 0.0;
+    for (int i = l; i < ACC_SLOTS; i += lanes) {
+        if (kind & ADV_PUSH) {
+            ke += d->ke[i];
+            px += d->px[i];
+            py += d->py[i];
         }
-        k = (int)((s + 1) % cap);
+        if (kind & ADV_FIELD) {
+            fe += d->fe[i];
+            q += d->q[i];
+        }
+    }
+    for (int i = l; i < ACC_SLOTS; i += lanes) {
+        if (kind & ADV_PUSH) d->ke[i] = d->px[i] = d->py[i] = 0.0;
+        if (kind & ADV_FIELD) {
+            d->fe[i] = 0.0;
+            d->q[i] = 0;
+        }
+    }
+    for (int o = lanes / 2; o > 0; o >>= 1) {
+        ke += __shfl_xor_sync(mask, ke, o);
+        px += __shfl_xor_sync(mask, px, o);
+        py += __shfl_xor_sync(mask, py, o);
+        fe += __shfl_xor_sync(mask, fe, o);
+        q += __shfl_xor_sync(mask, q, o);
+    }
+    if (l) return;
+    int k = (unsigned long long)s >> 32 ? (int)(s % cap) : (int)((unsigned)s % (unsigned)cap);
+    if (kind & ADV_PUSH) {
+        hist[1 * (size_t)cap + k] = ke;
+        hist[2 * (size_t)cap + k] = px;
+        hist[3 * (size_t)cap + k] = py;
+        d->step = s + 1;
+        if (++k == cap) k = 0;
     }
     if (kind & ADV_FIELD) {
-        const double fe = fold_slots(d->fe, lanes);
-        const unsigned long long q = fold_slots(d->q, lanes);
-        if (l == 0) {
-            hist[0 * (size_t)cap + k] = fe * fe_scale;
-            hist[4 * (size_t)cap + k] = (double)(long long)q;
-            hist[5 * (size_t)cap + k] = d->mode_amp;
-            d->mode_amp = 0.0;
-        }
+        hist[0 * (size_t)cap + k] = fe * fe_scale;
+        hist[4 * (size_t)cap + k] = (double)(long long)q;
+        hist[5 * (size_t)cap + k] = mode;
+        d->mode_amp = 0.0;
     }
 }
 

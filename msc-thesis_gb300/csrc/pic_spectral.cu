@@ -36,96 +36,9 @@
 #include <cmath>
 #include <vector>
 
-#include "pic_adjoint_dev.cuh"
-#include "pic_ensemble.cuh"
-#include "pic_fft_dev.cuh"
-#include "pic_field_dev.cuh"
+#include "pic_spectral_dev.cuh"
 
 namespace pic {
-
-struct SpecArgs {
-    unsigned long long *rho_fix;  // read by the forward rows, cleared by the columns
-    float *rho;
-    float2 *S;           // [nh][ny]: rows transformed along x
-    float2 *Tx, *Ty;     // [nh][ny]: Ex~, Ey~ after the inverse along y
-    float *ex, *ey;      // [ny][nx]
-    const float2 *twx, *twy;
-    int nx, ny, nh, lgx, lgy;
-    long long mean_fix;
-    float scale;
-    float kx1, ky1, inv_eps0_n;
-    int tmx, tmy;
-    // adjoint solve (psi = S^T g): the two gradient planes in, their half
-    // spectra in S and Sy, psi^ after the inverse along y in Tx; the inverse
-    // rows take rows y ys and y ys + yo of Tx and Ty into ex and ey (ys = 1,
-    // yo = 0 for the field; 2 and 1 for psi, two rows per transform)
-    float *gx, *gy;  // cleared by the columns
-    float2 *Sy;
-    int ys, yo;
-    int pairs, cols, rows;  // transforms (row pairs or rows), columns, rows per block
-    int sa, sb, sc;         // buffer strides (float2) of the three kernels
-    DevState *dev;
-    // diagnostics folds of the step (0: none), by one block of the inverse rows
-    double *hist;
-    int hist_cap, adv;
-    double fe_scale;
-    // ensemble: blockIdx.y picks run first + blockIdx.y of this table, whose
-    // grids sit at its offsets from the pointers above and whose constants
-    // replace the ones above (nullptr: a single run)
-    const EnsRun *runs;
-    int first;
-    int late;  // waits at its end (see pdl_wait): another group's kernel of this stage went before
-};
-
-// the arguments of this block's run
-__device__ __forceinline__ SpecArgs block_args(const SpecArgs &P)
-{
-    SpecArgs A = P;
-    if (P.runs) {
-        const int r = P.first + (int)blockIdx.y;
-        const EnsRun &R = P.runs[r];
-        A.rho_fix = P.rho_fix + R.goff;
-        A.rho = P.rho + R.goff;
-        A.S = P.S + R.khoff;
-        A.Tx = P.Tx + R.khoff;
-        A.Ty = A.Tx + R.nk;
-        A.ex = P.ex + 2 * R.goff;
-        A.ey = A.ex + R.ncp;
-        A.mean_fix = R.mean_fix;
-        A.scale = R.rho_scale;
-        A.kx1 = R.kx1;
-        A.ky1 = R.ky1;
-        A.inv_eps0_n = R.inv_eps0_n;
-        A.dev = P.dev + r;
-        A.hist = P.hist + (size_t)r * 6 * P.hist_cap;
-        A.fe_scale = R.fe_scale;
-    }
-    return A;
-}
-
-__device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) { return warp_sum_u64(v); }
-__device__ __forceinline__ double warp_sum(double v) { return warp_sum_d(v); }
-
-// Sum of v over the block, valid in thread 0.  Blocks of the small grids have
-// fewer than 32 threads (a partial warp, where full-warp shuffles are not
-// defined): their threads add through shared memory.  part: 32 entries.
-template <class T>
-__device__ __forceinline__ T block_sum(T v, T *part)
-{
-    if (blockDim.x >= 32) {
-        v = warp_sum(v);
-        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
-    } else {
-        part[threadIdx.x] = v;
-    }
-    __syncthreads();
-    T s = 0;
-    if (threadIdx.x == 0) {
-        const int np = blockDim.x >= 32 ? (int)(blockDim.x >> 5) : (int)blockDim.x;
-        for (int w = 0; w < np; ++w) s += part[w];
-    }
-    return s;
-}
 
 // LGX: log2 nx.  Block: `pairs` transforms, nx/16 threads each: a pair of
 // density rows, or with ADJ one row of the two gradient planes (gx + i gy).
@@ -422,14 +335,6 @@ pic_status spectral_twiddles(int nx, int ny, float2 **tw)
     return PIC_OK;
 }
 
-// The three kernels of a solve and their launch shapes.
-struct SpecLaunch {
-    SpecArgs A;
-    const void *kernel[3];
-    dim3 grid[3], block[3];
-    size_t smem[3];
-};
-
 // The solve of `batch` runs of one grid size (L.A.runs set) or one run: the
 // field solve, or with adj the adjoint solve (A.gx, A.gy -> psi in A.ex).  The
 // field solve leaves the fixed-point density cleared.
@@ -442,6 +347,7 @@ static pic_status plan_kernels(SpecLaunch &L, int batch, bool adj = false)
     A.twy = A.twx + fft::twiddle_len(A.lgx);
     A.ys = adj ? 2 : 1;
     A.yo = adj ? 1 : 0;
+    if (!adj && batch >= 1 && plan_small(L, A.lgx, A.lgy, batch)) return PIC_OK;
     const int tpx = nx >> 4, tpy = ny >> 4;
     // transforms of the forward and the inverse rows: row pairs and rows
     // (field), rows and row pairs (adjoint)
@@ -509,12 +415,16 @@ static pic_status plan_kernels(SpecLaunch &L, int batch, bool adj = false)
 // a step; 16 of four, 209 M, 1571 -> 1542).
 static pic_status launch_kernels(SpecLaunch *L, size_t count, cudaStream_t st)
 {
-    for (int k = 0; k < 3; ++k)
+    for (int k = 0; k < 3; ++k) {
+        int late = 0;
         for (size_t i = 0; i < count; ++i) {
-            L[i].A.late = i > 0 ? 1 : 0;
+            if (!L[i].kernel[k]) continue;
+            L[i].A.late = late;
+            late = 1;
             void *args[] = {&L[i].A};
             PIC_TRY(launch_dependent(L[i].kernel[k], L[i].grid[k], L[i].block[k], L[i].smem[k], st, args));
         }
+    }
     return PIC_OK;
 }
 

@@ -92,6 +92,15 @@ def test_spectral_solve_matches_fp64_and_cufft(nx, ny):
     assert rel_fe < 1e-5 and rel_mode < 1e-5 and rel_e < 1e-4
 
 
+@pytest.mark.parametrize("nx", [32, 64, 128])
+@pytest.mark.parametrize("ny", [32, 64, 128])
+def test_one_kernel_solve_matches_fp64_and_cufft(nx, ny):
+    """Every instance of the one-kernel solve (pic_spectral_small.cu), under
+    the checks and tolerances above: column counts that do and do not fill
+    the eight blocks, transforms that do and do not fill a warp."""
+    test_spectral_solve_matches_fp64_and_cufft(nx, ny)
+
+
 @pytest.mark.parametrize("nx,ny", [(64, 16), (32, 128)])
 def test_adjoint_solve_paths_agree(nx, ny):
     """The adjoint's transposed solve (psi = S^T g) through the spectral
