@@ -300,6 +300,8 @@ pic_status record_poisson(pic_handle *h, int adv, float *e)
 {
     if (h->spectral) {
         PIC_TRY(launch_spectral(h, adv, e));
+    } else if (h->mixed && !h->in_adjoint) {
+        PIC_TRY(launch_mixed(h, adv));
     } else {
         PIC_TRY(launch_convert(h));
         PIC_CUFFT(cufftExecR2C(h->plan_r2c, h->rho, (cufftComplex *)h->rhohat));
@@ -734,10 +736,13 @@ pic_status pic_create(const pic_config *cfg, pic_handle **out)
     H_CUFFT(cufftSetStream(h->plan_r2c, h->stream));
     H_CUFFT(cufftSetStream(h->plan_c2r2, h->stream));
     H_CUFFT(cufftSetStream(h->plan_c2r1, h->stream));
-    // the step's solve: the spectral kernels on power-of-two grids, unless
+    // the step's solve: the spectral kernels on power-of-two grids, the
+    // mixed-radix kernels on others with factors 2, 3, 5 and 7, unless
     // PIC_FIELD_SOLVER=cufft asks for the library transforms
     h->spectral = spectral_wanted(g.nx, g.ny);
+    h->mixed = mixed_wanted(g.nx, g.ny);
     if (h->spectral) H_TRY(spectral_twiddles(g.nx, g.ny, &h->tw));
+    if (h->mixed) H_TRY(mixed_twiddles(g.nx, g.ny, &h->tw));
     H_TRY(reset_device_state(h));
 #undef H_TRY
 #undef H_CUDA
@@ -1132,7 +1137,7 @@ pic_status pic_get_grid(pic_handle *h, int which, double *out)
         // phi^ into the first half of ehat, C2R into the second half (the
         // spectral solve leaves no full spectrum: transform rho first)
         const size_t nk = (size_t)h->g.ny * h->g.nh;
-        if (h->spectral)
+        if (h->spectral || h->mixed)
             PIC_CUFFT(cufftExecR2C(h->plan_r2c, h->rho, (cufftComplex *)h->rhohat));
         PIC_TRY(launch_kspace(h, true, h->ehat));
         PIC_CUFFT(cufftExecC2R(h->plan_c2r1, (cufftComplex *)h->ehat, (cufftReal *)(h->ehat + nk)));

@@ -230,6 +230,10 @@ struct pic_handle {
     // power-of-two grids: the step's solve runs in pic_spectral.cu's kernels
     // (rhohat and ehat then hold their column-major intermediates)
     bool spectral = false;
+    // other sides that are products of 2, 3, 5 and 7 (pic_spectral_mixed.cu);
+    // not while an adjoint runs: where the flow is chaotic its gradients follow
+    // the last bit of the forward fields, which stay those of cuFFT
+    bool mixed = false, in_adjoint = false;
     float2 *tw = nullptr;  // twiddles: nx entries, then ny
     // sort
     uint32_t *count = nullptr, *offset = nullptr, *cursor = nullptr, *bsum = nullptr;
@@ -290,6 +294,10 @@ bool spectral_size_ok(int nx, int ny);
 // spectral_size_ok, unless the environment variable PIC_FIELD_SOLVER=cufft
 bool spectral_wanted(int nx, int ny);
 pic_status spectral_twiddles(int nx, int ny, float2 **tw);  // cudaMalloc'd tables
+// pic_spectral_mixed.cu: likewise for the sizes of its solve
+bool mixed_wanted(int nx, int ny);
+pic_status mixed_twiddles(int nx, int ny, float2 **tw);
+pic_status launch_mixed(pic_handle *h, int adv);
 // convert + solve, rho_fix cleared, diagnostics folds `adv` (0: none)
 // (e: field planes to write, nullptr: the handle's)
 pic_status launch_spectral(pic_handle *h, int adv, float *e = nullptr);

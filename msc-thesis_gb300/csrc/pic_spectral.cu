@@ -428,11 +428,9 @@ static pic_status launch_kernels(SpecLaunch *L, size_t count, cudaStream_t st)
     return PIC_OK;
 }
 
-pic_status launch_spectral(pic_handle *h, int adv, float *e)
+void spectral_args(pic_handle *h, int adv, float *e, SpecArgs &A)
 {
     const Geometry &g = h->g;
-    SpecLaunch L;
-    SpecArgs &A = L.A;
     memset(&A, 0, sizeof A);
     A.rho_fix = h->rho_fix;
     A.rho = h->rho;
@@ -457,6 +455,12 @@ pic_status launch_spectral(pic_handle *h, int adv, float *e)
     A.hist_cap = h->hist_cap;
     A.adv = adv;
     A.fe_scale = 0.5 * h->cfg.eps0 * g.dx * g.dy * (double)g.nx * (double)g.ny;
+}
+
+pic_status launch_spectral(pic_handle *h, int adv, float *e)
+{
+    SpecLaunch L;
+    spectral_args(h, adv, e, L.A);
     PIC_TRY(plan_kernels(L, 1));
     return launch_kernels(&L, 1, h->stream);
 }

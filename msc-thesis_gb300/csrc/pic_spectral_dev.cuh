@@ -1,5 +1,5 @@
 // pic_spectral_dev.cuh -- arguments and helpers shared by the spectral solve's
-// kernels (pic_spectral.cu, pic_spectral_small.cu).
+// kernels (pic_spectral.cu, pic_spectral_small.cu, pic_spectral_mixed.cu).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -94,6 +94,43 @@ __device__ __forceinline__ T block_sum(T v, T *part)
     return s;
 }
 
+// ---- the solve in one cluster (pic_spectral_small.cu)
+constexpr int CL = 8;  // blocks per cluster (the portable maximum)
+
+__device__ __forceinline__ unsigned cluster_rank()
+{
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// (the built-in barriers, not inline asm: the compiler must not move threads of
+// a warp that took different branches to separate copies of one)
+__device__ __forceinline__ void cluster_arrive() { __cluster_barrier_arrive(); }
+__device__ __forceinline__ void cluster_wait() { __cluster_barrier_wait(); }
+// the address of this block's `p` in block `rank` of the cluster
+__device__ __forceinline__ unsigned remote(const void *p, unsigned rank)
+{
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;"
+        : "=r"(r)
+        : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void put2(unsigned a, float2 v)
+{
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v.x), "f"(v.y) : "memory");
+}
+__device__ __forceinline__ void put4(unsigned a, float2 u, float2 v)
+{
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(u.x), "f"(u.y),
+                 "f"(v.x), "f"(v.y)
+                 : "memory");
+}
+__device__ __forceinline__ void put(unsigned a, unsigned long long v)
+{
+    asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+}
+
 // The kernels of a solve and their launch shapes: three, or one (kernel[1] null).
 struct SpecLaunch {
     SpecArgs A;
@@ -102,6 +139,9 @@ struct SpecLaunch {
     size_t smem[3];
 };
 
+// the field solve's arguments on a handle (e: nullptr, or planes to write
+// instead of the handle's)
+void spectral_args(pic_handle *h, int adv, float *e, SpecArgs &A);
 // pic_spectral_small.cu: the whole field solve of `batch` runs in one kernel, for
 // the sides it takes (leaves L alone otherwise)
 bool plan_small(SpecLaunch &L, int lgx, int lgy, int batch);

@@ -30,7 +30,6 @@
 namespace pic {
 namespace {
 
-constexpr int CL = 8;  // blocks per cluster (the portable maximum)
 constexpr int E4 = 4;  // elements per thread
 
 constexpr int max_of(int a, int b) { return a > b ? a : b; }
@@ -55,44 +54,6 @@ struct Small {
     static constexpr size_t BYTES = sizeof(float2) * (WORK + COLS + 2 * ROWS);
     static_assert(WORK % 2 == 0, "the columns start on 16 bytes");
 };
-
-__device__ __forceinline__ unsigned cluster_rank()
-{
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_arrive()
-{
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void cluster_wait()
-{
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// the address of this block's `p` in block `rank` of the cluster
-__device__ __forceinline__ unsigned remote(const void *p, unsigned rank)
-{
-    unsigned r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;"
-        : "=r"(r)
-        : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void put2(unsigned a, float2 v)
-{
-    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v.x), "f"(v.y) : "memory");
-}
-__device__ __forceinline__ void put4(unsigned a, float2 u, float2 v)
-{
-    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(u.x), "f"(u.y),
-                 "f"(v.x), "f"(v.y)
-                 : "memory");
-}
-__device__ __forceinline__ void put(unsigned a, unsigned long long v)
-{
-    asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
-}
 
 __device__ __forceinline__ constexpr int rev2(int i) { return ((i & 1) << 1) | (i >> 1); }
 

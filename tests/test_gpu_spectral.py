@@ -132,3 +132,19 @@ def test_adjoint_solve_paths_agree(nx, ny):
     print(f"{nx}x{ny}: J {rs.J:.8e} vs {rc.J:.8e}; gradient rel norm differences", errs)
     assert rs.J == pytest.approx(rc.J, rel=1e-5)
     assert max(errs) < 1e-4
+
+
+@pytest.mark.parametrize("nx,ny", [(16, 18), (21, 35), (49, 64), (250, 180), (81, 100), (225, 243),
+                                   (128, 96), (256, 240), (17 * 7, 60), (63, 729), (1000, 50), (640, 700)])
+def test_mixed_radix_solve_matches_fp64_and_cufft(nx, ny):
+    """The solve of sides with factors 2, 3, 5 and 7
+    (pic_spectral_mixed.cu) under the checks and tolerances above: odd sides
+    (a last row without a partner, no Nyquist mode), every radix, rows and
+    columns that leave the last blocks with less or nothing; and a side it
+    does not take (119 = 7 x 17), where both runs use the library."""
+    if nx % 17:
+        test_spectral_solve_matches_fp64_and_cufft(nx, ny)
+    else:
+        _, gs, _ = run(nx, ny, "spectral")
+        _, gc, _ = run(nx, ny, "cufft")
+        np.testing.assert_array_equal(gs[P.GRID_EX], gc[P.GRID_EX])
