@@ -232,11 +232,13 @@ void ens_free(pic_ensemble *E)
         if (G.r2c2) cufftDestroy(G.r2c2);
         if (G.c2r1) cufftDestroy(G.c2r1);
         if (G.tw) cudaFree(G.tw);
+        if (G.done) cudaEventDestroy(G.done);
+        if (G.side) cudaStreamDestroy(G.side);
     }
-    for (int b = 0; b < 2; ++b) {
-        if (E->bounce[b]) cudaFreeHost(E->bounce[b]);
-        if (E->bounced[b]) cudaEventDestroy(E->bounced[b]);
-    }
+    if (E->fork) cudaEventDestroy(E->fork);
+    if (E->bounce) cudaFreeHost(E->bounce);
+    for (cudaEvent_t e : E->bounced)
+        if (e) cudaEventDestroy(e);
     if (E->g_one) cudaGraphExecDestroy(E->g_one);
     if (E->g_period) cudaGraphExecDestroy(E->g_period);
     if (E->g_sortstep) cudaGraphExecDestroy(E->g_sortstep);

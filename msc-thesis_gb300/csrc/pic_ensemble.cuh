@@ -76,10 +76,14 @@ struct pic_ensemble {
     struct Group {
         int nx, ny, first, count;
         cufftHandle r2c = 0, c2r = 0;
-        cufftHandle r2c2 = 0, c2r1 = 0;  // adjoint solve (made on first use)
+        // adjoint solve (made on first use), on a stream of its own but for the first group
+        cufftHandle r2c2 = 0, c2r1 = 0;
+        cudaStream_t side = nullptr;
+        cudaEvent_t done = nullptr;
         float2 *tw = nullptr;            // spectral solve's twiddle tables
     };
     std::vector<Group> groups;
+    cudaEvent_t fork = nullptr;
     // every group's side lengths are powers of two (16..4096): the step's
     // solve runs in the spectral kernels, one launch of each per group
     bool spectral = false;
@@ -87,10 +91,11 @@ struct pic_ensemble {
     cudaGraphExec_t g_one = nullptr, g_period = nullptr, g_sortstep = nullptr;
     int since_sort = 0;
     bool ready = false;
-    // page-locked buffers of the gradients' export
-    static constexpr size_t BOUNCE = 4u << 20;
-    void *bounce[2] = {nullptr, nullptr};
-    cudaEvent_t bounced[2] = {nullptr, nullptr};
+    // page-locked slots of the gradients' export
+    static constexpr size_t BOUNCE = 512u << 10;
+    static constexpr int BOUNCES = 16;
+    void *bounce = nullptr;
+    cudaEvent_t bounced[BOUNCES] = {};
     // export staging
     double *stage = nullptr;
     size_t stage_n = 0;

@@ -142,3 +142,25 @@ def test_torch_binding_of_the_batched_adjoint():
         assert amp.grad[r].item() == pytest.approx(w[r].item() * ref[r][2], rel=1e-5)
     assert J2[0].item() == J[0].item() and J2[2].item() == J[2].item()
     assert J2[1].item() != J[1].item()
+
+
+@pytest.mark.parametrize("runs", [[(64, 64, 31, 0.2, 1e-3, 21)],
+                                  [(128, 128, 33, 0.2, 1e-3, 22), (64, 32, 9, 0.15, 3e-3, 23),
+                                   (32, 32, 16, 0.25, 1e-2, 24)]])
+def test_gradient_export_fills_every_array(runs):
+    """Gradients of less than 16 MiB (copied out by the caller) and of more
+    (by threads, in parts that end inside a run), and the transposed solves of
+    one and of several grid sizes side by side: every array against the
+    single handle's, where one part astray would be an error of order one."""
+    cfgs, specs, _ = setup(runs)
+    with P.Ensemble(cfgs) as E:
+        _, grads = E.adjoint(specs, 2, 2)
+        _, again = E.adjoint(specs, 2, 2)
+    for r, (cfg, spec) in enumerate(zip(cfgs, specs)):
+        with P.Handle(cfg) as h:
+            h.init_particles(0, spec)
+            _, *sg = h.adjoint(2, every=2, spec=spec)
+        for g in (grads, again):
+            errs = [rel_norm(a, b) for a, b in zip(g[r], sg)]
+            print(f"run {r}: {max(errs):.2e}")
+            assert max(errs) < 1e-4
