@@ -166,3 +166,24 @@ def test_torch_binding_gradients(setup):
     for tt, g in zip(t, ref[1:]):
         np.testing.assert_allclose(tt.grad.numpy(), 2.0 * g, rtol=1e-4,
                                    atol=1e-4 * np.abs(g).max())
+
+
+@pytest.mark.parametrize("nsteps,every,speed", [(1, 1, 1.0), (1, 5, 1.0), (5, 1, 1.0), (7, 3, 1.0), (6, 6, 1.0),
+                                                (8, 4, 15.0)])
+def test_segments_and_scatter_windows_match_fp64(setup, nsteps, every, speed):
+    """Segments of one step, longer than the run, with and without a
+    remainder; at speed 15 (0.8 cells a step, no sort in between) particles
+    leave their blocks' windows, whose scatter is not the fixed-point one."""
+    cfg, q, m, ocfg = setup
+    with P.Handle(cfg) as h:
+        s0, _ = two_beam_handle_state(h, v0=0.2 * speed)
+        r, *g = h.adjoint(nsteps, every=every)
+        d = h.diagnostics()
+    J, *o = O.adjoint(ocfg, s0["x"], s0["y"], s0["vx"], s0["vy"], q, m, nsteps)
+    errs = [rel_norm(a, b) for a, b in zip(g, o)]
+    print(nsteps, every, speed, "J", r.J, J, errs)
+    assert d.step == nsteps and d.error_flags == 0
+    assert r.J == pytest.approx(J, rel=1e-5)
+    # the bound of up to ten steps above; an FP32 position carries 15 times the
+    # rounding of a displacement 15 times as long
+    assert max(errs) < 1e-4 * speed

@@ -121,3 +121,37 @@ def test_small_dsmc_with_mcc_electrons():
     assert d.error_flags == 0 and d.total_charge_fixed == d.expected_charge_fixed
     assert c[0] > 0 and c[5] > 0
     assert len(a["vx"]) == nn and np.isfinite(a["vx"]).all()
+
+
+@pytest.mark.parametrize("n,cells", [(1, 1), (2, 1), (3001, 1), (777, 400), (4099, 1024)])
+def test_lists_of_sparse_and_dense_cells(n, cells):
+    """The collision pass's lists: a lone particle, one pair, one cell with
+    every particle (a list of thousands), cells of one to a few particles,
+    counts that are no multiple of four: nothing lost, momentum and energy
+    kept, and collisions where cells hold pairs."""
+    nx, dt = 32, 5e-8
+    x, y, vx, vy, vz = bimodal(n, nx, seed=n)
+    c = np.arange(n) % cells
+    off = np.random.default_rng(n).random((2, n))
+    x, y = (c % nx + off[0]) * DX, (c // nx + off[1]) * DX
+    h, _ = neutral_handle(nx, nx * nx * PPC, dt)
+    with h:
+        h.set_particles(0, x, y, vx, vy, vz)
+        h.step(8)
+        a = h.get_particles(0, vz=True)
+        raw = h.get_particles_raw(0)
+        d = h.diagnostics()
+        counts = h.collision_counts()
+    assert d.error_flags == 0
+    live = raw["cell"] >= 0
+    np.testing.assert_array_equal(np.sort(raw["pid"][live]), np.arange(n, dtype=np.uint32))
+    # FP32 velocities of a few hundred m/s, each rounded a few times
+    e0 = (vx ** 2 + vy ** 2 + vz ** 2).sum()
+    for b, k in ((vx, "vx"), (vy, "vy"), (vz, "vz")):
+        assert abs(a[k].sum() - b.sum()) < 1e-5 * np.sqrt(n * e0)
+    assert abs((a["vx"] ** 2 + a["vy"] ** 2 + a["vz"] ** 2).sum() - e0) < 1e-5 * e0
+    print(n, cells, counts)
+    if n == 3001:
+        assert not np.array_equal(a["vx"], vx.astype(np.float32))
+    if n == 1:
+        np.testing.assert_array_equal(a["vx"], vx.astype(np.float32))

@@ -188,3 +188,28 @@ def test_ensemble_rejects_bad_configs():
             E.step(1)  # not initialised
         with pytest.raises(P.PicError):
             E.init([run_spec(n + 4, 0.2, 1e-3, 1)])  # over capacity
+
+
+def test_wide_windows_match_single_handles():
+    """A large ensemble of fast dense runs (512-thread blocks, wide windows)
+    beside a run whose particles hardly move and one of a particle per cell:
+    the single handles' particles, bit for bit."""
+    runs = [(128, 128, 400, 0.2, 1e-3, 51), (128, 64, 700, 0.25, 1e-2, 52), (64, 64, 20, 0.0, 1e-3, 53),
+            (32, 32, 1, 0.2, 1e-3, 54)]
+    cfgs, specs = build(runs, sort_every=20)
+    assert sum(s.n for s in specs) > 12_000_000
+    with P.Ensemble(cfgs) as E:
+        E.init(specs)
+        E.step(25)
+        ens = [E.get_particles(r) for r in range(len(runs))]
+        for r in range(len(runs)):
+            d = E.diagnostics(r)
+            assert d.error_flags == 0 and d.total_charge_fixed == d.expected_charge_fixed
+    for r, (cfg, spec) in enumerate(zip(cfgs, specs)):
+        with P.Handle(cfg) as h:
+            h.init_particles(0, spec)
+            h.prime_leapfrog()
+            h.step(25)
+            a = h.get_particles(0)
+        for k in a:
+            np.testing.assert_array_equal(ens[r][k], a[k], err_msg=f"run {r} {k}")

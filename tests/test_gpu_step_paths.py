@@ -1,0 +1,62 @@
+"""The step's launch rules change how the work is split, not its results: the
+deposit is an integer sum and a particle's push does not depend on its block,
+so the particles and the density agree bit for bit."""
+import numpy as np
+import pytest
+
+import picgpu as P
+
+pytestmark = pytest.mark.gpu
+
+NX, L, DT = 64, 4 * np.pi, 0.1
+
+
+def load(n, seed):
+    rng = np.random.default_rng(seed)
+    vx = np.where(np.arange(n) % 2 == 0, 0.2, -0.2) + 0.01 * rng.normal(size=n)
+    return rng.random(n) * L, rng.random(n) * L, vx, 0.3 * rng.normal(size=n)
+
+
+def run(parts, steps, **tuning):
+    """One species per part of the load, all of one charge and mass."""
+    total = sum(len(p[0]) for p in parts)
+    w = L * L / total
+    h = P.Handle(P.config(NX, NX, L, L, DT, [P.species(len(p[0]), -w, w, -1) for p in parts], **tuning))
+    with h:
+        for s, p in enumerate(parts):
+            h.set_particles(s, *p)
+        h.prime_leapfrog()
+        h.step(steps)
+        got = [h.get_particles(s) for s in range(len(parts))]
+        d = h.diagnostics()
+        rho = h.rho_fixed()
+    assert d.error_flags == 0 and d.total_charge_fixed == d.expected_charge_fixed
+    return {k: np.concatenate([g[k] for g in got]) for k in ("x", "y", "vx", "vy")}, rho
+
+
+def same(a, b):
+    for k in a[0]:
+        np.testing.assert_array_equal(a[0][k], b[0][k], err_msg=k)
+    np.testing.assert_array_equal(a[1], b[1])
+
+
+@pytest.mark.parametrize("n", [1, 1023, 1025, 152 * 4 * 1024 - 1, 152 * 4 * 1024 + 1, 1_500_003])
+def test_default_chunk_matches_given_chunks(n):
+    """Push blocks sized from the particle count, below and above one wave of
+    blocks on the GPU, with a last block of any length; through a sort."""
+    p = [load(n, n)]
+    auto = run(p, 7, sort_every=3)
+    for chunk in (1024, 4096):
+        same(auto, run(p, 7, sort_every=3, chunk=chunk))
+
+
+@pytest.mark.parametrize("split", [(0.5, 0.5), (0.9, 0.1), (0.4, 0.35, 0.25)])
+def test_species_pushed_side_by_side_match_one_species(split):
+    """Two or three species whose pushes overlap against one species of all
+    their particles."""
+    n = 300_001
+    p = load(n, 3)
+    cut = [0] + [int(round(n * c)) for c in np.cumsum(split)]
+    cut[-1] = n
+    parts = [tuple(a[i:j] for a in p) for i, j in zip(cut, cut[1:])]
+    same(run([p], 25, sort_every=10), run(parts, 25, sort_every=10))
