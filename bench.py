@@ -184,8 +184,9 @@ def warmup_alignment(warmup, S):
 
 def launches_for(k, since_sort, S, per_step, nspecies=1, per_sort=6):
     """Our kernels launched by k steps: per_step per step (single handle on a
-    power-of-two grid: push and the three spectral-solve kernels; ensemble of
-    such grids: push and three solve kernels per grid size); per sort
+    power-of-two grid of more than 128 cells a side: push and the three
+    spectral-solve kernels; ensemble of such grids: push and three solve
+    kernels per grid size, one for sides of 32 to 128); per sort
     and species histogram, 3 scan kernels, the scatter and the anchor kernel.
     Returns (count, sorts, since_sort)."""
     sorts, after = schedule(k, since_sort, S)
@@ -523,8 +524,9 @@ def bench_ensemble(args):
     ens_value = R.whole_job_rate(total_all * steps, ms / 1000.0)
     nb1 = -(-sum(int(g) * int(g) + 1 for g in grids) // 4096)
     per_sort = 6 if nb1 <= 4096 else 8  # two-level scan above 4096 block sums
-    ens_launches, ens_sorts, _ = launches_for(steps, S, S, 1 + 3 * len(set(int(g) for g in grids)),
-                                              per_sort=per_sort)
+    ens_launches, ens_sorts, _ = launches_for(
+        steps, S, S, 1 + sum(1 if 32 <= g <= 128 else 3 for g in set(int(g) for g in grids)),
+        per_sort=per_sort)
     plain_ms = m["plain_ms"]
     plain_value = R.whole_job_rate(total_all * steps, plain_ms / 1000.0) if plain_ms else None
     adj = ensemble_adjoint_rate(P, R, cfgs, specs, total_all, args.adjoint_steps, args.every, pg) \

@@ -220,5 +220,185 @@ __device__ __forceinline__ int result_index(int k, int t)
     return t + (k >> LGR) * (1 << (LGN - 4)) + (k & ((1 << LGR) - 1)) * (1 << (LGN - LGR));
 }
 
+// ---- radix-2 stages over four registers, shared by the transforms with four
+// elements per thread (here and in pic_spectral_small.cu)
+__device__ __forceinline__ constexpr int rev2(int i) { return ((i & 1) << 1) | (i >> 1); }
+
+// a (c -+ i s), - forward, + inverse: w16 for an angle that depends on the
+// thread (exact where w16 only swaps or keeps)
+template <bool INV>
+__device__ __forceinline__ float2 rot(float2 a, float c, float s)
+{
+    if (!INV) s = -s;
+    return make_float2(fmaf(a.x, c, -a.y * s), fmaf(a.x, s, a.y * c));
+}
+
+// one stage of a radix-2 decimation in frequency over the pairs (v0, v2), (v1, v3)
+template <bool INV>
+__device__ __forceinline__ void far_pairs(float2 (&v)[4], float c0, float s0, float c1, float s1)
+{
+    const float2 a = v[0], b = v[1], c = v[2], d = v[3];
+    v[0] = cadd(a, c);
+    v[1] = cadd(b, d);
+    v[2] = rot<INV>(csub(a, c), c0, s0);
+    v[3] = rot<INV>(csub(b, d), c1, s1);
+}
+// and over (v0, v1), (v2, v3)
+template <bool INV>
+__device__ __forceinline__ void near_pairs(float2 (&v)[4], float c0, float s0)
+{
+    const float2 a = v[0], b = v[1], c = v[2], d = v[3];
+    v[0] = cadd(a, b);
+    v[2] = cadd(c, d);
+    v[1] = rot<INV>(csub(a, b), c0, s0);
+    v[3] = rot<INV>(csub(c, d), c0, s0);
+}
+
+// A transform of length 2^LGN as the kernels hold it: n/EL threads with EL
+// elements each.  v[a][k] is element in(k, t) before and out(k, t) after run();
+// slot(i) is element i's place in a shared buffer of `room` slots.
+template <int LGN, int EL>
+struct Line;
+
+template <int LGN>
+struct Line<LGN, 16> {
+    static constexpr int TP = 1 << (LGN - 4);
+    static __device__ __forceinline__ int in(int k, int t) { return t + k * TP; }
+    static __device__ __forceinline__ int out(int k, int t) { return result_index<LGN>(k, t); }
+    static __device__ __forceinline__ int slot(int i) { return pad(i); }
+    template <bool INV, int NA>
+    static __device__ __forceinline__ void run(float2 (&v)[NA][16], float2 *const (&buf)[NA], int t,
+                                               const float2 *__restrict__ tw)
+    {
+        transform<LGN, INV, NA>(v, buf, t, tw);
+    }
+};
+
+// Four elements per thread (2^LGN >= 128, whole warps): the passes of
+// transform<LGN> in the same order of operations, each radix-16 butterfly
+// over four neighbouring lanes and a radix-8 one over two, so that every
+// result keeps its bits.  A quarter of the chain per thread and four times
+// the threads: for grids that do not fill the GPU.
+template <int LGN>
+struct Line<LGN, 4> {
+    static_assert(LGN >= 7, "whole warps");
+    static constexpr int N = 1 << LGN, TP = N / 4;
+    static __host__ __device__ constexpr int lgr(int lgns) { return pass_lgr(LGN, lgns); }
+    // register k's butterfly and its input and output there, pass lgns
+    static __device__ __forceinline__ int fly(int lgns, int k, int t)
+    {
+        return lgr(lgns) == 4 ? t >> 2 : lgr(lgns) == 3 ? t >> 1 : lgr(lgns) == 2 ? t : t + (k & 1) * TP;
+    }
+    static __device__ __forceinline__ int rin(int lgns, int k, int t)
+    {
+        return lgr(lgns) == 4 ? (t & 3) + 4 * k : lgr(lgns) == 3 ? (t & 1) + 2 * k : lgr(lgns) == 2 ? k : k >> 1;
+    }
+    static __device__ __forceinline__ int rout(int lgns, int k, int t)
+    {
+        return lgr(lgns) == 4 ? 4 * rev2(k) + rev2(t & 3) : lgr(lgns) == 3 ? 4 * (t & 1) + rev2(k)
+             : lgr(lgns) == 2 ? k : k >> 1;
+    }
+    static __device__ __forceinline__ int src(int lgns, int k, int t)
+    {
+        return fly(lgns, k, t) + rin(lgns, k, t) * (N >> lgr(lgns));
+    }
+    static __device__ __forceinline__ int dst(int lgns, int k, int t)
+    {
+        const int j = fly(lgns, k, t);
+        return ((j >> lgns) << (lgns + lgr(lgns))) + (j & ((1 << lgns) - 1)) + (rout(lgns, k, t) << lgns);
+    }
+    static __host__ __device__ constexpr int last_lgns() { return (LGN - 1) / 4 * 4; }
+    static __device__ __forceinline__ int in(int k, int t) { return src(0, k, t); }
+    static __device__ __forceinline__ int out(int k, int t) { return dst(last_lgns(), k, t); }
+    // four slots between rows of sixteen: the butterflies' lanes on different banks
+    static __device__ __forceinline__ int slot(int i) { return i + 4 * (i >> 4); }
+
+    // register q of lane g and register g of lane q change places (four lanes)
+    static __device__ __forceinline__ void turn(float2 (&v)[4], int t)
+    {
+#pragma unroll
+        for (int m = 1; m <= 2; m <<= 1)
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                const int lo = m == 1 ? 2 * p : p, hi = lo + m;
+                const bool up = t & m;
+                float2 z = up ? v[lo] : v[hi];
+                z.x = __shfl_xor_sync(0xffffffffu, z.x, m);
+                z.y = __shfl_xor_sync(0xffffffffu, z.y, m);
+                if (up)
+                    v[lo] = z;
+                else
+                    v[hi] = z;
+            }
+    }
+
+    template <bool INV, int NA, int LGNS = 0>
+    static __device__ __forceinline__ void run(float2 (&v)[NA][4], float2 *const (&buf)[NA], int t,
+                                               const float2 *__restrict__ tw)
+    {
+        constexpr float C = 0.92387953251128675613f;  // cos(pi / 8)
+        constexpr float S = 0.38268343236508977173f;  // sin(pi / 8)
+        constexpr float H = 0.70710678118654752440f;  // sqrt(1 / 2)
+        constexpr int LGR = lgr(LGNS), NS = 1 << LGNS;
+        constexpr bool LAST = LGNS + LGR == LGN;
+        if (LGNS > 0) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (LGR <= 2 && rin(LGNS, k, 0) == 0) continue;
+                float2 w = __ldg(tw + rin(LGNS, k, t) * NS + (fly(LGNS, k, t) & (NS - 1)));
+                if (INV) w.y = -w.y;
+#pragma unroll
+                for (int a = 0; a < NA; ++a) v[a][k] = cmul(v[a][k], w);
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            if (LGR == 4) {
+                // stages h = 8 and 4 over inputs q, q + 4, q + 8, q + 12, then
+                // h = 2 and 1 over positions 4 q .. 4 q + 3
+                const int q = t & 3;
+                const float c1 = q == 0 ? 1.f : q == 1 ? C : q == 2 ? H : S;
+                const float s1 = q == 0 ? 0.f : q == 1 ? S : q == 2 ? H : C;
+                const float c2 = q == 0 ? 1.f : q == 1 ? H : q == 2 ? 0.f : -H;
+                const float s2 = q == 0 ? 0.f : q == 2 ? 1.f : H;
+                far_pairs<INV>(v[a], c1, s1, -s1, c1);
+                near_pairs<INV>(v[a], c2, s2);
+                turn(v[a], t);
+                far_pairs<INV>(v[a], 1.f, 0.f, 0.f, 1.f);
+                near_pairs<INV>(v[a], 1.f, 0.f);
+            } else if (LGR == 3) {
+                // h = 4 and 2 over inputs q, q + 2, q + 4, q + 6, then h = 1
+                // with the other lane
+                const bool q = t & 1;
+                far_pairs<INV>(v[a], q ? H : 1.f, q ? H : 0.f, q ? -H : 0.f, q ? H : 1.f);
+                near_pairs<INV>(v[a], q ? 0.f : 1.f, q ? 1.f : 0.f);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float2 z = make_float2(__shfl_xor_sync(0xffffffffu, v[a][k].x, 1),
+                                                 __shfl_xor_sync(0xffffffffu, v[a][k].y, 1));
+                    v[a][k] = q ? csub(z, v[a][k]) : cadd(v[a][k], z);
+                }
+            } else if (LGR == 2) {
+                dft<4, INV>(v[a]);
+            } else {
+                far_pairs<INV>(v[a], 1.f, 0.f, 1.f, 0.f);
+            }
+        }
+        if constexpr (!LAST) {
+            __syncthreads();  // every thread has read the previous contents
+#pragma unroll
+            for (int a = 0; a < NA; ++a)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) buf[a][slot(dst(LGNS, k, t))] = v[a][k];
+            __syncthreads();
+#pragma unroll
+            for (int a = 0; a < NA; ++a)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) v[a][k] = buf[a][slot(src(LGNS + LGR, k, t))];
+            run<INV, NA, LGNS + LGR>(v, buf, t, tw + (LGNS > 0 ? NS << LGR : 0));
+        }
+    }
+};
+
 }  // namespace fft
 }  // namespace pic

@@ -22,14 +22,13 @@
 // are integers that sum to 2^32 for every particle, so the density in
 // 2^-32 charge units is an integer sum, independent of summation order, and
 // the total charge is exact.  Each thread owns four consecutive particles of
-// the sorted array (one 128-bit load per field); those that land in the same
-// cell are combined in registers (the four weights of a group follow from the
-// group's count and sums of fx, fy and fx*fy) before one set of atomics.
-// Because the weights are linear in those moments, the shared-memory window
-// keeps per cell five 32-bit sums (count, sum fx, sum fy, and the low 16 and
-// the high bits of sum fx*fy): five native 32-bit atomics per group instead
-// of two per node (eight), on the shared-memory pipe that limits this
-// kernel.  At the end of the block each window node forms its weight from
+// the sorted array (one 128-bit load per field) and adds each on its own
+// (collecting those of one cell in registers first, which only push_variant 3
+// still does, costs more instructions than the atomics it saves).  Because
+// the weights are linear in the moments, the shared-memory window keeps per
+// cell five 32-bit sums (count, sum fx, sum fy, and the low 16 and the high
+// bits of sum fx*fy): five native 32-bit atomics per particle instead of two
+// per node (eight), on the shared-memory pipe that limits this kernel.  At the end of the block each window node forms its weight from
 // the moments of its four cells and the charge sign is applied once per
 // node in a 64-bit atomic to the global density.  Per block and cell the
 // sums stay at most 2^31 for chunks of at most 32768 particles.
@@ -168,8 +167,8 @@ static PushArgs push_args(pic_handle *h, int s, int src, float dt_scale)
     A.geo.qmul = (unsigned long long)(long long)D.q_int;
     A.geo.ke_scale = move ? 0.25 * D.m : 0.0;
     A.geo.p_scale = 0.5 * D.m;
-    // the DSMC species, sorted every step, keeps its cell counts current here
-    // so that its sort can skip the histogram
+    // the DSMC species keeps its cell counts current here: the collision pass
+    // needs them every step
     A.geo.recount = (h->dsmc.on && s == h->dsmc.s) ? h->dsmc.count : nullptr;
     A.geo.ntx = g.ntx;
     return A;

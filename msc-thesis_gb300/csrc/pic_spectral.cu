@@ -1,6 +1,8 @@
 // pic_spectral.cu -- the step's Poisson solve for power-of-two grids
 // (16..4096 cells a side) in three hand-written kernels instead of the
-// conversion kernel, two cuFFT transforms and the k-space kernel:
+// conversion kernel, two cuFFT transforms and the k-space kernel.  (Sides of
+// 32 to 128 run the same operations in one kernel, pic_spectral_small.cu;
+// other sides with factors 2, 3, 5 and 7 in pic_spectral_mixed.cu.)
 //
 //   rows_fwd  fixed-point density -> float rho (background removed, charge
 //             summed), then the real FFT of each row along x: two rows per
@@ -16,7 +18,9 @@
 //   rows_inv  per row y: Z = Ex~ + i Ey~ extended to all nx modes by
 //             Hermitian symmetry (imaginary parts at kx = 0 and nx/2
 //             dropped, as a complex-to-real transform does), one inverse
-//             complex FFT, Ex = Re z, Ey = Im z.
+//             complex FFT, Ex = Re z, Ey = Im z; one block more folds the
+//             step's diagnostics.
+// The columns also clear the density for the next deposit.
 //
 // The same launches serve an ensemble's runs of one grid size (blockIdx.y
 // picks the run from the run table) and, in their adjoint mode, the
@@ -40,58 +44,59 @@
 
 namespace pic {
 
-// LGX: log2 nx.  Block: `pairs` transforms, nx/16 threads each: a pair of
+// LGX: log2 nx.  Block: `pairs` transforms, nx/EL threads each: a pair of
 // density rows, or with ADJ one row of the two gradient planes (gx + i gy).
-template <int LGX, bool ADJ>
+template <int LGX, int EL, bool ADJ>
 __global__ void __launch_bounds__(256) spec_rows_fwd_kernel(SpecArgs P)
 {
     const SpecArgs A = block_args(P);
-    constexpr int NX = 1 << LGX, TP = NX >> 4;
+    using L = fft::Line<LGX, EL>;
+    constexpr int NX = 1 << LGX, TP = L::TP;
     extern __shared__ float2 smem[];
     __shared__ unsigned long long s_q[32];
     const int f = threadIdx.x / TP, t = threadIdx.x - f * TP;
     float2 *buf[1] = {smem + f * A.sa};
-    float2 v[1][fft::E];
+    float2 v[1][EL];
     unsigned long long qs = 0;
     if (!A.late) pdl_wait();
     pdl_trigger();
     if (ADJ) {
         const size_t r0 = (size_t)(blockIdx.x * A.pairs + f) * NX;
 #pragma unroll
-        for (int k = 0; k < fft::E; ++k)
-            v[0][k] = make_float2(A.gx[r0 + t + k * TP], A.gy[r0 + t + k * TP]);
+        for (int k = 0; k < EL; ++k)
+            v[0][k] = make_float2(A.gx[r0 + L::in(k, t)], A.gy[r0 + L::in(k, t)]);
     } else {
         // all loads first (the density is read-only here), then the
         // conversions and the float density's stores
         const size_t r0 = (size_t)(blockIdx.x * A.pairs + f) * 2 * NX;
-        unsigned long long a[fft::E], b[fft::E];
+        unsigned long long a[EL], b[EL];
 #pragma unroll
-        for (int k = 0; k < fft::E; ++k) {
-            a[k] = __ldcg(A.rho_fix + r0 + t + k * TP);
-            b[k] = __ldcg(A.rho_fix + r0 + NX + t + k * TP);
+        for (int k = 0; k < EL; ++k) {
+            a[k] = __ldcg(A.rho_fix + r0 + L::in(k, t));
+            b[k] = __ldcg(A.rho_fix + r0 + NX + L::in(k, t));
         }
 #pragma unroll
-        for (int k = 0; k < fft::E; ++k) {
+        for (int k = 0; k < EL; ++k) {
             qs += a[k] + b[k];
             const float fa = fixed_to_float(a[k], A.mean_fix, A.scale);
             const float fb = fixed_to_float(b[k], A.mean_fix, A.scale);
-            A.rho[r0 + t + k * TP] = fa;
-            A.rho[r0 + NX + t + k * TP] = fb;
+            A.rho[r0 + L::in(k, t)] = fa;
+            A.rho[r0 + NX + L::in(k, t)] = fb;
             v[0][k] = make_float2(fa, fb);
         }
     }
-    fft::transform<LGX, false, 1>(v, buf, t, A.twx);
+    L::template run<false, 1>(v, buf, t, A.twx);
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < fft::E; ++k) buf[0][fft::pad(fft::result_index<LGX>(k, t))] = v[0][k];
+    for (int k = 0; k < EL; ++k) buf[0][L::slot(L::out(k, t))] = v[0][k];
     __syncthreads();
     // split each transform's spectrum; (mode, transform) with the transform
     // fastest, so that the block's rows of one mode are written together
-    const int np = A.pairs;
+    const int lg = 31 - __clz(A.pairs), np = A.pairs;  // a power of two
     for (int w = threadIdx.x; w < A.nh * np; w += blockDim.x) {
-        const int ff = w % np, k = w / np;
+        const int ff = w & (np - 1), k = w >> lg;
         const float2 *bb = smem + ff * A.sa;
-        const float2 z = bb[fft::pad(k)], m = bb[fft::pad((NX - k) & (NX - 1))];
+        const float2 z = bb[L::slot(k)], m = bb[L::slot((NX - k) & (NX - 1))];
         const float2 ra = make_float2(0.5f * (z.x + m.x), 0.5f * (z.y - m.y));
         const float2 rb = make_float2(0.5f * (z.y + m.y), 0.5f * (m.x - z.x));
         if (ADJ) {
@@ -112,11 +117,12 @@ __global__ void __launch_bounds__(256) spec_rows_fwd_kernel(SpecArgs P)
 
 // LGY: log2 ny.  Block: `cols` columns, ny/16 threads each; two buffers per
 // column (phi^, then Ey^).
-template <int LGY, bool ADJ>
+template <int LGY, int EL, bool ADJ>
 __global__ void __launch_bounds__(256, 2) spec_cols_kernel(SpecArgs P)
 {
     const SpecArgs A = block_args(P);
-    constexpr int NY = 1 << LGY, TP = NY >> 4;
+    using L = fft::Line<LGY, EL>;
+    constexpr int NY = 1 << LGY, TP = L::TP;
     extern __shared__ float2 smem[];
     __shared__ double s_fe[32];
     const int c = threadIdx.x / TP, t = threadIdx.x - c * TP;
@@ -125,7 +131,7 @@ __global__ void __launch_bounds__(256, 2) spec_cols_kernel(SpecArgs P)
     float2 *const b0 = smem + (2 * c) * A.sb, *const b1 = b0 + A.sb;
     const size_t col = (size_t)(on ? mx : 0) * NY;
     float fe = 0.f;
-    float2 v[1][fft::E];
+    float2 v[1][EL];
     if (!A.late) pdl_wait();
     pdl_trigger();
     if (!ADJ) {
@@ -146,12 +152,12 @@ __global__ void __launch_bounds__(256, 2) spec_cols_kernel(SpecArgs P)
     auto forward = [&](const float2 *src, float2 *bs) {
         float2 *buf[1] = {bs};
 #pragma unroll
-        for (int k = 0; k < fft::E; ++k)
-            v[0][k] = on ? __ldcg(src + col + t + k * TP) : make_float2(0.f, 0.f);
-        fft::transform<LGY, false, 1>(v, buf, t, A.twy);
+        for (int k = 0; k < EL; ++k)
+            v[0][k] = on ? __ldcg(src + col + L::in(k, t)) : make_float2(0.f, 0.f);
+        L::template run<false, 1>(v, buf, t, A.twy);
         __syncthreads();
 #pragma unroll
-        for (int k = 0; k < fft::E; ++k) bs[fft::pad(fft::result_index<LGY>(k, t))] = v[0][k];
+        for (int k = 0; k < EL; ++k) bs[L::slot(L::out(k, t))] = v[0][k];
         __syncthreads();
     };
     forward(A.S, b0);
@@ -159,31 +165,31 @@ __global__ void __launch_bounds__(256, 2) spec_cols_kernel(SpecArgs P)
         // psi^ = i (kx g^x + ky g^y) / (eps0 N k^2) per mode, inverse along y
         forward(A.Sy, b1);
 #pragma unroll
-        for (int k = 0; k < fft::E; ++k) {
-            const int my = t + k * TP;
-            v[0][k] = adj_mode(b0[fft::pad(my)], b1[fft::pad(my)], mx, my, A.nx, NY, A.kx1, A.ky1,
+        for (int k = 0; k < EL; ++k) {
+            const int my = L::in(k, t);
+            v[0][k] = adj_mode(b0[L::slot(my)], b1[L::slot(my)], mx, my, A.nx, NY, A.kx1, A.ky1,
                                A.inv_eps0_n, mx == 0 && my == 0);
         }
         float2 *buf[1] = {b0};
-        fft::transform<LGY, true, 1>(v, buf, t, A.twy);
+        L::template run<true, 1>(v, buf, t, A.twy);
         if (on) {
 #pragma unroll
-            for (int k = 0; k < fft::E; ++k) A.Tx[col + fft::result_index<LGY>(k, t)] = v[0][k];
+            for (int k = 0; k < EL; ++k) A.Tx[col + L::out(k, t)] = v[0][k];
         }
         return;
     }
     // k-space: phi^ stays in registers, Ey^ goes to the second buffer; the
     // two inverse transforms run one after the other
 #pragma unroll
-    for (int k = 0; k < fft::E; ++k) {
-        const int my = t + k * TP;
-        const float2 r = b0[fft::pad(my)];
+    for (int k = 0; k < EL; ++k) {
+        const int my = L::in(k, t);
+        const float2 r = b0[L::slot(my)];
         const KMode K = kspace_mode(r, mx, my, A.nx, NY, A.kx1, A.ky1, A.inv_eps0_n,
                                     mx == 0 && my == 0);
         if (on && mx == A.tmx && my == A.tmy)
             A.dev->mode_amp = sqrt((double)r.x * r.x + (double)r.y * r.y) / ((double)A.nx * NY);
         v[0][k] = K.ph;
-        b1[fft::pad(my)] = K.ey;
+        b1[L::slot(my)] = K.ey;
         fe += on ? K.fe : 0.f;
     }
     // the two inverse transforms share one copy of the code: s = 0 turns
@@ -196,16 +202,16 @@ __global__ void __launch_bounds__(256, 2) spec_cols_kernel(SpecArgs P)
         if (s) {
             __syncthreads();  // Ey^ in the second buffer is complete
 #pragma unroll
-            for (int k = 0; k < fft::E; ++k) v[0][k] = b1[fft::pad(t + k * TP)];
+            for (int k = 0; k < EL; ++k) v[0][k] = b1[L::slot(L::in(k, t))];
         }
         float2 *buf[1] = {bs};
-        fft::transform<LGY, true, 1>(v, buf, t, A.twy);
+        L::template run<true, 1>(v, buf, t, A.twy);
         if (on) {
             float2 *const out = (s ? A.Ty : A.Tx) + col;
 #pragma unroll
-            for (int k = 0; k < fft::E; ++k) {
+            for (int k = 0; k < EL; ++k) {
                 const float2 u = v[0][k];
-                out[fft::result_index<LGY>(k, t)] = s ? u : make_float2(kxe * u.y, -kxe * u.x);
+                out[L::out(k, t)] = s ? u : make_float2(kxe * u.y, -kxe * u.x);
             }
         }
     }
@@ -219,14 +225,15 @@ __global__ void __launch_bounds__(256, 2) spec_cols_kernel(SpecArgs P)
 // A.adv one block more than the rows need folds the step's diagnostics into
 // the history beside them (the push's, rows' and columns' sums are complete
 // here; a launch of its own before; figures at pdl_wait).
-template <int LGX>
+template <int LGX, int EL>
 __global__ void __launch_bounds__(256) spec_rows_inv_kernel(SpecArgs P)
 {
     const SpecArgs A = block_args(P);
-    constexpr int NX = 1 << LGX, TP = NX >> 4, HALF = NX >> 1;
+    using L = fft::Line<LGX, EL>;
+    constexpr int NX = 1 << LGX, TP = L::TP, HALF = NX >> 1;
     extern __shared__ float2 smem[];
     const int f = threadIdx.x / TP, t = threadIdx.x - f * TP;
-    const int nr = A.rows;
+    const int nr = A.rows, lg = 31 - __clz(nr);  // a power of two
     const int y0 = blockIdx.x * nr;
     if (!A.late) pdl_wait();
     pdl_trigger();
@@ -238,17 +245,17 @@ __global__ void __launch_bounds__(256) spec_rows_inv_kernel(SpecArgs P)
         return;
     }
     // (mode, row) with the row fastest: the block's rows of one mode are
-    // adjacent in Tx and Ty.  nh nr = (8 + 16 / nx) times the block's
-    // threads: at most 9 items per thread, all loads issued before the
+    // adjacent in Tx and Ty.  nh nr = (EL/2 + EL/nx) times the block's
+    // threads: at most EL/2 + 1 items per thread, all loads issued before the
     // shared-memory stores
-    constexpr int ITEMS = 9;
+    constexpr int ITEMS = EL / 2 + 1;
     const int total = (HALF + 1) * nr;
     float2 X[ITEMS], Y[ITEMS];
 #pragma unroll
     for (int q = 0; q < ITEMS; ++q) {
         const int w = threadIdx.x + q * blockDim.x;
         if (w < total) {
-            const size_t i = (size_t)(w / nr) * A.ny + (size_t)(y0 + (w % nr)) * A.ys;
+            const size_t i = (size_t)(w >> lg) * A.ny + (size_t)(y0 + (w & (nr - 1))) * A.ys;
             X[q] = __ldcg(A.Tx + i);
             Y[q] = __ldcg(A.Ty + i + A.yo);
         }
@@ -257,24 +264,24 @@ __global__ void __launch_bounds__(256) spec_rows_inv_kernel(SpecArgs P)
     for (int q = 0; q < ITEMS; ++q) {
         const int w = threadIdx.x + q * blockDim.x;
         if (w < total) {
-            const int ff = w % nr, k = w / nr;
+            const int ff = w & (nr - 1), k = w >> lg;
             float2 x = X[q], y = Y[q];
             if (k == 0 || k == HALF) x.y = y.y = 0.f;
             float2 *bb = smem + ff * A.sc;
-            bb[fft::pad(k)] = make_float2(x.x - y.y, x.y + y.x);
-            if (k > 0 && k < HALF) bb[fft::pad(NX - k)] = make_float2(x.x + y.y, y.x - x.y);
+            bb[L::slot(k)] = make_float2(x.x - y.y, x.y + y.x);
+            if (k > 0 && k < HALF) bb[L::slot(NX - k)] = make_float2(x.x + y.y, y.x - x.y);
         }
     }
     __syncthreads();
-    float2 v[1][fft::E];
+    float2 v[1][EL];
     float2 *buf[1] = {smem + f * A.sc};
 #pragma unroll
-    for (int k = 0; k < fft::E; ++k) v[0][k] = buf[0][fft::pad(t + k * TP)];
-    fft::transform<LGX, true, 1>(v, buf, t, A.twx);
+    for (int k = 0; k < EL; ++k) v[0][k] = buf[0][L::slot(L::in(k, t))];
+    L::template run<true, 1>(v, buf, t, A.twx);
     const size_t rx = (size_t)(y0 + f) * A.ys * NX, ry = rx + (size_t)A.yo * NX;
 #pragma unroll
-    for (int k = 0; k < fft::E; ++k) {
-        const int i = fft::result_index<LGX>(k, t);
+    for (int k = 0; k < EL; ++k) {
+        const int i = L::out(k, t);
         A.ex[rx + i] = v[0][k].x;
         A.ey[ry + i] = v[0][k].y;
     }
@@ -348,7 +355,16 @@ static pic_status plan_kernels(SpecLaunch &L, int batch, bool adj = false)
     A.ys = adj ? 2 : 1;
     A.yo = adj ? 1 : 0;
     if (!adj && batch >= 1 && plan_small(L, A.lgx, A.lgy, batch)) return PIC_OK;
-    const int tpx = nx >> 4, tpy = ny >> 4;
+    // Elements per thread: 16, or 4 where the grids leave the GPU to the latency
+    // of one thread's chain.  Step on single handles (23 particles per cell, 16
+    // and 4): 128x512 38.4 and 29.5 us, 256^2 35.2 and 28.8, 512^2 80.2 and 72.9,
+    // 1024x512 131.3 and 128.0, 1024^2 228.6 and 235.2; ensembles (16 per cell):
+    // two 256^2 runs 44.4 and 38.4, eight 116.5 and 114.4, 32 352 and 358; two
+    // 512^2 runs 125.6 and 124.6, four 216.6 and 220.8.
+    const bool quads = (long long)nx * ny * batch <= 524288;
+    auto elements = [&](int lg) { return quads && lg >= 7 && lg <= 10 ? 4 : 16; };
+    const int ex = elements(A.lgx), ey = elements(A.lgy);
+    const int tpx = nx / ex, tpy = ny / ey;
     // transforms of the forward and the inverse rows: row pairs and rows
     // (field), rows and row pairs (adjoint)
     const int na = adj ? ny : ny / 2, nc = adj ? ny / 2 : ny;
@@ -366,31 +382,37 @@ static pic_status plan_kernels(SpecLaunch &L, int batch, bool adj = false)
     A.cols = per_block(tpy, nh);
     A.rows = per_block(tpx, nc);
     // interleaved buffers read by consecutive lanes start on different banks
-    A.sa = fft::buf_stride(nx, 16 / std::min(A.pairs, 16));
-    A.sb = fft::buf_stride(ny, 8);
-    A.sc = fft::buf_stride(nx, 16 / std::min(A.rows, 16));
+    auto stride = [](int n, int el, int extra) {
+        return el == 4 ? n + n / 4 + extra : fft::buf_stride(n, extra);
+    };
+    A.sa = stride(nx, ex, 16 / std::min(A.pairs, 16));
+    A.sb = stride(ny, ey, 8);
+    A.sc = stride(nx, ex, 16 / std::min(A.rows, 16));
     const size_t ma = (size_t)A.pairs * A.sa * sizeof(float2);
     const size_t mb = (size_t)2 * A.cols * A.sb * sizeof(float2);
     const size_t mc = (size_t)A.rows * A.sc * sizeof(float2);
     const void *ka = nullptr, *kb = nullptr, *kc = nullptr;
-    switch (A.lgx) {
-#define PIC_SPEC_X(L)                                                                          \
-    case L:                                                                                    \
-        ka = adj ? (const void *)spec_rows_fwd_kernel<L, true>                                 \
-                 : (const void *)spec_rows_fwd_kernel<L, false>;                               \
-        kc = (const void *)spec_rows_inv_kernel<L>;                                            \
+    switch (A.lgx * 32 + ex) {
+#define PIC_SPEC_X(L, EL)                                                                      \
+    case L * 32 + EL:                                                                          \
+        ka = adj ? (const void *)spec_rows_fwd_kernel<L, EL, true>                             \
+                 : (const void *)spec_rows_fwd_kernel<L, EL, false>;                           \
+        kc = (const void *)spec_rows_inv_kernel<L, EL>;                                        \
         break;
-        PIC_SPEC_X(4) PIC_SPEC_X(5) PIC_SPEC_X(6) PIC_SPEC_X(7) PIC_SPEC_X(8) PIC_SPEC_X(9)
-        PIC_SPEC_X(10) PIC_SPEC_X(11) PIC_SPEC_X(12)
+        PIC_SPEC_X(4, 16) PIC_SPEC_X(5, 16) PIC_SPEC_X(6, 16) PIC_SPEC_X(7, 16) PIC_SPEC_X(8, 16)
+        PIC_SPEC_X(9, 16) PIC_SPEC_X(10, 16) PIC_SPEC_X(11, 16) PIC_SPEC_X(12, 16)
+        PIC_SPEC_X(7, 4) PIC_SPEC_X(8, 4) PIC_SPEC_X(9, 4) PIC_SPEC_X(10, 4)
 #undef PIC_SPEC_X
     }
-    switch (A.lgy) {
-#define PIC_SPEC_Y(L)                                                                          \
-    case L:                                                                                    \
-        kb = adj ? (const void *)spec_cols_kernel<L, true> : (const void *)spec_cols_kernel<L, false>; \
+    switch (A.lgy * 32 + ey) {
+#define PIC_SPEC_Y(L, EL)                                                                      \
+    case L * 32 + EL:                                                                          \
+        kb = adj ? (const void *)spec_cols_kernel<L, EL, true>                                 \
+                 : (const void *)spec_cols_kernel<L, EL, false>;                               \
         break;
-        PIC_SPEC_Y(4) PIC_SPEC_Y(5) PIC_SPEC_Y(6) PIC_SPEC_Y(7) PIC_SPEC_Y(8) PIC_SPEC_Y(9)
-        PIC_SPEC_Y(10) PIC_SPEC_Y(11) PIC_SPEC_Y(12)
+        PIC_SPEC_Y(4, 16) PIC_SPEC_Y(5, 16) PIC_SPEC_Y(6, 16) PIC_SPEC_Y(7, 16) PIC_SPEC_Y(8, 16)
+        PIC_SPEC_Y(9, 16) PIC_SPEC_Y(10, 16) PIC_SPEC_Y(11, 16) PIC_SPEC_Y(12, 16)
+        PIC_SPEC_Y(7, 4) PIC_SPEC_Y(8, 4) PIC_SPEC_Y(9, 4) PIC_SPEC_Y(10, 4)
 #undef PIC_SPEC_Y
     }
     if (!ka || !kb || batch < 1) {

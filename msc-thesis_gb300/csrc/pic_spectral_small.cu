@@ -55,38 +55,6 @@ struct Small {
     static_assert(WORK % 2 == 0, "the columns start on 16 bytes");
 };
 
-__device__ __forceinline__ constexpr int rev2(int i) { return ((i & 1) << 1) | (i >> 1); }
-
-// a (c -+ i s), - forward, + inverse: w16 of pic_fft_dev.cuh for an angle that
-// depends on the thread (exact where w16 only swaps or keeps)
-template <bool INV>
-__device__ __forceinline__ float2 rot(float2 a, float c, float s)
-{
-    if (!INV) s = -s;
-    return make_float2(fmaf(a.x, c, -a.y * s), fmaf(a.x, s, a.y * c));
-}
-
-// one stage of a radix-2 decimation in frequency over the pairs (v0, v2), (v1, v3)
-template <bool INV>
-__device__ __forceinline__ void far_pairs(float2 (&v)[E4], float c0, float s0, float c1, float s1)
-{
-    const float2 a = v[0], b = v[1], c = v[2], d = v[3];
-    v[0] = fft::cadd(a, c);
-    v[1] = fft::cadd(b, d);
-    v[2] = rot<INV>(fft::csub(a, c), c0, s0);
-    v[3] = rot<INV>(fft::csub(b, d), c1, s1);
-}
-// and over (v0, v1), (v2, v3)
-template <bool INV>
-__device__ __forceinline__ void near_pairs(float2 (&v)[E4], float c0, float s0)
-{
-    const float2 a = v[0], b = v[1], c = v[2], d = v[3];
-    v[0] = fft::cadd(a, b);
-    v[2] = fft::cadd(c, d);
-    v[1] = rot<INV>(fft::csub(a, b), c0, s0);
-    v[3] = rot<INV>(fft::csub(c, d), c0, s0);
-}
-
 // A thread's part in transforms of length 2^LGN (32 <= n <= 128) on n/4
 // threads of a warp: the radix-16 pass and the radix-2, 4 or 8 pass of
 // fft::transform in the same order of operations, split over the four (and
@@ -115,7 +83,7 @@ struct Part {
     // element index of register k after run(): natural but for n = 128
     __device__ __forceinline__ int index(int k) const
     {
-        return LGN == 7 ? (t & 15) + 64 * (t >> 4) + 16 * rev2(k) : t + k * TP;
+        return LGN == 7 ? (t & 15) + 64 * (t >> 4) + 16 * fft::rev2(k) : t + k * TP;
     }
 
     // v[a][k] holds element t + k TP on entry, element index(k) on exit
@@ -126,8 +94,8 @@ struct Part {
         // radix 16, outputs 4 g + j' of stages h = 8 and 4 in register g
 #pragma unroll
         for (int a = 0; a < NA; ++a) {
-            far_pairs<INV>(v[a], c1, s1, -s1, c1);
-            near_pairs<INV>(v[a], c2, s2);
+            fft::far_pairs<INV>(v[a], c1, s1, -s1, c1);
+            fft::near_pairs<INV>(v[a], c2, s2);
         }
         __syncwarp();  // every thread has read the previous contents
 #pragma unroll
@@ -143,15 +111,15 @@ struct Part {
 #pragma unroll
             for (int i = 0; i < E4; ++i) v[a][i] = buf[a][o + 4 * j + i];
             // stages h = 2 and 1
-            far_pairs<INV>(v[a], 1.f, 0.f, 0.f, 1.f);
-            near_pairs<INV>(v[a], 1.f, 0.f);
+            fft::far_pairs<INV>(v[a], 1.f, 0.f, 0.f, 1.f);
+            fft::near_pairs<INV>(v[a], 1.f, 0.f);
         }
         __syncwarp();
-        // position 4 j + i is output 4 rev2(i) + rev2(j)
+        // position 4 j + i is output 4 fft::rev2(i) + fft::rev2(j)
 #pragma unroll
         for (int a = 0; a < NA; ++a)
 #pragma unroll
-            for (int i = 0; i < E4; ++i) buf[a][o + 4 * rev2(i) + rev2(j)] = v[a][i];
+            for (int i = 0; i < E4; ++i) buf[a][o + 4 * fft::rev2(i) + fft::rev2(j)] = v[a][i];
         __syncwarp();
 #pragma unroll
         for (int a = 0; a < NA; ++a) {
@@ -165,7 +133,7 @@ struct Part {
                 }
             }
             if (LGN == 5) {
-                far_pairs<INV>(v[a], 1.f, 0.f, 1.f, 0.f);
+                fft::far_pairs<INV>(v[a], 1.f, 0.f, 1.f, 0.f);
             } else if (LGN == 6) {
                 fft::dft<4, INV>(v[a]);
             } else {
@@ -173,8 +141,8 @@ struct Part {
                 // h = 4 and 2, then h = 1 with the thread of the other q
                 const float H = 0.70710678118654752440f;
                 const bool q = t & 16;
-                far_pairs<INV>(v[a], q ? H : 1.f, q ? H : 0.f, q ? -H : 0.f, q ? H : 1.f);
-                near_pairs<INV>(v[a], q ? 0.f : 1.f, q ? 1.f : 0.f);
+                fft::far_pairs<INV>(v[a], q ? H : 1.f, q ? H : 0.f, q ? -H : 0.f, q ? H : 1.f);
+                fft::near_pairs<INV>(v[a], q ? 0.f : 1.f, q ? 1.f : 0.f);
 #pragma unroll
                 for (int k = 0; k < E4; ++k) {
                     const float2 z = make_float2(__shfl_xor_sync(~0u, v[a][k].x, 16),

@@ -213,3 +213,25 @@ def test_wide_windows_match_single_handles():
             a = h.get_particles(0)
         for k in a:
             np.testing.assert_array_equal(ens[r][k], a[k], err_msg=f"run {r} {k}")
+
+
+@pytest.mark.parametrize("nx,ny", [(128, 1024), (256, 256), (1024, 512), (512, 16)])
+def test_solves_with_4_and_16_elements_per_thread_agree(nx, ny):
+    """One run (4 elements per thread) against as many as take the transforms
+    to 16: the same operations, so the same bits.  512x16 in both: 16-point
+    columns beside 512-point rows."""
+    count = min(524288 // (nx * ny) + 1, 9)
+    cfgs, specs = build([(nx, ny, 4, 0.2, 1e-2, 60 + r) for r in range(count)], sort_every=5,
+                        chunk=1024)
+    with P.Ensemble(cfgs) as E:
+        E.init(specs)
+        E.step(12)
+        ens = {r: E.get_particles(r) for r in (0, count - 1)}
+    for r, e in ens.items():
+        with P.Handle(cfgs[r]) as h:
+            h.init_particles(0, specs[r])
+            h.prime_leapfrog()
+            h.step(12)
+            a = h.get_particles(0)
+        for k in a:
+            np.testing.assert_array_equal(e[k], a[k], err_msg=f"run {r} {k}")
