@@ -291,7 +291,10 @@ pic_status pic_step(pic_handle *h, long long nsteps);
 /* Whole run from and to host memory through one call, as the reference's
  * GPU driver is used: copy species 0 in (global coordinates), deposit,
  * solve, prime the leapfrog when prime != 0, step nsteps times and copy the
- * final state back (in id order).  Outputs may alias inputs. */
+ * final state back (in id order).  Outputs may alias inputs.  On sides that
+ * are not powers of two the fields of this call and of the adjoint come from
+ * the library's transforms, those of pic_step from the framework's own: they
+ * agree to rounding. */
 pic_status pic_run_host(pic_handle *h, long long n, const double *x, const double *y,
                         const double *vx, const double *vy, long long nsteps, int prime,
                         double *x_out, double *y_out, double *vx_out, double *vy_out);

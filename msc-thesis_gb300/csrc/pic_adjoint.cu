@@ -249,11 +249,7 @@ pic_status adjoint_run(pic_handle *h, const pic_init_spec *spec, long long nstep
 
     // ---- forward: prime, checkpoints every K steps, the last segment into
     // the ring, no re-sorting
-    struct Mark {  // the solves of this call (see in_adjoint)
-        pic_handle *h;
-        explicit Mark(pic_handle *h) : h(h) { h->in_adjoint = true; }
-        ~Mark() { h->in_adjoint = false; }
-    } mark(h);
+    const LibrarySolve mark(h);
     PIC_TRY(pic_prime_leapfrog(h));
     if (!h->rho_clear) PIC_CUDA(cudaMemsetAsync(h->rho_fix, 0, ncell * 8, st));
     for (int m = 0; m + 1 < nseg; ++m) {

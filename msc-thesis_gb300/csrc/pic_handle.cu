@@ -95,6 +95,16 @@ int pick_tile_h(int ny, int tcells, int tw)
     return best;
 }
 
+static void drop_graphs(pic_handle *h)
+{
+    for (pic_handle::StepGraphs &G : h->graphs) {
+        for (cudaGraphExec_t g : {G.period, G.sortstep, G.one})
+            if (g) cudaGraphExecDestroy(g);
+        G = pic_handle::StepGraphs();
+    }
+    h->graphs_valid = false;
+}
+
 static void free_handle_buffers(pic_handle *h)
 {
     for (int s = 0; s < PIC_MAX_SPECIES; ++s) {
@@ -130,9 +140,7 @@ static void free_handle_buffers(pic_handle *h)
     if (h->plan_r2c) cufftDestroy(h->plan_r2c);
     if (h->plan_c2r2) cufftDestroy(h->plan_c2r2);
     if (h->plan_c2r1) cufftDestroy(h->plan_c2r1);
-    if (h->g_period) cudaGraphExecDestroy(h->g_period);
-    if (h->g_sortstep) cudaGraphExecDestroy(h->g_sortstep);
-    if (h->g_one) cudaGraphExecDestroy(h->g_one);
+    drop_graphs(h);
     if (h->cub_temp) cudaFree(h->cub_temp);
     for (auto &e : h->field_ready)
         if (e) cudaEventDestroy(e);
@@ -300,7 +308,7 @@ pic_status record_poisson(pic_handle *h, int adv, float *e)
 {
     if (h->spectral) {
         PIC_TRY(launch_spectral(h, adv, e));
-    } else if (h->mixed && !h->in_adjoint) {
+    } else if (h->mixed && !h->library_solve) {
         PIC_TRY(launch_mixed(h, adv));
     } else {
         PIC_TRY(launch_convert(h));
@@ -418,14 +426,6 @@ pic_status refresh(pic_handle *h)
     return PIC_OK;
 }
 
-static void drop_graphs(pic_handle *h)
-{
-    if (h->g_period) cudaGraphExecDestroy(h->g_period);
-    if (h->g_sortstep) cudaGraphExecDestroy(h->g_sortstep);
-    if (h->g_one) cudaGraphExecDestroy(h->g_one);
-    h->g_period = h->g_sortstep = h->g_one = nullptr;
-    h->graphs_valid = false;
-}
 
 template <class F> static pic_status capture(pic_handle *h, cudaGraphExec_t *out, F &&body)
 {
@@ -446,23 +446,28 @@ template <class F> static pic_status capture(pic_handle *h, cudaGraphExec_t *out
 
 static pic_status build_graphs(pic_handle *h)
 {
-    if (h->graphs_valid) return PIC_OK;
-    drop_graphs(h);
+    if (!h->graphs_valid) drop_graphs(h);
+    h->graphs_valid = true;
+    pic_handle::StepGraphs &G = h->graphs[h->mixed && h->library_solve];
+    if (G.period) return PIC_OK;  // the last one captured
+    for (cudaGraphExec_t *g : {&G.one, &G.sortstep}) {  // of an attempt that failed
+        if (*g) cudaGraphExecDestroy(*g);
+        *g = nullptr;
+    }
     const int S = h->cfg.sort_every;
     const bool clear = h->rho_clear;  // capturing a solve runs none
-    PIC_TRY(capture(h, &h->g_one, [&] { return record_step(h, 0); }));
-    PIC_TRY(capture(h, &h->g_sortstep, [&] {
+    PIC_TRY(capture(h, &G.one, [&] { return record_step(h, 0); }));
+    PIC_TRY(capture(h, &G.sortstep, [&] {
         PIC_TRY(record_sort_all(h));
         return record_step(h, 1);
     }));
-    PIC_TRY(capture(h, &h->g_period, [&] {
+    PIC_TRY(capture(h, &G.period, [&] {
         PIC_TRY(record_sort_all(h));
         PIC_TRY(record_step(h, 1));
         for (int k = 1; k < S; ++k) PIC_TRY(record_step(h, 0));
         return PIC_OK;
     }));
     h->rho_clear = clear;
-    h->graphs_valid = true;
     return PIC_OK;
 }
 
@@ -1016,21 +1021,22 @@ pic_status pic_step(pic_handle *h, long long nsteps)
         return PIC_ERR_STATE;
     }
     PIC_TRY(build_graphs(h));
+    const pic_handle::StepGraphs &G = h->graphs[h->mixed && h->library_solve];
     const int S = h->cfg.sort_every;
     long long n = nsteps;
     while (n > 0) {
         if (h->since_sort >= S) {
             if (n >= S) {
-                PIC_CUDA(cudaGraphLaunch(h->g_period, h->stream));
+                PIC_CUDA(cudaGraphLaunch(G.period, h->stream));
                 n -= S;
                 h->since_sort = S;
             } else {
-                PIC_CUDA(cudaGraphLaunch(h->g_sortstep, h->stream));
+                PIC_CUDA(cudaGraphLaunch(G.sortstep, h->stream));
                 n -= 1;
                 h->since_sort = 1;
             }
         } else {
-            PIC_CUDA(cudaGraphLaunch(h->g_one, h->stream));
+            PIC_CUDA(cudaGraphLaunch(G.one, h->stream));
             n -= 1;
             h->since_sort += 1;
         }
@@ -1044,6 +1050,8 @@ pic_status pic_run_host(pic_handle *h, long long n, const double *x, const doubl
                         const double *vx, const double *vy, long long nsteps, int prime,
                         double *x_out, double *y_out, double *vx_out, double *vy_out)
 {
+    PIC_TRY(need(h));
+    const LibrarySolve mark(h);
     PIC_TRY(pic_set_particles(h, 0, n, x, y, vx, vy, nullptr));
     if (prime) PIC_TRY(pic_prime_leapfrog(h));
     PIC_TRY(pic_step(h, nsteps));

@@ -231,9 +231,9 @@ struct pic_handle {
     // (rhohat and ehat then hold their column-major intermediates)
     bool spectral = false;
     // other sides that are products of 2, 3, 5 and 7 (pic_spectral_mixed.cu);
-    // not while an adjoint runs: where the flow is chaotic its gradients follow
-    // the last bit of the forward fields, which stay those of cuFFT
-    bool mixed = false, in_adjoint = false;
+    // library_solve: within a call that hands its results back in 64 bits
+    // (LibrarySolve), whose fields stay those of cuFFT to the last bit
+    bool mixed = false, library_solve = false;
     float2 *tw = nullptr;  // twiddles: nx entries, then ny
     // sort
     uint32_t *count = nullptr, *offset = nullptr, *cursor = nullptr, *bsum = nullptr;
@@ -244,7 +244,9 @@ struct pic_handle {
     int hist_cap = 0;
     int track_mx = -1, track_my = -1;
     // graphs
-    cudaGraphExec_t g_period = nullptr, g_sortstep = nullptr, g_one = nullptr;
+    struct StepGraphs {
+        cudaGraphExec_t period = nullptr, sortstep = nullptr, one = nullptr;
+    } graphs[2];  // [1]: with library_solve on a handle whose solve it changes
     int since_sort = 0;
     bool graphs_valid = false;
     bool fields_valid = false;
@@ -298,6 +300,15 @@ pic_status spectral_twiddles(int nx, int ny, float2 **tw);  // cudaMalloc'd tabl
 bool mixed_wanted(int nx, int ny);
 pic_status mixed_twiddles(int nx, int ny, float2 **tw);
 pic_status launch_mixed(pic_handle *h, int adv);
+// pic_run_host and the adjoint: their arrays are doubles, and where the flow is
+// chaotic an adjoint's gradients follow the last bit of the forward fields
+struct LibrarySolve {
+    pic_handle *h;
+    explicit LibrarySolve(pic_handle *h) : h(h) { h->library_solve = true; }
+    ~LibrarySolve() { h->library_solve = false; }
+    LibrarySolve(const LibrarySolve &) = delete;
+    LibrarySolve &operator=(const LibrarySolve &) = delete;
+};
 // convert + solve, rho_fix cleared, diagnostics folds `adv` (0: none)
 // (e: field planes to write, nullptr: the handle's)
 pic_status launch_spectral(pic_handle *h, int adv, float *e = nullptr);

@@ -84,3 +84,37 @@ def test_run_host_rejects_more_particles_than_capacity():
     with P.Handle(cfg) as h:
         with pytest.raises(P.PicError):
             h.run_host(x, y, vx, vy, 1)
+
+
+def test_run_host_keeps_the_library_transforms(monkeypatch):
+    """On sides with factors 2, 3 and 5 the one-call run solves through the
+    library, as PIC_FIELD_SOLVER=cufft does everywhere, while plain steps do
+    not: the same bits before and after steps on the same handle, whose two
+    sets of graphs stay apart."""
+    nx, ny, n = 54, 45, 54 * 45 * 20 + 3
+    cfg, _, _ = normalized_electrons(nx, ny, L, L, n, DT)
+    arrs = _load(n, seed=23)
+
+    def stepped(h):
+        h.set_particles(0, *arrs)
+        h.prime_leapfrog()
+        h.step(25)
+        return h.get_particles()
+
+    with P.Handle(cfg) as h:
+        first = h.run_host(*[a.copy() for a in arrs], 25)
+        plain = stepped(h)
+        again = h.run_host(*[a.copy() for a in arrs], 25)
+        assert h.diagnostics().error_flags == 0
+    monkeypatch.setenv("PIC_FIELD_SOLVER", "cufft")
+    with P.Handle(cfg) as h:
+        lib = h.run_host(*[a.copy() for a in arrs], 25)
+        lib_stepped = stepped(h)
+    for k, a, b, c in zip(("x", "y", "vx", "vy"), first, again, lib):
+        np.testing.assert_array_equal(a, b, err_msg=k)
+        np.testing.assert_array_equal(a, c, err_msg=k)
+        np.testing.assert_array_equal(a, lib_stepped[k], err_msg=k)
+        # rounding of the fields over 25 steps, as in test_gpu_spectral.py
+        d = periodic_diff(plain[k], a, L) if k in "xy" else plain[k] - a
+        assert np.abs(d).max() < 1e-4
+    assert not np.array_equal(plain["vx"], first[2])
