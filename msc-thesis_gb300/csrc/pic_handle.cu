@@ -201,14 +201,22 @@ static pic_status validate(const pic_config *c, pic_handle *h)
 // blocks (four per SM): as few waves as keep a block at most 13824 particles
 // (its window stays small against them) and at most `limit` (about one and
 // a third of the particles of its tile, so that a block rarely reaches a
-// third tile), and at least 1024 (one pass of its threads).  us per step with
+// third tile), and at least 1024 (one pass of its threads).  What one wave
+// of more than 6912 would hold goes into several of at most 4608: a block that
+// goes on into the next tile row, whose tile is no neighbour, sends that part
+// through the global path, and a single wave waits for it (four loads each,
+// 512^2 x 32 per cell 95 to 104 us a step with 13800, 94.7 with 4600; 256^2 x
+// 100 76 to 80 with 10780, 74.6 with 3600; 512^2 x 20 72 to 74 with 8620, 71.4
+// with 4310; but 512^2 x 16 59 to 64 with 6900, 62 with 3450, 256^2 x 64 50 to 53
+// and 53.3, and in two waves 1024^2 x 16 164 with 13800, 174 with 6900).  us per step with
 // 8192 for all sizes before: 64^2 x 16 per cell 42.0 -> 21.9, 128^2 x 32 41.5
 // -> 26.3, 250 x 180 x 23 49.9 -> 36.3, 128^2 x 100 45.3 -> 35.2, 256^2 x 32
 // 53.2 -> 40.5, 512^2 x 32 109 -> 100, 1024^2 x 32 317 -> 308.
 static int push_chunk(long long n, double limit)
 {
     const double per = std::ceil((double)std::max(1ll, n) / (4.0 * device_sms()));
-    const double waves = std::ceil(per / std::min(13824.0, std::max(1024.0, limit)));
+    const double most = per > 13824.0 ? 13824.0 : per <= 6912.0 ? 6912.0 : 4608.0;
+    const double waves = std::ceil(per / std::min(most, std::max(1024.0, limit)));
     return std::max(1024, ((int)std::ceil(per / waves) + 3) & ~3);
 }
 
