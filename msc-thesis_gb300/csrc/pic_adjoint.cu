@@ -250,6 +250,10 @@ pic_status adjoint_run(pic_handle *h, const pic_init_spec *spec, long long nstep
     // ---- forward: prime, checkpoints every K steps, the last segment into
     // the ring, no re-sorting
     const LibrarySolve mark(h);
+    if (h->mixed) {  // the field that the caller's last call left is not the library's
+        PIC_TRY(deposit_now(h));
+        PIC_TRY(record_poisson(h, ADV_FIELD));
+    }
     PIC_TRY(pic_prime_leapfrog(h));
     if (!h->rho_clear) PIC_CUDA(cudaMemsetAsync(h->rho_fix, 0, ncell * 8, st));
     for (int m = 0; m + 1 < nseg; ++m) {

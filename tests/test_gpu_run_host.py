@@ -118,3 +118,26 @@ def test_run_host_keeps_the_library_transforms(monkeypatch):
         d = periodic_diff(plain[k], a, L) if k in "xy" else plain[k] - a
         assert np.abs(d).max() < 1e-4
     assert not np.array_equal(plain["vx"], first[2])
+
+
+def test_adjoint_keeps_the_library_transforms(monkeypatch):
+    """Likewise for the adjoint's forward steps, from its first field on: the
+    final state and J to the last bit, the gradients to the order of their
+    float sums."""
+    nx, ny, n = 54, 45, 54 * 45 * 20 + 3
+    cfg, _, _ = normalized_electrons(nx, ny, L, L, n, DT)
+    arrs = _load(n, seed=24)
+    got = []
+    for solver in ("spectral", "cufft"):
+        monkeypatch.setenv("PIC_FIELD_SOLVER", solver)
+        with P.Handle(cfg) as h:
+            h.set_particles(0, *arrs)
+            r, *g = h.adjoint(20, every=6)
+            got.append((r.J, g, h.get_particles(), h.history(P.HIST_FIELD_ENERGY, 0, 21)))
+    (Ja, ga, pa, fa), (Jb, gb, pb, fb) = got
+    assert Ja == Jb
+    np.testing.assert_array_equal(fa, fb)
+    for k in pa:
+        np.testing.assert_array_equal(pa[k], pb[k], err_msg=k)
+    for a, b in zip(ga, gb):
+        assert np.linalg.norm(a - b) < 1e-5 * np.linalg.norm(b)
