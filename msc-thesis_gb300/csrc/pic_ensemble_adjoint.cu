@@ -344,7 +344,7 @@ pic_status transform_groups(pic_ensemble *E, F transform)
 // Device arrays to pageable host memory through a ring of page-locked slots,
 // copied out by a few threads beside the transfers.  Into memory that the
 // caller has never touched (a fresh array) the pages fault in one by one: 330 MB
-// of gradients took 140 ms by the driver's own copy, 38 ms through a vector that
+// of gradients took 140 ms by cudaMemcpy itself, 38 ms through a vector that
 // stayed touched, 32 ms by one thread from two slots, 9 ms by eight.  The
 // threads live for one call; where none can be started the caller copies.
 class Export {

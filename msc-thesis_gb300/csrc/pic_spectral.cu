@@ -360,8 +360,11 @@ static pic_status plan_kernels(SpecLaunch &L, int batch, bool adj = false)
     // and 4): 128x512 38.4 and 29.5 us, 256^2 35.2 and 28.8, 512^2 80.2 and 72.9,
     // 1024x512 131.3 and 128.0, 1024^2 228.6 and 235.2; ensembles (16 per cell):
     // two 256^2 runs 44.4 and 38.4, eight 116.5 and 114.4, 32 352 and 358; two
-    // 512^2 runs 125.6 and 124.6, four 216.6 and 220.8.
-    const bool quads = (long long)nx * ny * batch <= 524288;
+    // 512^2 runs 125.6 and 124.6, four 216.6 and 220.8.  The field keeps its
+    // bits; the adjoint's psi^ goes from its operator straight into the transform
+    // and does not (a chaotic run's gradients three times as far off as by the
+    // order of their sums), so that solve stays at 16.
+    const bool quads = !adj && (long long)nx * ny * batch <= 524288;
     auto elements = [&](int lg) { return quads && lg >= 7 && lg <= 10 ? 4 : 16; };
     const int ex = elements(A.lgx), ey = elements(A.lgy);
     const int tpx = nx / ex, tpy = ny / ey;
@@ -395,7 +398,7 @@ static pic_status plan_kernels(SpecLaunch &L, int batch, bool adj = false)
     switch (A.lgx * 32 + ex) {
 #define PIC_SPEC_X(L, EL)                                                                      \
     case L * 32 + EL:                                                                          \
-        ka = adj ? (const void *)spec_rows_fwd_kernel<L, EL, true>                             \
+        ka = adj ? (const void *)spec_rows_fwd_kernel<L, 16, true>                             \
                  : (const void *)spec_rows_fwd_kernel<L, EL, false>;                           \
         kc = (const void *)spec_rows_inv_kernel<L, EL>;                                        \
         break;
@@ -407,7 +410,7 @@ static pic_status plan_kernels(SpecLaunch &L, int batch, bool adj = false)
     switch (A.lgy * 32 + ey) {
 #define PIC_SPEC_Y(L, EL)                                                                      \
     case L * 32 + EL:                                                                          \
-        kb = adj ? (const void *)spec_cols_kernel<L, EL, true>                                 \
+        kb = adj ? (const void *)spec_cols_kernel<L, 16, true>                                 \
                  : (const void *)spec_cols_kernel<L, EL, false>;                               \
         break;
         PIC_SPEC_Y(4, 16) PIC_SPEC_Y(5, 16) PIC_SPEC_Y(6, 16) PIC_SPEC_Y(7, 16) PIC_SPEC_Y(8, 16)
