@@ -137,9 +137,10 @@ typedef struct pic_config {
 typedef struct pic_handle pic_handle;
 
 pic_status pic_config_default(pic_config *cfg);
-/* Power-of-two grids of 16..4096 cells a side solve the field with the
- * library's spectral kernels, other sizes with cuFFT; the environment
- * variable PIC_FIELD_SOLVER=cufft, read here, selects cuFFT for any size. */
+/* Power-of-two grids of 16..4096 cells a side, and others of 16..1024 whose
+ * sides are products of 2, 3, 5 and 7, solve the field with this library's
+ * spectral kernels, other sizes with cuFFT; the environment variable
+ * PIC_FIELD_SOLVER=cufft, read here, selects cuFFT for any size. */
 pic_status pic_create(const pic_config *cfg, pic_handle **out);
 pic_status pic_destroy(pic_handle *h);
 /* The CUDA stream all of the handle's work runs on (cudaStream_t). */
@@ -293,8 +294,8 @@ pic_status pic_step(pic_handle *h, long long nsteps);
  * solve, prime the leapfrog when prime != 0, step nsteps times and copy the
  * final state back (in id order).  Outputs may alias inputs.  On sides that
  * are not powers of two the fields of this call and of the adjoint come from
- * the library's transforms, those of pic_step from the framework's own: they
- * agree to rounding. */
+ * cuFFT, those of pic_step from this library's kernels: they agree to
+ * rounding. */
 pic_status pic_run_host(pic_handle *h, long long n, const double *x, const double *y,
                         const double *vx, const double *vy, long long nsteps, int prime,
                         double *x_out, double *y_out, double *vx_out, double *vy_out);

@@ -19,8 +19,9 @@
 // whose extra warp does the diagnostics fold beside the inverse rows.
 // One step of 64^2 cells with 16 particles each: 20.5 -> 12.0 us, of 128^2 with
 // 100 each: 34.2 -> 27.1 us; eight runs of small grids in one ensemble: 87 ->
-// 79 us.  The results keep their bits.  The same split with the three kernels' radix-16 transforms, block
-// barriers, global sums and the fold by atomics: 17.5, 31.9 and 93 us.
+// 79 us.  The results keep their bits.  The same split with the three kernels'
+// radix-16 transforms, block barriers, global sums and the fold by atomics:
+// 17.5, 31.9 and 93 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
