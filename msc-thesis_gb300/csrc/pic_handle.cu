@@ -306,7 +306,9 @@ static void update_mean(pic_handle *h)
     for (int s = 0; s < h->cfg.nspecies; ++s)
         total += (__int128)h->cfg.species[s].q_int * h->sp[s].n * ((__int128)1 << 32);
     const __int128 nc = (__int128)h->g.nx * h->g.ny;
-    h->mean_fix = (long long)(total / nc);
+    const long long mean = (long long)(total / nc);
+    if (mean != h->mean_fix) drop_graphs(h);  // the solve's launches hold it
+    h->mean_fix = mean;
 }
 
 // ---------------------------------------------------------------- stages

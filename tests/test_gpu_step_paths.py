@@ -60,3 +60,21 @@ def test_species_pushed_side_by_side_match_one_species(split):
     cut[-1] = n
     parts = [tuple(a[i:j] for a in p) for i, j in zip(cut, cut[1:])]
     same(run([p], 25, sort_every=10), run(parts, 25, sort_every=10))
+
+
+def test_a_reload_with_another_count_steps_as_a_fresh_handle():
+    """The background that the solve subtracts follows the loaded count: a
+    handle with a given push chunk, stepped, loaded with more particles and
+    stepped again, against a handle loaded with them at once."""
+    first, then = load(NX * NX * 16, 5), load(NX * NX * 20, 6)
+    n = len(then[0])
+    cfg = P.config(NX, NX, L, L, DT, [P.species(n, -L * L / n, L * L / n, -1)], chunk=1024, sort_every=3)
+    got = []
+    for loads in ((first, then), (then,)):
+        with P.Handle(cfg) as h:
+            for a in loads:
+                h.set_particles(0, *a)
+                h.prime_leapfrog()
+                h.step(7)
+            got.append((h.get_particles(0), h.grid(P.GRID_RHO)))
+    same(*got)
