@@ -68,24 +68,26 @@ __device__ __forceinline__ KMode kspace_mode(float2 r, int mx, int my, int nx, i
 // accumulators; amp: the tracked mode, where it is not in d.  Loads come
 // before the first store, so that their latencies overlap: one after the other
 // they were 2.5 us of a small grid's step (figures in pic_spectral_small.cu).
+// They go to L2 (late kernels fold too, see pdl_wait): an SM that folded the
+// step before may still hold the cleared lines, from before this step's atomics.
 __device__ __forceinline__ void advance_state(DevState *d, double *hist, int cap, int kind,
                                               double fe_scale, int lanes, double fe = 0.0,
                                               unsigned long long q = 0, const double *amp = nullptr)
 {
     const int l = threadIdx.x & 31;
     const unsigned mask = lanes >= 32 ? 0xffffffffu : (1u << lanes) - 1u;
-    const long long s = d->step;
-    const double mode = amp ? *amp : d->mode_amp;
+    const long long s = __ldcg(&d->step);
+    const double mode = amp ? *amp : __ldcg(&d->mode_amp);
     double ke = 0.0, px = 0.0, py = 0.0;
     for (int i = l; i < ACC_SLOTS; i += lanes) {
         if (kind & ADV_PUSH) {
-            ke += d->ke[i];
-            px += d->px[i];
-            py += d->py[i];
+            ke += __ldcg(&d->ke[i]);
+            px += __ldcg(&d->px[i]);
+            py += __ldcg(&d->py[i]);
         }
         if (kind & ADV_FIELD) {
-            fe += d->fe[i];
-            q += d->q[i];
+            fe += __ldcg(&d->fe[i]);
+            q += __ldcg(&d->q[i]);
         }
     }
     for (int i = l; i < ACC_SLOTS; i += lanes) {

@@ -313,8 +313,8 @@ spec_small_kernel(SpecArgs P)
             advance_state(A.dev, A.hist, A.hist_cap, A.adv, A.fe_scale, 32, fe, q, tracked ? &s_amp : nullptr);
         } else {
             if (A.adv) advance_state(A.dev, A.hist, A.hist_cap, A.adv, A.fe_scale, 32);
-            A.dev->q[lane] += q;
-            A.dev->fe[lane] += fe;
+            A.dev->q[lane] = __ldcg(&A.dev->q[lane]) + q;
+            A.dev->fe[lane] = __ldcg(&A.dev->fe[lane]) + fe;
             if (tracked && lane == 0) A.dev->mode_amp = s_amp;
         }
     }

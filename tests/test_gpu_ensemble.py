@@ -235,3 +235,38 @@ def test_solves_with_4_and_16_elements_per_thread_agree(nx, ny):
             a = h.get_particles(0)
         for k in a:
             np.testing.assert_array_equal(e[k], a[k], err_msg=f"run {r} {k}")
+
+
+@pytest.mark.parametrize("runs", [[(32, 32, 10, 0.2, 1e-3, 71), (16, 64, 10, 0.1, 1e-2, 72), (64, 64, 10, 0.25, 5e-4, 73)],
+                                  [(32, 32, 16, 0.2, 1e-3, 74), (64, 32, 12, 0.15, 3e-3, 75), (32, 32, 12, 0.3, 1e-4, 76),
+                                   (16, 64, 16, 0.1, 1e-2, 77), (256, 256, 10, 0.2, 1e-2, 78), (64, 64, 20, 0.25, 5e-4, 79)]])
+def test_histories_of_several_grid_sizes_match_single_handles(runs):
+    """Every step's energies, momentum and charge of every run where grid sizes
+    solve and fold side by side: a few blocks on a mostly idle GPU, and a
+    large run among small ones."""
+    nst = 60
+    cfgs, specs = build(runs, sort_every=20, chunk=1024)
+    which = (P.HIST_FIELD_ENERGY, P.HIST_KINETIC, P.HIST_MOMENTUM_X, P.HIST_MOMENTUM_Y, P.HIST_CHARGE)
+
+    def histories(get):
+        return [get(w, 0, nst + (w in (P.HIST_FIELD_ENERGY, P.HIST_CHARGE))) for w in which]
+
+    with P.Ensemble(cfgs) as E:
+        E.init(specs)
+        E.step(nst)
+        ens = [histories(lambda w, a, k: E.history(r, w, a, k)) for r in range(len(runs))]
+    for r, (cfg, spec) in enumerate(zip(cfgs, specs)):
+        with P.Handle(cfg) as h:
+            h.init_particles(0, spec)
+            h.prime_leapfrog()
+            h.step(nst)
+            one = histories(h.history)
+        # the particles agree bit for bit; the sums are of up to 64 squares or
+        # velocities in FP32 per thread (64 roundings, 4e-6), then in FP64
+        fe, ke, mx, my, q = range(5)
+        np.testing.assert_allclose(ens[r][fe], one[fe], rtol=1e-5)
+        np.testing.assert_allclose(ens[r][ke], one[ke], rtol=1e-5)
+        scale = 1e-5 * cfg.species[0].m * spec.n * (spec.beam_v + 3 * spec.vth[0])
+        np.testing.assert_allclose(ens[r][mx], one[mx], rtol=0, atol=scale)
+        np.testing.assert_allclose(ens[r][my], one[my], rtol=0, atol=scale)
+        np.testing.assert_array_equal(ens[r][q], one[q])
