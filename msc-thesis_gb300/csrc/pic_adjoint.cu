@@ -41,7 +41,7 @@ struct AdjArgs {
 // (adj_kick_block; 128^2 x 32 per cell: 16 us against 21 us with eight global
 // float adds per particle).
 __global__ void __launch_bounds__(256, 3)
-adj_kick_kernel(KickArgs A, KickGeo K, const int32_t *__restrict__ anchor, int chunk, long long n4)
+adj_kick_kernel(KickArgs A, KickGeo K, const int32_t *anchor, int chunk, long long n4)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     pdl_wait();

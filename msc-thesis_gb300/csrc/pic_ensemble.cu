@@ -39,7 +39,7 @@ namespace pic {
 template <bool GATHER, bool DEPOSIT>
 __global__ void __launch_bounds__(512, 2)
 ens_push_kernel(PushArgs A, const SegBlock *__restrict__ blk, const EnsRun *__restrict__ runs,
-                const int32_t *__restrict__ anchor, float kick, float drift)
+                const int32_t *anchor, float kick, float drift)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const SegBlock b = blk[blockIdx.x];

@@ -74,7 +74,7 @@ __device__ __forceinline__ PushGeo adj_geo(const EnsRun &R, const float *e)
 template <bool UNKICK>
 __global__ void __launch_bounds__(256, 3)
 ens_adj_kick_kernel(EnsAdjArgs A, const SegBlock *__restrict__ blk, const EnsRun *__restrict__ runs,
-                    const int32_t *__restrict__ anchor, float cscale, float dscale)
+                    const int32_t *anchor, float cscale, float dscale)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const SegBlock b = blk[blockIdx.x];

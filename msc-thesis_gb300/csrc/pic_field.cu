@@ -20,8 +20,8 @@ namespace pic {
 // large mean keep their relative precision.  Two cells per thread per
 // iteration (16-byte loads, 8-byte stores; n is even).
 __global__ void __launch_bounds__(256)
-convert_kernel(const unsigned long long *__restrict__ rho_fix, float *__restrict__ rho, long long n,
-               long long mean_fix, float scale, DevState *dev)
+convert_kernel(const unsigned long long *rho_fix, float *__restrict__ rho, long long n, long long mean_fix,
+               float scale, DevState *dev)
 {
     __shared__ unsigned long long s_part[8];
     pdl_wait();

@@ -113,6 +113,9 @@ enum : uint32_t {
 // launched calls pdl_wait in all of its blocks before it touches anything an
 // earlier kernel reads or writes, so that the end of one kernel implies the
 // end of all before it; kernels of the chain trigger after their own wait.
+// What earlier kernels write is no const __restrict__ argument of such a
+// kernel: that would allow loads through the path for data that nothing writes
+// while the kernel runs, and its writers may still run when it starts.
 // Hides the launch and the ramp of the next kernel behind the tail of the one
 // before: with the density's clearing and the diagnostics folds moved into the
 // solve's kernels (four kernels a step instead of five and a memset), 128^2 x
