@@ -295,7 +295,7 @@ pic_status pic_step(pic_handle *h, long long nsteps);
  * final state back (in id order).  Outputs may alias inputs.  On sides that
  * are not powers of two the fields of this call and of the adjoint come from
  * cuFFT, those of pic_step from this library's kernels: they agree to
- * rounding. */
+ * rounding.  Both calls leave the field of pic_step's solve. */
 pic_status pic_run_host(pic_handle *h, long long n, const double *x, const double *y,
                         const double *vx, const double *vy, long long nsteps, int prime,
                         double *x_out, double *y_out, double *vx_out, double *vy_out);

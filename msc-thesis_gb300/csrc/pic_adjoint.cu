@@ -388,9 +388,11 @@ pic_status adjoint_run(pic_handle *h, const pic_init_spec *spec, long long nstep
         PIC_TRY(launch_init_dA(h, spec, lx, ly, buf, buf + n));
         PIC_CUDA(cudaMemcpyAsync(dA.data(), buf, dA.size() * 8, cudaMemcpyDeviceToHost, st));
     }
-    // ---- leave the handle at step nsteps
-    if (nseg > 1) {
-        PIC_TRY(snap_copy(h, fin, false, np));
+    // ---- leave the handle at step nsteps, with the field of its own solve (as
+    // a state file of these particles would)
+    h->library_solve = false;
+    if (nseg > 1) PIC_TRY(snap_copy(h, fin, false, np));
+    if (nseg > 1 || h->mixed) {
         PIC_TRY(deposit_now(h));
         PIC_TRY(record_poisson(h, 0));
     }

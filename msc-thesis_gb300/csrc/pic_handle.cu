@@ -1066,7 +1066,17 @@ pic_status pic_run_host(pic_handle *h, long long n, const double *x, const doubl
     if (prime) PIC_TRY(pic_prime_leapfrog(h));
     PIC_TRY(pic_step(h, nsteps));
     PIC_TRY(check_flags(h));
-    return pic_get_particles(h, 0, nullptr, x_out, y_out, vx_out, vy_out, nullptr);
+    PIC_TRY(pic_get_particles(h, 0, nullptr, x_out, y_out, vx_out, vy_out, nullptr));
+    if (!h->mixed) return PIC_OK;
+    // the handle's field is that of its own solve again, as a state file of
+    // these particles would leave it; the history keeps this run's sums
+    h->library_solve = false;
+    PIC_TRY(ensure_stage(h, sizeof(DevState)));
+    PIC_CUDA(cudaMemcpyAsync(h->stage, h->dev, sizeof(DevState), cudaMemcpyDeviceToDevice, h->stream));
+    PIC_TRY(deposit_now(h));
+    PIC_TRY(record_poisson(h, 0));
+    PIC_CUDA(cudaMemcpyAsync(h->dev, h->stage, sizeof(DevState), cudaMemcpyDeviceToDevice, h->stream));
+    return PIC_OK;
 }
 
 pic_status pic_diagnostics(pic_handle *h, pic_diag *d)

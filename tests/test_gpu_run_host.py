@@ -141,3 +141,33 @@ def test_adjoint_keeps_the_library_transforms(monkeypatch):
         np.testing.assert_array_equal(pa[k], pb[k], err_msg=k)
     for a, b in zip(ga, gb):
         assert np.linalg.norm(a - b) < 1e-5 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("call", ["run_host", "one segment", "segments"])
+def test_steps_after_a_library_solve_resume_bit_for_bit(call, tmp_path):
+    """On sides with factors 2, 3 and 5 the field that the one-call run and the
+    adjoint leave is a function of the particles alone, as after every other
+    call: steps go on as from a state file of them."""
+    nx, ny, n = 54, 45, 54 * 45 * 20 + 3
+    cfg, _, _ = normalized_electrons(nx, ny, L, L, n, DT)
+    arrs = _load(n, seed=25)
+    path = str(tmp_path / "run.picstate")
+    with P.Handle(cfg) as h:
+        if call == "run_host":
+            h.run_host(*[a.copy() for a in arrs], 20)
+        else:
+            h.set_particles(0, *arrs)
+            h.adjoint(20, every=20 if call == "one segment" else 6)
+        kept = h.history(P.HIST_FIELD_ENERGY, 0, 21)
+        h.save(path)
+        h.step(15)
+        a, d, fa = h.get_particles(), h.diagnostics(), h.history(P.HIST_FIELD_ENERGY, 0, 36)
+    with P.Handle(cfg) as h:
+        h.load(path)
+        h.step(15)
+        b, fb = h.get_particles(), h.history(P.HIST_FIELD_ENERGY, 21, 15)
+    for k in a:
+        np.testing.assert_array_equal(a[k], b[k], err_msg=k)
+    np.testing.assert_array_equal(fa[:21], kept)
+    np.testing.assert_array_equal(fa[21:], fb)
+    assert d.step == 35 and d.error_flags == 0 and d.total_charge_fixed == d.expected_charge_fixed
