@@ -465,20 +465,22 @@ static pic_status build_graphs(pic_handle *h)
         *g = nullptr;
     }
     const int S = h->cfg.sort_every;
-    const bool clear = h->rho_clear;  // capturing a solve runs none
-    PIC_TRY(capture(h, &G.one, [&] { return record_step(h, 0); }));
-    PIC_TRY(capture(h, &G.sortstep, [&] {
-        PIC_TRY(record_sort_all(h));
-        return record_step(h, 1);
-    }));
-    PIC_TRY(capture(h, &G.period, [&] {
-        PIC_TRY(record_sort_all(h));
-        PIC_TRY(record_step(h, 1));
-        for (int k = 1; k < S; ++k) PIC_TRY(record_step(h, 0));
-        return PIC_OK;
-    }));
+    const bool clear = h->rho_clear;  // capturing a push or a solve runs none
+    pic_status s = capture(h, &G.one, [&] { return record_step(h, 0); });
+    if (s == PIC_OK)
+        s = capture(h, &G.sortstep, [&] {
+            PIC_TRY(record_sort_all(h));
+            return record_step(h, 1);
+        });
+    if (s == PIC_OK)
+        s = capture(h, &G.period, [&] {
+            PIC_TRY(record_sort_all(h));
+            PIC_TRY(record_step(h, 1));
+            for (int k = 1; k < S; ++k) PIC_TRY(record_step(h, 0));
+            return PIC_OK;
+        });
     h->rho_clear = clear;
-    return PIC_OK;
+    return s;
 }
 
 static pic_status need(pic_handle *h)
@@ -1031,6 +1033,8 @@ pic_status pic_step(pic_handle *h, long long nsteps)
         return PIC_ERR_STATE;
     }
     PIC_TRY(build_graphs(h));
+    if (nsteps == 0) return PIC_OK;
+    PIC_TRY(clear_rho(h));  // of a deposit that no solve followed
     const pic_handle::StepGraphs &G = h->graphs[h->mixed && h->library_solve];
     const int S = h->cfg.sort_every;
     long long n = nsteps;
@@ -1052,7 +1056,7 @@ pic_status pic_step(pic_handle *h, long long nsteps)
         }
     }
     h->steps_host += nsteps;
-    if (nsteps > 0) h->rho_clear = true;
+    h->rho_clear = true;
     return PIC_OK;
 }
 

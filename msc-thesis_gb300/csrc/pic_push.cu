@@ -199,6 +199,7 @@ static pic_status launch_push_args(pic_handle *h, int s, bool deposit, PushArgs 
     const size_t sm = push_smem(g);
     PIC_TRY(allow_dynamic_smem(k, sm));
     void *args[] = {&A};
+    if (dep) h->rho_clear = false;
     return launch_dependent(k, (unsigned)B.nchunks, 256, sm, h->stream, args);
 }
 

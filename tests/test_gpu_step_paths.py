@@ -78,3 +78,24 @@ def test_a_reload_with_another_count_steps_as_a_fresh_handle():
                 h.step(7)
             got.append((h.get_particles(0), h.grid(P.GRID_RHO)))
     same(*got)
+
+
+@pytest.mark.parametrize("before", ["deposit", "gather_push"])
+def test_steps_after_a_deposit_without_a_solve(before):
+    """A density that was deposited and never solved for is not counted twice
+    by the step that follows."""
+    n = NX * NX * 16
+    w = L * L / n
+    with P.Handle(P.config(NX, NX, L, L, DT, [P.species(n, -w, w, -1)])) as h:
+        h.set_particles(0, *load(n, 8))
+        h.prime_leapfrog()
+        getattr(h, before)()
+        h.step(1)
+        d = h.diagnostics()
+        assert d.error_flags == 0 and d.total_charge_fixed == d.expected_charge_fixed
+        if before == "deposit":
+            got = h.get_particles(0), h.rho_fixed()
+            h.set_particles(0, *load(n, 8))
+            h.prime_leapfrog()
+            h.step(1)
+            same(got, (h.get_particles(0), h.rho_fixed()))
