@@ -547,9 +547,26 @@ pic_status ensure_stage(pic_handle *h, size_t bytes)
     return PIC_OK;
 }
 
+// The host's counts of the species that collisions have added to.
+static pic_status sync_counts(pic_handle *h)
+{
+    bool any = false;
+    for (const SpeciesBuf &B : h->sp) any = any || B.grows;
+    if (!any) return PIC_OK;
+    long long n[PIC_MAX_SPECIES];
+    PIC_CUDA(cudaStreamSynchronize(h->stream));
+    PIC_CUDA(cudaMemcpy(n, h->dev->n, sizeof n, cudaMemcpyDeviceToHost));
+    for (int s = 0; s < PIC_MAX_SPECIES; ++s)
+        if (h->sp[s].grows) h->sp[s].n = std::min(n[s], h->sp[s].cap);
+    return PIC_OK;
+}
+
 static pic_status set_count(pic_handle *h, int s, long long n)
 {
+    // of every species: the load that follows resets the device's counts from them
+    PIC_TRY(sync_counts(h));
     SpeciesBuf &B = h->sp[s];
+    B.grows = h->mcc.on && (s == h->mcc.e || s == h->mcc.i);
     const long long old4 = (B.n + 3) & ~3ll;
     B.n = n;
     const int chunk = B.chunk;
@@ -965,6 +982,7 @@ pic_status pic_particles_device(pic_handle *h, int s, pic_particles_view *v)
 {
     PIC_TRY(need_species(h, s));
     if (!v) return PIC_ERR_INVALID_ARG;
+    PIC_TRY(sync_counts(h));
     const SpeciesBuf &B = h->sp[s];
     v->n = B.n;
     v->cell_dev = B.cell[0];
@@ -1262,6 +1280,8 @@ extern "C" pic_status pic_set_mcc(pic_handle *h, const pic_mcc_params *p)
     M.seed = p->seed;
     M.on = true;
     drop_graphs(h);
+    for (int s : {M.e, M.i})
+        if (s >= 0) h->sp[s].grows = true;
     return PIC_OK;
 }
 

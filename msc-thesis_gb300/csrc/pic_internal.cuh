@@ -146,6 +146,7 @@ struct SpeciesBuf {
     int32_t *anchor = nullptr;  // per push chunk: tile (tx | ty << 16) or -1
     long long cap = 0;          // allocated slots (multiple of 4)
     long long n = 0;            // host mirror of the count
+    bool grows = false;         // collisions add to the device's count (sync_counts)
     int chunk = 0;              // particles per push block (push_chunk)
     long long nchunks = 0;      // push grid size for this species
     bool records_ready = false; // import keys and records already in the stage

@@ -133,3 +133,35 @@ def test_mcc_inside_the_step_small():
     assert c[0] > 0
     assert (q == 0.0).all() and d.total_charge_fixed == d.expected_charge_fixed
     assert d.n[0] - n == d.n[1] - n == c[2]
+
+
+def test_loads_after_births_replace_one_species_and_keep_the_other():
+    """A species loaded again after ionisation has added to it holds what a
+    fresh handle would, and the other species all of its newborn particles."""
+    n, dt = 2001, 2e-10
+    with mcc_handle(n, 200.0, dt, nx=64) as h:
+        fresh = h.get_particles(0, vz=True)
+        set_tabulated_mcc(h, 5)
+        h.prime_leapfrog()
+        h.step(80)
+        d = h.diagnostics()
+        born = h.collision_counts()[2]
+        assert born > n and d.n[0] == d.n[1] == n + born and h.particles_device(1).n == n + born
+    ve = np.sqrt(200.0 * E_CH / ME)
+    with mcc_handle(n, 200.0, dt, nx=64) as h:
+        set_tabulated_mcc(h, 5)
+        h.prime_leapfrog()
+        h.step(80)
+        h.synchronize()
+        raw = h.get_particles_raw(1)  # (reads no count into the handle)
+        h.init_particles(0, P.init_spec(n, vth=(ve, ve, ve), seed=11))
+        again = h.get_particles(0, vz=True)
+        now = h.get_particles_raw(1)
+        d = h.diagnostics()
+    assert len(raw["pid"]) > 2 * n and d.n[0] == n and d.n[1] == len(raw["pid"]) and d.error_flags == 0
+    for k in fresh:
+        np.testing.assert_array_equal(again[k], fresh[k], err_msg=k)
+    by_id = [np.argsort(r["pid"]) for r in (raw, now)]
+    for k in raw:
+        np.testing.assert_array_equal(raw[k][by_id[0]], now[k][by_id[1]], err_msg=k)
+    assert d.total_charge_fixed == d.expected_charge_fixed == (d.n[1] - d.n[0]) << 32
