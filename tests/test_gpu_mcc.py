@@ -165,3 +165,37 @@ def test_loads_after_births_replace_one_species_and_keep_the_other():
     for k in raw:
         np.testing.assert_array_equal(raw[k][by_id[0]], now[k][by_id[1]], err_msg=k)
     assert d.total_charge_fixed == d.expected_charge_fixed == (d.n[1] - d.n[0]) << 32
+
+
+@pytest.mark.parametrize("chunk", [0, 256])
+def test_newborn_particles_are_pushed_beyond_the_loaded_blocks(chunk):
+    """Species that grow to many times the loaded count, with the collisions
+    configured after the load and a second load after them: every particle is
+    in the density, and every electron moves."""
+    nx, n, cap, dt = 64, 2001, 80000, 2e-10
+    L, w = nx * DX, 1e4
+    sp = [P.species(cap, -E_CH * w, ME * w, -1, P.SPECIES_HAS_VZ),
+          P.species(cap, E_CH * w, MI * w, 1, P.SPECIES_HAS_VZ)]
+    cfg = P.config(nx, nx, L, L, dt, sp, eps0=8.8541878128e-12, sort_every=7, chunk=chunk, tile_w=16, tile_h=16)
+    ve, vi = np.sqrt(200.0 * E_CH / ME), np.sqrt(TN_EV * E_CH / MI)
+    with P.Handle(cfg) as h:
+        for seed in (1, 2):
+            h.init_particles(0, P.init_spec(n, vth=(ve, ve, ve), seed=seed))
+            h.init_particles(1, P.init_spec(n, vth=(vi, vi, vi), seed=seed))
+            if seed == 1:
+                set_tabulated_mcc(h, 5)
+            h.prime_leapfrog()
+            h.step(160)
+            d = h.diagnostics()
+            print("electrons", d.n[0], "of", n)
+            assert d.error_flags == 0 and 4 * n < d.n[0] < cap
+            a, ions = h.get_particles_raw(0), h.get_particles_raw(1)
+            rho = sum(O.deposit_fixed(nx, nx, r["cell"], r["ox"], r["oy"], q) for r, q in ((a, -1), (ions, 1)))
+            np.testing.assert_array_equal(h.rho_fixed(), np.reshape(rho, (nx, nx)))
+            h.step(1)
+            b = h.get_particles_raw(0)
+            place = {k: np.empty((d.n[0], 3)) for k in "ab"}
+            for k, r in (("a", a), ("b", b)):
+                old = r["pid"] < d.n[0]  # not those of this step
+                place[k][r["pid"][old]] = np.stack([r["cell"], r["ox"], r["oy"]], 1)[old]
+            assert (place["a"] != place["b"]).any(1).all()

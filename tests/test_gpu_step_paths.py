@@ -99,3 +99,33 @@ def test_steps_after_a_deposit_without_a_solve(before):
             h.prime_leapfrog()
             h.step(1)
             same(got, (h.get_particles(0), h.rho_fixed()))
+
+
+def test_a_mostly_empty_handle_steps_as_fast_as_a_full_one():
+    """A step's cost follows the particles, not the room for them: 16 per cell
+    on 64^2 in a handle for 64 M (which took six times as long with a block
+    for every 1024 slots; the bound leaves a factor of two for noise)."""
+    import torch
+
+    n = NX * NX * 16
+    w = L * L / n
+    best, got = [], []
+    for cap in (n, 1 << 26):
+        with P.Handle(P.config(NX, NX, L, L, DT, [P.species(cap, -w, w, -1)], sort_every=200)) as h:
+            h.set_particles(0, *load(n, 9))
+            h.prime_leapfrog()
+            h.step(1)
+            st = torch.cuda.ExternalStream(h.stream())
+            times = []
+            for _ in range(5):
+                a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+                a.record(st)
+                h.step(30)
+                b.record(st)
+                h.synchronize()
+                times.append(a.elapsed_time(b))
+            best.append(min(times))
+            got.append((h.get_particles(0), h.rho_fixed()))
+    print("ms for 30 steps", best)
+    same(*got)
+    assert best[1] < 2.0 * best[0]
