@@ -196,25 +196,37 @@ static pic_status validate(const pic_config *c, pic_handle *h)
     return PIC_OK;
 }
 
-// Particles per push block for n particles at ppc per cell where the caller
-// leaves it open.  Blocks of one size fill whole waves of the resident
-// blocks (four per SM): as few waves as keep a block at most 13824 particles
-// (its window stays small against them) and at most `limit` (about one and
-// a third of the particles of its tile, so that a block rarely reaches a
-// third tile), and at least 1024 (one pass of its threads).  What one wave
-// of more than 6912 would hold goes into several of at most 4608: a block that
-// goes on into the next tile row, whose tile is no neighbour, sends that part
-// through the global path, and a single wave waits for it (four loads each,
-// 512^2 x 32 per cell 95 to 104 us a step with 13800, 94.7 with 4600; 256^2 x
-// 100 76 to 80 with 10780, 74.6 with 3600; 512^2 x 20 72 to 74 with 8620, 71.4
-// with 4310; but 512^2 x 16 59 to 64 with 6900, 62 with 3450, 256^2 x 64 50 to 53
-// and 53.3, and in two waves 1024^2 x 16 164 with 13800, 174 with 6900).  us per step with
-// 8192 for all sizes before: 64^2 x 16 per cell 42.0 -> 21.9, 128^2 x 32 41.5
-// -> 26.3, 250 x 180 x 23 49.9 -> 36.3, 128^2 x 100 45.3 -> 35.2, 256^2 x 32
-// 53.2 -> 40.5, 512^2 x 32 109 -> 100, 1024^2 x 32 317 -> 308.
-static int push_chunk(long long n, double limit)
+// Particles per push block for n particles on `cells` cells where the caller
+// leaves it open.
+//
+// Up to about two waves of the resident blocks (four per SM) the blocks fill
+// whole waves: as few as keep a block at most 13824 particles (its window stays
+// small against them) and at most `limit` (about one and a third of the
+// particles of its tile, so that a block rarely reaches a third tile), and at
+// least 1024 (one pass of its threads).  What one wave of more than 6912 would
+// hold goes into several of at most 4608: a block that goes on into the next
+// tile row, whose tile is no neighbour, sends that part through the global path,
+// and a single wave waits for it (four loads each, 512^2 x 32 per cell 95 to 104
+// us a step with 13800, 94.7 with 4600; 256^2 x 100 76 to 80 with 10780, 74.6
+// with 3600; 512^2 x 20 72 to 74 with 8620, 71.4 with 4310; but 512^2 x 16 59 to
+// 64 with 6900, 62 with 3450, 256^2 x 64 50 to 53 and 53.3, and in two waves 1024^2
+// x 10 132 with 8620, 147 with 8192).  us per step with 8192 for all sizes
+// before: 64^2 x 16 per cell 42.0 -> 21.9, 128^2 x 32 41.5 -> 26.3, 250 x 180 x 23
+// 49.9 -> 36.3, 128^2 x 100 45.3 -> 35.2, 256^2 x 32 53.2 -> 40.5, 512^2 x 20 79.5 ->
+// 69.5, 512^2 x 32 109 -> 100.
+//
+// In more waves the last one matters less than blocks that hold their tile's
+// particles: 8192 and tiles of as many, unless those would cover more than 690
+// cells (their windows crowd the SM: 2048^2 x 10 per cell 440 us with whole waves
+// of 8620, 488 with 8192).  Two-stream and Landau loads, whole waves and 8192:
+// 700x640 x 32 206 and 196, 152 and 146; 512^2 x 128 338 and 330, 278 and 262;
+// 1024^2 x 40 572 and 562, 369 and 347; 2048^2 x 25 1956 and 1808, 852 and 847.
+// The line lies at 2.2 waves of 8192, between 512^2 x 40 (2.1: 130 and 132, 110
+// and 113) and 700x640 x 25 (2.25: 172 and 166, 128 and 128).
+static int push_chunk(long long n, double cells, double limit)
 {
     const double per = std::ceil((double)std::max(1ll, n) / (4.0 * device_sms()));
+    if (per > 2.2 * 8192.0 && 690.0 * (double)n >= 8192.0 * cells) return 8192;
     const double most = per > 13824.0 ? 13824.0 : per <= 6912.0 ? 6912.0 : 4608.0;
     const double waves = std::ceil(per / std::min(most, std::max(1024.0, limit)));
     return std::max(1024, ((int)std::ceil(per / waves) + 3) & ~3);
@@ -231,8 +243,8 @@ static void set_chunk(pic_handle *h, int s, long long n)
 {
     const Geometry &g = h->g;
     SpeciesBuf &B = h->sp[s];
-    const double tile = (double)g.tw * g.th * (double)n / ((double)g.nx * g.ny);
-    B.chunk = h->cfg.chunk ? h->cfg.chunk : push_chunk(n, 1.35 * tile);
+    const double cells = (double)g.nx * g.ny, tile = (double)g.tw * g.th * (double)n / cells;
+    B.chunk = h->cfg.chunk ? h->cfg.chunk : push_chunk(n, cells, 1.35 * tile);
     if (B.grows && !h->cfg.chunk && B.cap > 64ll * device_sms() * B.chunk) B.chunk = std::max(B.chunk, 8192);
     const long long slots = B.grows ? B.cap : n;
     B.nchunks = std::max((slots + B.chunk - 1) / B.chunk, B.cap ? 1ll : 0ll);
@@ -287,7 +299,7 @@ static pic_status setup_geometry(pic_handle *h)
         // 32: its window fits four blocks per SM), unless its divisors of nx
         // and ny make a worse window than 8192's
         const Geometry base = g;
-        const size_t smem = lay(push_chunk(maxcap, 690.0 * ppc));
+        const size_t smem = lay(push_chunk(maxcap, (double)c.nx * c.ny, 690.0 * ppc));
         if (smem > WINDOW_SMEM_TARGET || g.halo < base.halo) g = base;
     }
     return PIC_OK;

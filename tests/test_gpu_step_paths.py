@@ -129,3 +129,18 @@ def test_a_mostly_empty_handle_steps_as_fast_as_a_full_one():
     print("ms for 30 steps", best)
     same(*got)
     assert best[1] < 2.0 * best[0]
+
+
+@pytest.mark.parametrize("nx,ny,ppc", [(512, 512, 64), (700, 640, 32), (1024, 512, 26)])
+def test_default_blocks_of_large_runs_hold_their_tile(nx, ny, ppc):
+    """From about two waves of blocks on the default is the layout of a chunk of
+    8192 (a few per cent faster there than whole waves of another size): the
+    same storage order after a sort."""
+    n = nx * ny * ppc + 3
+    w = L * L / n
+    order = []
+    for chunk in (0, 8192):
+        with P.Handle(P.config(nx, ny, L, L, DT, [P.species(n, -w, w, -1)], chunk=chunk)) as h:
+            h.init_particles(0, P.init_spec(n, vth=(0.1, 0.1, 0.0), seed=4))
+            order.append(h.get_particles_raw(0)["cell"])
+    np.testing.assert_array_equal(*order)
