@@ -339,8 +339,9 @@ pic_status pic_load(pic_handle *h, const char *path);
  * PIC_PERT_DENSITY; 0 for the other kinds).  The 2^-16 quantisation of the
  * deposit weights is not differentiated.  Device memory: 20 bytes per
  * particle slot per checkpoint plus `every` x (12 bytes per slot + 8 bytes
- * per cell) for the ring.  Leaves the handle at step nsteps, with the
- * history of the forward run.  No counterpart in the reference. */
+ * per cell) for the ring; up to 256 MiB of it stay with the handle for later
+ * calls, unless the environment variable PIC_STAGE_MAX_BYTES caps that.
+ * Leaves the handle at step nsteps, with the history of the forward run.  No counterpart in the reference. */
 typedef struct pic_adjoint_result {
     double J;           /* final field energy                                 */
     double dJ_dbeam_v;  /* d J / d(spec->beam_v)   (spec given)               */

@@ -107,8 +107,8 @@ namespace {
 
 // An adjoint run's device memory: one block, carved up by a layout that is
 // run twice (sizes, then addresses).  Up to ADJ_STAGE_MAX bytes lie in the
-// handle's stage, which later runs find in place; more is allocated for the
-// call alone.
+// handle's stage, which later runs find in place; more, or more than the
+// caller's budget for the stage (stage_fits), is allocated for the call alone.
 constexpr size_t ADJ_STAGE_MAX = 256ull << 20;
 
 struct AdjWork {
@@ -212,7 +212,7 @@ pic_status adjoint_run(pic_handle *h, const pic_init_spec *spec, long long nstep
         saved = W.take<DevState>(1);
     };
     layout();
-    if (W.used <= ADJ_STAGE_MAX) {
+    if (W.used <= ADJ_STAGE_MAX && stage_fits(h, W.used)) {
         PIC_TRY(ensure_stage(h, W.used));
         W.base = (char *)h->stage;
     } else {

@@ -187,3 +187,31 @@ def test_segments_and_scatter_windows_match_fp64(setup, nsteps, every, speed):
     # the bound of up to ten steps above; an FP32 position carries 15 times the
     # rounding of a displacement 15 times as long
     assert max(errs) < 1e-4 * speed
+
+
+def test_workspace_stays_within_the_stage_budget(setup, monkeypatch):
+    """With PIC_STAGE_MAX_BYTES an adjoint run gives its workspace back (some
+    30 MB here) and has the same gradients."""
+    import torch
+
+    cfg, q, m, ocfg = setup
+    n = cfg.species[0].capacity
+    every = -(-32_000_000 // (12 * n))
+
+    def go():
+        with P.Handle(cfg) as h:
+            two_beam_handle_state(h)
+            free = torch.cuda.mem_get_info()[0]
+            r, *g = h.adjoint(every, every=every)
+            return free - torch.cuda.mem_get_info()[0], r.J, g
+
+    go()  # libraries loaded
+    monkeypatch.setenv("PIC_STAGE_MAX_BYTES", str(1 << 20))
+    kept, J, g = go()
+    monkeypatch.delenv("PIC_STAGE_MAX_BYTES")
+    _, J2, g2 = go()
+    print("bytes kept", kept)
+    assert kept < 8 << 20
+    assert J == J2
+    for a, b in zip(g, g2):  # the order of float sums over a long run; a wrong array is off by one
+        assert rel_norm(a, b) < 1e-3
