@@ -81,7 +81,10 @@ typedef struct pic_ref_params {
  * positions back.  *seconds (may be NULL) receives the elapsed time of the
  * whole call, as picFloatGpu returns it.  Unlike picFloatGpu the deposit
  * is atomic, the density is zeroed each step and forceOld starts at zero for
- * every particle, so the result follows the reference's CPU path. */
+ * every particle, so the result follows the reference's CPU path.  Device
+ * memory: 88 bytes per particle, 56 where that does not fit or exceeds the
+ * environment variable PIC_STAGE_MAX_BYTES (the CIC weights are then computed
+ * twice a step). */
 pic_status pic_compat_run(const pic_ref_params *p, const double *posX, const double *posY,
                           const double *velX, const double *velY, double *xOut, double *yOut,
                           double *seconds);

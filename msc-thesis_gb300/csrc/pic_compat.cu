@@ -42,7 +42,7 @@ struct CompatDev {
     long long np;
     double *px, *py, *vx, *vy;
     double *kox, *koy;       // dt/2 times the last force (the lagged half kick)
-    double *w;               // four CIC weights per particle, planes of np
+    double *w;               // four CIC weights per particle, planes of np, or null (KEPT)
     int2 *cell;
     double *rho;             // padded
     double2 *e;              // padded: Ex, Ey (ghosts stay zero)
@@ -90,35 +90,40 @@ __device__ __forceinline__ double wrap_ref(double x, double dim)
     return x;
 }
 
-// Cell and weights of a position, kept for the gather of the next push, and
-// with DEPOSIT the particle's charge.  Cells run 0..nx (a particle exactly at
-// x = xDim has cell nx); any other would index outside the padded grid: it is
-// kept as it is and the particle skipped.
-template <bool DEPOSIT>
-__device__ __forceinline__ void compat_place(const CompatDev &D, long long k, double X, double Yp)
+// CIC weights of a position in the cell whose indices are cx, cy
+__device__ __forceinline__ void compat_weights(const CompatDev &D, double X, double Yp, double cx, double cy,
+                                               double (&a)[4])
 {
-    double cx, cy;
-    const int ix = cell_of(X, D.dx, D.rdx, cx), iy = cell_of(Yp, D.dy, D.rdy, cy);
-    D.cell[k] = make_int2(ix, iy);
-    if ((unsigned)ix > (unsigned)D.nx || (unsigned)iy > (unsigned)D.ny) return;
     const double bx = __dmul_rn(cx, D.dx), by = __dmul_rn(cy, D.dy);
     const double lx = __dsub_rn(X, bx), ly = __dsub_rn(Yp, by);
     const double hx = __dsub_rn(__dadd_rn(bx, D.dx), X), hy = __dsub_rn(__dadd_rn(by, D.dy), Yp);
-    const double a1 = div_known(__dmul_rn(lx, ly), D.area, D.rarea);
-    const double a2 = div_known(__dmul_rn(hx, ly), D.area, D.rarea);
-    const double a3 = div_known(__dmul_rn(lx, hy), D.area, D.rarea);
-    const double a4 = div_known(__dmul_rn(hx, hy), D.area, D.rarea);
-    D.w[k] = a1;
-    D.w[k + D.np] = a2;
-    D.w[k + 2 * D.np] = a3;
-    D.w[k + 3 * D.np] = a4;
-    if (!DEPOSIT) return;
+    a[0] = div_known(__dmul_rn(lx, ly), D.area, D.rarea);
+    a[1] = div_known(__dmul_rn(hx, ly), D.area, D.rarea);
+    a[2] = div_known(__dmul_rn(lx, hy), D.area, D.rarea);
+    a[3] = div_known(__dmul_rn(hx, hy), D.area, D.rarea);
+}
+
+// Cell and weights of a position, kept for the gather of the next push, and
+// the particle's charge.  Cells run 0..nx (a particle exactly at x = xDim has
+// cell nx); any other would index outside the padded grid: it is kept as it is
+// and the particle skipped.
+template <bool KEPT>
+__device__ __forceinline__ void compat_place(const CompatDev &D, long long k, double X, double Yp)
+{
+    double cx, cy, a[4];
+    const int ix = cell_of(X, D.dx, D.rdx, cx), iy = cell_of(Yp, D.dy, D.rdy, cy);
+    D.cell[k] = make_int2(ix, iy);
+    if ((unsigned)ix > (unsigned)D.nx || (unsigned)iy > (unsigned)D.ny) return;
+    compat_weights(D, X, Yp, cx, cy, a);
+    if (KEPT)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) D.w[k + i * D.np] = a[i];
     const int ix1 = ix + 1 >= D.nx ? ix + 1 - D.nx : ix + 1, iy1 = iy + 1 >= D.ny ? iy + 1 - D.ny : iy + 1;
     double *r0 = D.rho + (size_t)(1 + ix) * D.Y, *r1 = D.rho + (size_t)(1 + ix1) * D.Y;
-    atomicAdd(r0 + 1 + iy, __dmul_rn(a1, D.q));
-    atomicAdd(r1 + 1 + iy, __dmul_rn(a2, D.q));
-    atomicAdd(r0 + 1 + iy1, __dmul_rn(a3, D.q));
-    atomicAdd(r1 + 1 + iy1, __dmul_rn(a4, D.q));
+    atomicAdd(r0 + 1 + iy, __dmul_rn(a[0], D.q));
+    atomicAdd(r1 + 1 + iy, __dmul_rn(a[1], D.q));
+    atomicAdd(r0 + 1 + iy1, __dmul_rn(a[2], D.q));
+    atomicAdd(r1 + 1 + iy1, __dmul_rn(a[3], D.q));
 }
 
 // Gather, lagged kick-drift-kick and the deposit of the new position for the
@@ -127,7 +132,10 @@ __device__ __forceinline__ void compat_place(const CompatDev &D, long long k, do
 // 128^2, 1.6 M particles: 220 us against 377 us for a push and 194 us for a
 // deposit that each computed cells and weights with general divisions; 64
 // FP64 operations per particle, 168 us at the pipe's rate.
-template <bool DEPOSIT>
+// !KEPT: the weights are computed again for the gather (the same operations on
+// the same position), where memory for them is short: 56 bytes per particle
+// instead of 88.
+template <bool DEPOSIT, bool KEPT>
 __global__ void compat_push_kernel(CompatDev D)
 {
     pdl_wait();
@@ -139,16 +147,21 @@ __global__ void compat_push_kernel(CompatDev D)
     const int ix1 = c.x + 1 >= D.nx ? c.x + 1 - D.nx : c.x + 1, iy1 = c.y + 1 >= D.ny ? c.y + 1 - D.ny : c.y + 1;
     const double2 *r0 = D.e + (size_t)c.x * D.Y, *r1 = D.e + (size_t)ix1 * D.Y;
     const double2 e1 = r0[c.y], e2 = r1[c.y], e3 = r0[iy1], e4 = r1[iy1];
-    const double a1 = D.w[k], a2 = D.w[k + D.np], a3 = D.w[k + 2 * D.np], a4 = D.w[k + 3 * D.np];
-    double fx = __dmul_rn(a1, e1.x);
-    fx = __dadd_rn(fx, __dmul_rn(a2, e2.x));
-    fx = __dadd_rn(fx, __dmul_rn(a3, e3.x));
-    fx = __dadd_rn(fx, __dmul_rn(a4, e4.x));
+    double a[4];
+    if (KEPT)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i] = D.w[k + i * D.np];
+    else
+        compat_weights(D, D.px[k], D.py[k], (double)c.x, (double)c.y, a);
+    double fx = __dmul_rn(a[0], e1.x);
+    fx = __dadd_rn(fx, __dmul_rn(a[1], e2.x));
+    fx = __dadd_rn(fx, __dmul_rn(a[2], e3.x));
+    fx = __dadd_rn(fx, __dmul_rn(a[3], e4.x));
     fx = __dmul_rn(fx, D.qm);
-    double fy = __dmul_rn(a1, e1.y);
-    fy = __dadd_rn(fy, __dmul_rn(a2, e2.y));
-    fy = __dadd_rn(fy, __dmul_rn(a3, e3.y));
-    fy = __dadd_rn(fy, __dmul_rn(a4, e4.y));
+    double fy = __dmul_rn(a[0], e1.y);
+    fy = __dadd_rn(fy, __dmul_rn(a[1], e2.y));
+    fy = __dadd_rn(fy, __dmul_rn(a[2], e3.y));
+    fy = __dadd_rn(fy, __dmul_rn(a[3], e4.y));
     fy = __dmul_rn(fy, D.qm);
     const double vxh = __dadd_rn(D.vx[k], D.kox[k]);
     const double vyh = __dadd_rn(D.vy[k], D.koy[k]);
@@ -161,18 +174,19 @@ __global__ void compat_push_kernel(CompatDev D)
     D.koy[k] = koy;
     D.px[k] = X;
     D.py[k] = Yp;
-    if (DEPOSIT) compat_place<true>(D, k, X, Yp);
+    if (DEPOSIT) compat_place<KEPT>(D, k, X, Yp);
 }
 
 // Particle::Particle (particle.cc:21-29): cell from position, forces zero;
 // and the first step's deposit.
+template <bool KEPT>
 __global__ void compat_setup_kernel(CompatDev D)
 {
     const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= D.np) return;
     D.kox[k] = 0.0;
     D.koy[k] = 0.0;
-    compat_place<true>(D, k, D.px[k], D.py[k]);
+    compat_place<KEPT>(D, k, D.px[k], D.py[k]);
 }
 
 // Periodic ghost copy of a padded grid, two loops as the reference runs them
@@ -582,7 +596,14 @@ static pic_status compat_core(const pic_ref_params *p, const double *x0, const d
     double2 *pool16 = nullptr;
     double *pool = nullptr;
     PIC_TRY(R.alloc(&pool16, n16));
-    PIC_TRY(R.alloc(&pool, 11 * np + 4 * ng));
+    // the weights (4 np) only where they fit the device and the caller's budget
+    const size_t lean = 7 * np + 4 * ng;
+    bool kept = stage_budget((lean + 4 * np) * sizeof(double));
+    if (kept && R.alloc(&pool, lean + 4 * np) != PIC_OK) {
+        cudaGetLastError();
+        kept = false;
+    }
+    if (!kept) PIC_TRY(R.alloc(&pool, lean));
     D.e = pool16;
     D.fout = (cufftDoubleComplex *)(D.e + ng);
     D.kmode = (double2 *)D.fout + nk;
@@ -596,8 +617,8 @@ static pic_status compat_core(const pic_ref_params *p, const double *x0, const d
     D.vy = D.vx + np;
     D.kox = D.vy + np;
     D.koy = D.kox + np;
-    D.w = D.koy + np;
-    D.rho = D.w + 4 * np;
+    D.w = kept ? D.koy + np : nullptr;
+    D.rho = D.koy + (kept ? 5 : 1) * np;
     double *dphi = D.rho + ng, *dex = dphi + ng, *dey = dex + ng;
     D.fin = (double *)(tw + p->nx + p->ny);
     PIC_CUDA(cudaMemsetAsync(D.e, 0, sizeof(double2) * ng, R.st));
@@ -627,7 +648,10 @@ static pic_status compat_core(const pic_ref_params *p, const double *x0, const d
     const int gg = grid_for((long long)n, 256);
     if (nsteps > 0) {
         compat_modes_kernel<<<grid_for((long long)nk, 256), 256, 0, R.st>>>(D);
-        compat_setup_kernel<<<gp, bt, 0, R.st>>>(D);
+        if (kept)
+            compat_setup_kernel<true><<<gp, bt, 0, R.st>>>(D);
+        else
+            compat_setup_kernel<false><<<gp, bt, 0, R.st>>>(D);
         PIC_CUDA(cudaGetLastError());
     }
     for (long long s = 0; s < nsteps; ++s) {
@@ -635,9 +659,11 @@ static pic_status compat_core(const pic_ref_params *p, const double *x0, const d
         int more = s + 1 < nsteps;
         void *ae[] = {&D, &more}, *ap[] = {&D};
         PIC_TRY(launch_dependent((const void *)compat_efield_kernel, gg, 256, 0, R.st, ae));
-        PIC_TRY(launch_dependent(more ? (const void *)compat_push_kernel<true>
-                                      : (const void *)compat_push_kernel<false>,
-                                 gp, bt, 0, R.st, ap));
+        const void *push = kept ? (more ? (const void *)compat_push_kernel<true, true>
+                                        : (const void *)compat_push_kernel<false, true>)
+                                : (more ? (const void *)compat_push_kernel<true, false>
+                                        : (const void *)compat_push_kernel<false, false>);
+        PIC_TRY(launch_dependent(push, gp, bt, 0, R.st, ap));
     }
     // the last step's grids
     compat_ghost_kernel<<<1, 1024, 0, R.st>>>(D.rho, D.nx, D.ny, 0);

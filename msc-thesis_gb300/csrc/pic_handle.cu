@@ -536,17 +536,24 @@ template <class T> static T *mapped(T *p)
     return a.type == cudaMemoryTypeHost ? (T *)a.devicePointer : nullptr;
 }
 
-// Whether the stage holds `bytes` now or can grow to it and leave 1 GiB of
-// device memory free (callers fall back to a leaner layout otherwise).  The
-// environment variable PIC_STAGE_MAX_BYTES caps the layouts chosen this way
-// for callers that keep a device-memory budget.
+// Whether a layout of `bytes` is within the environment variable
+// PIC_STAGE_MAX_BYTES, for callers that keep a device-memory budget (a leaner
+// layout is taken otherwise).
+bool stage_budget(size_t bytes)
+{
+    const char *cap = getenv("PIC_STAGE_MAX_BYTES");
+    if (!cap) return true;
+    char *end = nullptr;
+    const unsigned long long v = strtoull(cap, &end, 10);
+    return end == cap || bytes <= v;
+}
+
+// Whether the stage holds `bytes` now or can grow to it within the budget and
+// leave 1 GiB of device memory free (callers fall back to a leaner layout
+// otherwise).
 bool stage_fits(pic_handle *h, size_t bytes)
 {
-    if (const char *cap = getenv("PIC_STAGE_MAX_BYTES")) {
-        char *end = nullptr;
-        const unsigned long long v = strtoull(cap, &end, 10);
-        if (end != cap && bytes > v) return false;
-    }
+    if (!stage_budget(bytes)) return false;
     if (h->stage_bytes >= bytes) return true;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {

@@ -409,6 +409,7 @@ pic_status record_push_all(pic_handle *h, int src, bool deposit, bool fold = tru
 pic_status deposit_now(pic_handle *h);
 pic_status refresh(pic_handle *h);
 pic_status ensure_stage(pic_handle *h, size_t bytes);
+bool stage_budget(size_t bytes);
 bool stage_fits(pic_handle *h, size_t bytes);
 pic_status lattice_dims(pic_handle *h, long long n, int *lx, int *ly);
 pic_status lattice_dims_for(int nx, int ny, long long n, int *lx, int *ly);

@@ -83,3 +83,41 @@ def test_compat_grid_sizes_vs_restatement(nx, ny):
     for k in ("rho", "phi", "ex", "ey"):
         scale = max(np.abs(ref[k]).max(), 1e-300)
         np.testing.assert_allclose(out[k], ref[k], rtol=0, atol=1e-10 * scale, err_msg=k)
+
+
+@pytest.mark.parametrize("nx,ny", [(64, 64), (30, 20)])
+def test_short_memory_computes_the_weights_again(nx, ny, monkeypatch):
+    """Within PIC_STAGE_MAX_BYTES a run holds no weights per particle (at most 64
+    bytes each instead of 88) and agrees to the order of the deposit's sums."""
+    import threading
+
+    import torch
+
+    kw = dict(xDim=10, yDim=10, nx=nx, ny=ny, npx=2000, npy=1500, dt=0.01, tmax=1.0)
+    n = 3_000_000
+    rng = np.random.default_rng(nx)
+    state = [rng.uniform(0, 10, n), rng.uniform(0, 10, n), rng.normal(0, 1, n), rng.normal(0, 1, n)]
+
+    def go():
+        torch.cuda.synchronize()
+        free, least, stop = torch.cuda.mem_get_info()[0], [1 << 60], threading.Event()
+
+        def watch():
+            while not stop.is_set():
+                least[0] = min(least[0], torch.cuda.mem_get_info()[0])
+
+        t = threading.Thread(target=watch)
+        t.start()
+        out = P.compat_run_steps(P.ref_params(**kw), *state, 20)
+        stop.set()
+        t.join()
+        return out, free - least[0]
+
+    go()  # libraries loaded
+    ref, _ = go()
+    monkeypatch.setenv("PIC_STAGE_MAX_BYTES", str(1 << 20))
+    out, used = go()
+    print("bytes per particle", used / n)
+    assert used < 64 * n + (24 << 20)
+    for k in ("x", "y", "vx", "vy"):
+        np.testing.assert_allclose(out[k], ref[k], rtol=0, atol=1e-9, err_msg=k)
