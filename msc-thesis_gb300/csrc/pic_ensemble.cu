@@ -848,6 +848,7 @@ pic_status pic::ens_init(pic_ensemble *e, const pic_init_spec *specs, bool wide)
     cudaStream_t st = e->stream;
     PIC_CUDA(cudaStreamSynchronize(st));
     const size_t ns = (size_t)e->nslots;
+    e->ready = false;  // the graphs hold the block table that is replaced below
     for (int b = 0; b < 2; ++b) PIC_CUDA(cudaMemsetAsync(e->cell[b], 0xFF, ns * 4, st));
     ens_windows(e, specs, wide);
     PIC_TRY(ens_push_table(e, n_slot));
