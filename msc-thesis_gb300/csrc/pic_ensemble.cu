@@ -912,6 +912,19 @@ pic_status pic::ens_init(pic_ensemble *e, const pic_init_spec *specs, bool wide)
     return PIC_OK;
 }
 
+pic_status pic::ens_rewindow(pic_ensemble *E, const pic_init_spec *specs)
+{
+    ens_windows(E, specs, true);
+    if (E->push_threads == 256) return PIC_OK;  // narrow ones, as they were
+    std::vector<long long> n_slot;
+    for (const EnsRun &R : E->runs) n_slot.push_back(R.n);
+    E->ready = false;
+    PIC_TRY(ens_push_table(E, n_slot));
+    PIC_TRY(ens_graphs(E));
+    E->ready = true;
+    return PIC_OK;
+}
+
 extern "C" {
 
 pic_status pic_ensemble_step(pic_ensemble *e, long long nsteps)

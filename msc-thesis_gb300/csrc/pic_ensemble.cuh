@@ -121,6 +121,9 @@ pic_status ens_poisson(pic_ensemble *E, int adv = ADV_FIELD);
 // arrays xin -> xout when given), push-block anchors
 pic_status ens_sort(pic_ensemble *E, const float *const *xin = nullptr, float *const *xout = nullptr);
 pic_status ens_graphs(pic_ensemble *E);
+// the push windows that pic_ensemble_init would choose for these loads, after
+// ens_init without wide ones; a sort has to come before the next push
+pic_status ens_rewindow(pic_ensemble *E, const pic_init_spec *specs);
 // pic_ensemble_init; wide: push windows may be wide (see ens_windows)
 pic_status ens_init(pic_ensemble *E, const pic_init_spec *specs, bool wide);
 // pic_import.cu: every run, arbitrary order in buffer 0 -> key order in

@@ -648,6 +648,7 @@ pic_status ens_adjoint(pic_ensemble *E, const pic_init_spec *specs, long long ns
     PIC_CUDA(cudaMemcpyAsync(E->hist, hist_saved.data(), hist_n * 8, cudaMemcpyHostToDevice, st));
     PIC_CUDA(cudaStreamSynchronize(st));
     E->since_sort = std::max(since_saved, S);  // anchors are stale: sort before the next step
+    PIC_TRY(ens_rewindow(E, specs));           // the backward walk's windows were narrow
     if (out) {
         for (int r = 0; r < nr; ++r) {
             const int sidx = E->slot_of[r];

@@ -164,3 +164,37 @@ def test_gradient_export_fills_every_array(runs):
             errs = [rel_norm(a, b) for a, b in zip(g[r], sg)]
             print(f"run {r}: {max(errs):.2e}")
             assert max(errs) < 1e-4
+
+
+def test_steps_after_an_adjoint_are_as_fast_as_after_a_load():
+    """A large ensemble of fast runs steps with wide push windows, after an
+    adjoint too, whose own passes take narrow ones.  Once the beams are
+    thermal (t = 25) narrow windows take 1.6 times as long (278 and 172 us on
+    this load); the bound leaves a quarter for noise.  The particles are the
+    same, bit for bit."""
+    import torch
+
+    cfgs, specs, _ = setup([(256, 256, 256, 0.3, 1e-3, 31)])
+    times, got = [], []
+    for adjoint in (False, True):
+        with P.Ensemble(cfgs) as E:
+            if adjoint:
+                E.adjoint(specs, 10, 5, gradients=False)
+            else:
+                E.init(specs)
+                E.step(10)
+            E.step(250)
+            st, best = torch.cuda.ExternalStream(E.stream()), []
+            for _ in range(3):
+                a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+                a.record(st)
+                E.step(20)
+                b.record(st)
+                E.synchronize()
+                best.append(a.elapsed_time(b))
+            times.append(min(best))
+            got.append(E.get_particles(0))
+    print("ms for 20 steps", times)
+    for k in got[0]:
+        np.testing.assert_array_equal(got[0][k], got[1][k], err_msg=k)
+    assert times[1] < 1.25 * times[0]
