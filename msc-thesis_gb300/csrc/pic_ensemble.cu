@@ -383,17 +383,37 @@ pic_status ens_layout(pic_ensemble *E)
 // runs of up to 512^2 x 256 (209 M particles, a sort every 20 steps), us per
 // step at t < 4, t < 24 and t < 32: narrow 1734, 2676, 3458; wide 1571, 1733,
 // 1802 (blocks of at most 16384: 1684, 1859, 1941; tiles of at most 256 cells:
-// 1599, 1759, 1830; halos of half the drift: 1687, 1803, 1899).  They need
-// particles to fill their blocks (8 runs of up to 256^2 x 64, 10 M particles:
-// 103 us narrow, 110 wide) and fast ones; so they are taken when three
-// quarters of at least 12 M particles belong to runs of 32 or more per cell
-// that drift four cells or more between sorts, and then for every run (the
-// other runs on narrow windows: 1656 us per step instead of 1571).  A block of
-// a dense run then holds just its tile's particles; sized to whole waves
-// instead, blocks straddle two tiles: 1635 us.
+// 1599, 1759, 1830; halos of half the drift: 1687, 1803, 1899).  A block of a
+// dense run then holds just its tile's particles; sized to whole waves instead,
+// blocks straddle two tiles: 1635 us.
+//
+// They pay by the particles that a narrow window loses, which grow with a run's
+// density and drift, and cost by blocks too large to fill the last wave of few
+// particles.  So they are taken when three quarters of the particles belong to
+// runs of 32 or more per cell that drift four cells or more between sorts, and
+// those runs' sum of particles x particles per cell x cells of drift reaches
+// 1.4e10, or 1e10 for 30 M particles and more; and then for every run (the other
+// runs on narrow windows: 1656 us per step instead of 1571).  us per step at
+// t = 2, 16 and 32, narrow and wide, of two-stream runs, with that sum in 1e10
+// (the drift counts 4 thermal speeds):
+//   6.0  33.6 M, 512^2 x 64, 28 cells   323 412 562   347 350 372
+//   5.1  33.6 M, 128^2 x 256, 6 cells   280 336 391   273 283 273
+//   4.2  33.6 M, 256^2 x 128, 10 cells  287 355 429   284 291 293
+//   2.5  16.8 M, 128^2 x 256, 6 cells   150 180 208   155 171 159
+//   2.4  67.1 M, 256^2 x 64, 6 cells    561 589 597   549 551 548
+//   2.1  16.8 M, 256^2 x 128, 10 cells  155 191 229   161 168 175
+//   1.6  12.6 M, 128^2 x 256, 5 cells   117 134 146   129 137 131
+//   1.5  16.8 M, 256^2 x 64, 14 cells   162 200 233   184 198 200
+//   1.2  33.6 M, 512^2 x 32, 11 cells   317 346 362   325 330 334
+//   1.1  33.6 M, 256^2 x 32, 10 cells   323 348 367   326 331 339
+//   1.2  16.8 M, 256^2 x 128, 6 cells   151 163 168   165 182 174
+//   1.1  16.8 M, 256^2 x 64, 10 cells   160 182 198   179 185 188
+//   0.7  16.8 M, 256^2 x 32, 14 cells   175 199 217   197 210 210
+//   0.6  33.6 M, 256^2 x 32, 6 cells    308 317 322   323 331 328
 struct RunDrift {
     double ppc, x, y;  // particles per cell; cells crossed in a sort period
-    bool fast() const { return ppc >= 32.0 && std::max(x, y) >= 4.0; }
+    double cells() const { return std::max(x, y); }
+    bool fast() const { return ppc >= 32.0 && cells() >= 4.0; }
 };
 
 static RunDrift run_drift(const pic_ensemble *E, int s, const pic_init_spec &S)
@@ -409,12 +429,16 @@ static RunDrift run_drift(const pic_ensemble *E, int s, const pic_init_spec &S)
 void ens_windows(pic_ensemble *E, const pic_init_spec *specs, bool allow_wide)
 {
     long long total = 0, fast = 0;
+    double lost = 0.0;
     for (int s = 0; s < E->nruns; ++s) {
         const pic_init_spec &S = specs[E->run_of[s]];
+        const RunDrift D = run_drift(E, s, S);
         total += S.n;
-        if (run_drift(E, s, S).fast()) fast += S.n;
+        if (!D.fast()) continue;
+        fast += S.n;
+        lost += (double)S.n * D.ppc * D.cells();
     }
-    const bool wide = allow_wide && total >= 12000000 && 4 * fast >= 3 * total;
+    const bool wide = allow_wide && 4 * fast >= 3 * total && lost >= (total >= 30000000 ? 1.0e10 : 1.4e10);
     E->push_threads = wide ? 512 : 256;
     E->push_smem = 0;
     E->per.assign(E->nruns, E->chunk);

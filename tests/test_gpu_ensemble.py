@@ -270,3 +270,25 @@ def test_histories_of_several_grid_sizes_match_single_handles(runs):
         np.testing.assert_allclose(ens[r][mx], one[mx], rtol=0, atol=scale)
         np.testing.assert_allclose(ens[r][my], one[my], rtol=0, atol=scale)
         np.testing.assert_array_equal(ens[r][q], one[q])
+
+
+@pytest.mark.parametrize("runs", [[(128, 128, 400, 0.3, 1e-3, 81), (128, 64, 700, 0.35, 1e-2, 82), (64, 64, 20, 0.0, 1e-3, 83)],
+                                  [(256, 256, 64, 0.2, 1e-3, 84 + r) for r in range(4)],
+                                  [(256, 256, 64, 0.2, 1e-3, 88 + r) for r in range(8)]])
+def test_either_side_of_the_window_rule(runs):
+    """Dense fast runs (wide windows), sparser ones too few for them, and twice as
+    many, which take them: the particles of single handles, bit for bit."""
+    cfgs, specs = build(runs, sort_every=20)
+    with P.Ensemble(cfgs) as E:
+        E.init(specs)
+        E.step(50)
+        assert all(E.diagnostics(r).error_flags == 0 for r in range(len(runs)))
+        ens = {r: E.get_particles(r) for r in (0, len(runs) - 1)}
+    for r in ens:
+        with P.Handle(cfgs[r]) as h:
+            h.init_particles(0, specs[r])
+            h.prime_leapfrog()
+            h.step(50)
+            a = h.get_particles(0)
+        for k in a:
+            np.testing.assert_array_equal(ens[r][k], a[k], err_msg=f"run {r} {k}")
