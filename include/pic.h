@@ -420,8 +420,14 @@ pic_status pic_get_history(pic_handle *h, int which, long long first, long long 
  * Run r follows runs[r]: nx, ny, Lx, Ly, dt, eps0 and species[0] (one
  * charged species: capacity, q, m, q_int); its sort tiles are chosen from
  * its particles per cell.  chunk, halo, sort_every, history and device are
- * taken from runs[0] (0: the handle defaults).  A run gives the same
- * particles as a handle created from runs[r] and stepped alike.  No
+ * taken from runs[0] (0: chunk from the particle count, at most 8192; the
+ * handle defaults otherwise).  chunk sets the tiles and push blocks of ordinary
+ * loads; where most particles belong to dense runs that cross many cells
+ * between sorts (tens of millions of them), tiles and blocks follow the loads
+ * whatever chunk says.  A run gives the same particles as a handle created
+ * from runs[r] and stepped alike, where every side of the ensemble is a power
+ * of two; otherwise all of its runs solve through cuFFT, and agree to
+ * rounding with handles that do not.  No
  * counterpart in the reference (it runs one simulation per process). */
 typedef struct pic_ensemble pic_ensemble;
 pic_status pic_ensemble_create(const pic_config *runs, int nruns, pic_ensemble **out);
@@ -457,8 +463,8 @@ pic_status pic_ensemble_adjoint(pic_ensemble *e, const pic_init_spec *specs, lon
                                 double *dJ_dvy0, pic_adjoint_result *out);
 /* Pick the push chunk (and with it every run's sort tile) and the sort
  * cadence of an ensemble by timing short runs of it, as pic_autotune does
- * for one handle: chunk from (2048, 4096, 8192, 16384), then cadence from
- * (1, 2, 3, 5, 10, 20).  The chosen chunk and sort_every are written into
+ * for one handle: chunk from (2048, 4096, 8192, 16384; or 0, where the loads
+ * set the blocks whatever chunk says), then cadence from (1, 2, 3, 5, 10, 20).  The chosen chunk and sort_every are written into
  * runs[0]; out->tile_w/tile_h are 0 (tiles differ per run).  Needs the
  * memory of one ensemble at a time. */
 pic_status pic_ensemble_autotune(pic_config *runs, int nruns, const pic_init_spec *specs,

@@ -1081,12 +1081,14 @@ pic_status pic_ensemble_get_particles(pic_ensemble *e, int run, long long *n, do
 // ------------------------------------------------------------------ autotuner
 namespace {
 
+// wide: whether the loads took wide push windows, whose blocks do not follow the chunk
 pic_status ens_time_candidate(const std::vector<pic_config> &runs, const pic_init_spec *specs,
-                              int trial_steps, double *ms)
+                              int trial_steps, double *ms, bool *wide)
 {
     pic_ensemble *e = nullptr;
     PIC_TRY(pic_ensemble_create(runs.data(), (int)runs.size(), &e));
     pic_status st = pic_ensemble_init(e, specs);
+    *wide = e->push_threads == 512;
     const int S = e->sort_every;
     const long long steps = ((long long)(trial_steps + S - 1) / S) * S;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -1127,7 +1129,8 @@ extern "C" pic_status pic_ensemble_autotune(pic_config *runs, int nruns, const p
     for (int c : {2048, 4096, 8192, 16384}) {
         cur[0].chunk = c;
         double ms = 0.0;
-        const pic_status st = ens_time_candidate(cur, specs, trial_steps, &ms);
+        bool wide = false;
+        pic_status st = ens_time_candidate(cur, specs, trial_steps, &ms, &wide);
         if (st == PIC_ERR_INVALID_ARG) continue;  // a run's window too large for this chunk
         if (st != PIC_OK) return st;
         ++tried;
@@ -1135,6 +1138,18 @@ extern "C" pic_status pic_ensemble_autotune(pic_config *runs, int nruns, const p
             best_ms = ms;
             best_chunk = c;
         }
+        if (!wide) continue;
+        // no chunk to choose here: left to the loads, where that is accepted
+        cur[0].chunk = 0;
+        st = ens_time_candidate(cur, specs, trial_steps, &ms, &wide);
+        if (st == PIC_OK) {
+            ++tried;
+            best_ms = ms;
+            best_chunk = 0;
+        } else if (st != PIC_ERR_INVALID_ARG) {
+            return st;
+        }
+        break;
     }
     if (!tried) {
         set_error("pic_ensemble_autotune: no candidate could be created");
@@ -1146,7 +1161,8 @@ extern "C" pic_status pic_ensemble_autotune(pic_config *runs, int nruns, const p
         if (se == first_se) continue;
         cur[0].sort_every = se;
         double ms = 0.0;
-        PIC_TRY(ens_time_candidate(cur, specs, trial_steps, &ms));
+        bool wide = false;
+        PIC_TRY(ens_time_candidate(cur, specs, trial_steps, &ms, &wide));
         ++tried;
         if (ms < best_ms) {
             best_ms = ms;

@@ -292,3 +292,15 @@ def test_either_side_of_the_window_rule(runs):
             a = h.get_particles(0)
         for k in a:
             np.testing.assert_array_equal(ens[r][k], a[k], err_msg=f"run {r} {k}")
+
+
+def test_autotuner_leaves_the_chunk_to_loads_that_set_their_blocks():
+    """Dense fast runs take their push blocks from the load whatever the chunk:
+    the tuner times no chunks against each other there."""
+    cfgs, specs = build([(128, 128, 400, 0.3, 1e-3, 91), (128, 64, 700, 0.35, 1e-2, 92)], chunk=4096)
+    r = P.ensemble_autotune(cfgs, specs, trial_steps=5)
+    assert r.chunk == cfgs[0].chunk == 0 and cfgs[0].sort_every == r.sort_every
+    assert r.tried == 2 + 5  # the first chunk and none, then the other cadences
+    cfgs, specs = build(RUNS)
+    r = P.ensemble_autotune(cfgs, specs, trial_steps=5)
+    assert r.chunk in (2048, 4096, 8192, 16384) and r.tried > 5
