@@ -99,26 +99,35 @@ __device__ __forceinline__ float fixed_sum(const unsigned *m, float inv_scale)
 // compare-and-swap loops.  A first pass over the block's adjoint velocities
 // finds their largest magnitude, which sets the scale (31 bits for the largest
 // mu, at most 32768 particles a block: the 16-bit halves cannot overflow); it
-// also brings the four arrays into L2 for the second.  Sums are exact to
-// 2^-32 of the block's largest mu and independent of order.  Blocks whose
-// largest value is not finite or too small to scale, and particles outside
-// the window, add to the grid in float.  8 runs of up to 256^2 x 64 (10.3 M
-// particles): 171 us against 316 us with float sums over a warp's equal cells
-// first and compare-and-swap adds of the rest (60 bytes per particle: 91 us).
+// also brings the four arrays into L2 for the second.  A contribution is rounded
+// to 2^-31 of the largest at most, and the sums are exact from there and
+// independent of order.  So that a few values far above the others do not
+// take their bits, the largest counts as no more than 2^KICK_SPAN times the
+// geometric mean (by the mean exponent of the nonzero values; it is 2^2 to 2^5
+// times that in ordinary runs): the rounding is then below 2^-24 of that mean, as
+// a float's is of values of its size.  Particles above that, blocks whose largest value is not finite or too small
+// to scale, and particles outside the window add to the grid in float.  8 runs
+// of up to 256^2 x 64 (10.3 M particles): 171 us against 316 us with float sums
+// over a warp's equal cells first and compare-and-swap adds of the rest (60
+// bytes per particle: 91 us).
+constexpr int KICK_SPAN = 6;
+
 template <bool UNKICK>
 __device__ __forceinline__ void adj_kick_block(const KickArgs &A, const KickGeo &K,
                                                unsigned char *smem, long long base, long long end,
                                                int anc)
 {
-    __shared__ unsigned s_max;
+    __shared__ unsigned s_max, s_exp, s_cnt;
     const PushGeo &G = K.G;
     const Window W = setup_window(G, smem, anc);
-    if (threadIdx.x == 0) s_max = 0u;
+    if (threadIdx.x == 0) s_max = s_exp = s_cnt = 0u;
     load_window<true, false>(G, W);
     if (W.on)
         for (int i = threadIdx.x; i < 5 * W.nw; i += blockDim.x) W.sM[i] = 0u;
     __syncthreads();
-    unsigned big = 0u;  // largest |a_v| after the drift, as its bits (a NaN above all)
+    // largest |a_v| after the drift, as its bits (a NaN above all); sum of the
+    // biased exponents and number of the normal values
+    unsigned big = 0u, exps = 0u, cnt = 0u;
     for (long long q = base + 4ll * threadIdx.x; q < end; q += 4ll * blockDim.x) {
         const float4 x4 = *reinterpret_cast<const float4 *>(A.ax + q);
         const float4 y4 = *reinterpret_cast<const float4 *>(A.ay + q);
@@ -128,17 +137,31 @@ __device__ __forceinline__ void adj_kick_block(const KickArgs &A, const KickGeo 
                             fmaf(K.ddt, x4.w, u4.w), fmaf(K.ddt, y4.x, w4.x), fmaf(K.ddt, y4.y, w4.y),
                             fmaf(K.ddt, y4.z, w4.z), fmaf(K.ddt, y4.w, w4.w)};
 #pragma unroll
-        for (int k = 0; k < 8; ++k) big = max(big, __float_as_uint(m[k]) & 0x7FFFFFFFu);
+        for (int k = 0; k < 8; ++k) {
+            const unsigned bits = __float_as_uint(m[k]) & 0x7FFFFFFFu, ex = bits >> 23;
+            big = max(big, bits);
+            exps += ex;
+            cnt += min(ex, 1u);
+        }
     }
     big = __reduce_max_sync(0xffffffffu, big);
-    if ((threadIdx.x & 31) == 0) atomicMax(&s_max, big);
+    exps = __reduce_add_sync(0xffffffffu, exps);
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(&s_max, big);
+        atomicAdd(&s_exp, exps);
+        atomicAdd(&s_cnt, cnt);
+    }
     __syncthreads();
-    // mu < 2^e for e in [-94, 128]; scale = 2^(31 - e)
-    const float top = __uint_as_float(s_max) * fabsf(K.muc);
+    // the values summed in fixed point are below 2^e, e in [-94, 128]; scale = 2^(31 - e)
+    big = s_max;
+    if (s_cnt && big < 0x7F800000u) big = min(big, min(s_exp / s_cnt + KICK_SPAN + 1, 254u) << 23);
+    const float top = __uint_as_float(big) * fabsf(K.muc);
     const int e = (int)(__float_as_uint(top) >> 23) - 126;
     const bool fixed = W.on && e >= -94 && e <= 128;
     const float scale = __uint_as_float((unsigned)(158 - e) << 23);
     const float inv_scale = __uint_as_float((unsigned)(96 + e) << 23);
+    const float below = __uint_as_float((unsigned)(127 + e) << 23);  // 2^e
     const int nx = G.nx, ny = G.ny;
     for (long long q = base + 4ll * threadIdx.x; q < end; q += 4ll * blockDim.x) {
         const int4 c4 = *reinterpret_cast<const int4 *>(A.cell + q);
@@ -184,7 +207,7 @@ __device__ __forceinline__ void adj_kick_block(const KickArgs &A, const KickGeo 
                 e01 = make_float2(G.ex[w.i01], G.ey[w.i01]);
                 e11 = make_float2(G.ex[w.i11], G.ey[w.i11]);
             }
-            if (in && fixed) {
+            if (in && fixed && fmaxf(fabsf(mx), fabsf(my)) < below) {
                 unsigned *m0 = W.sM + 5 * l, *m1 = m0 + 5 * W.nwx;
                 add_fixed(m0, w00 * mx, scale);
                 add_fixed(m0 + 2, w00 * my, scale);
