@@ -88,12 +88,12 @@ struct PushArgs {
 // the tile of the block's first particle.  The deposit keeps per-cell CIC
 // moments in sM, five words per cell: one address for a particle's five
 // atomics (the rest is immediate offsets), and the odd stride puts
-// neighbouring cells on different banks.  sLo and sHi are the same area seen
-// as two node planes by the ensemble adjoint kick.  wcx is 0 where the block
-// has no window (!on), so that no cell lies in it.
+// neighbouring cells on different banks (the adjoint's kick keeps its sums
+// there, see kick_bytes).  wcx is 0 where the block has no window (!on), so that
+// no cell lies in it.
 struct Window {
     float2 *sE;
-    unsigned *sLo, *sHi, *sM;
+    unsigned *sM;
     int wx0, wy0, nwx, nw, nc;
     unsigned wcx, wcy;
     bool on;
@@ -105,9 +105,7 @@ __device__ __forceinline__ Window setup_window(const PushGeo &A, unsigned char *
     W.nwx = A.wcx + 1;
     W.nw = W.nwx * (A.wcy + 1);
     W.sE = reinterpret_cast<float2 *>(smem);
-    W.sLo = reinterpret_cast<unsigned *>(smem + (size_t)W.nw * sizeof(float2));
-    W.sHi = W.sLo + W.nw;
-    W.sM = W.sLo;
+    W.sM = reinterpret_cast<unsigned *>(smem + (size_t)W.nw * sizeof(float2));
     W.nc = A.wcx * A.wcy;
     W.on = anc >= 0;
     W.wcx = W.on ? A.wcx : 0;
@@ -257,125 +255,6 @@ __device__ __forceinline__ bool warp_group_sum(int key, unsigned &c, unsigned &f
     return head;
 }
 
-// Gather, push and deposit four consecutive particles held in registers, any
-// of which may be empty or corrupt: the general form, used where push_four is
-// not (quads with such slots, and AGG).
-// AGG: the lanes' main groups are summed across the warp (warp_group_sum)
-// before the deposit, so that a warp whose particles share a cell issues
-// one set of atomics instead of 32 conflicting ones; every lane of the warp
-// must then call this function together.  !MOVE: deposit the particles
-// where they are (no gather, no push, velocities not read).
-template <bool GATHER, bool DEPOSIT, bool AGG, bool MOVE = true>
-__device__ __forceinline__ void push_quad(const PushGeo &A, const Window &W, int (&cc)[4],
-                                          float (&xo)[4], float (&yo)[4], float (&xv)[4],
-                                          float (&yv)[4], float &ke, float &px, float &py,
-                                          bool &bad)
-{
-    const int nx = A.nx, ny = A.ny;
-    // register aggregate of the particles that share the first one's new cell
-    unsigned gcnt = 0u, gfx = 0u, gfy = 0u;
-    unsigned long long gxy = 0ull;
-    int gkey = -1, gdx = 0, gdy = 0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int c = cc[j];
-        if (c < 0) continue;  // empty slot
-        int cx = c & 0xFFFF, cy = c >> 16;
-        if (cx >= nx || cy >= ny) {  // corrupt cell: flag, leave untouched
-            bad = true;
-            atomicOr(&A.dev->err, (unsigned)PIC_DEVERR_CELL);
-            continue;
-        }
-        float ox = xo[j], oy = yo[j], vx = xv[j], vy = yv[j];
-        int dxl, dyl;  // window coordinates, advanced with the cell below
-        window_coords(A, W, cx, cy, dxl, dyl);
-        if (!MOVE) {
-        } else if (GATHER) {
-            const float gx = 1.f - ox, gy = 1.f - oy;
-            float2 e00, e10, e01, e11;
-            if ((unsigned)dxl < W.wcx && (unsigned)dyl < W.wcy) {
-                const int i = dyl * W.nwx + dxl;
-                e00 = W.sE[i];
-                e10 = W.sE[i + 1];
-                e01 = W.sE[i + W.nwx];
-                e11 = W.sE[i + W.nwx + 1];
-            } else {
-                const int cx1 = (cx + 1 == nx) ? 0 : cx + 1;
-                const int cy1 = (cy + 1 == ny) ? 0 : cy + 1;
-                const size_t i00 = (size_t)cy * nx + cx, i10 = (size_t)cy * nx + cx1;
-                const size_t i01 = (size_t)cy1 * nx + cx, i11 = (size_t)cy1 * nx + cx1;
-                e00 = make_float2(A.ex[i00], A.ey[i00]);
-                e10 = make_float2(A.ex[i10], A.ey[i10]);
-                e01 = make_float2(A.ex[i01], A.ey[i01]);
-                e11 = make_float2(A.ex[i11], A.ey[i11]);
-            }
-            const float Ex = gy * fmaf(gx, e00.x, ox * e10.x) + oy * fmaf(gx, e01.x, ox * e11.x);
-            const float Ey = gy * fmaf(gx, e00.y, ox * e10.y) + oy * fmaf(gx, e01.y, ox * e11.y);
-            const float vx0 = vx, vy0 = vy;
-            vx = fmaf(A.qm_dt, Ex, vx);
-            vy = fmaf(A.qm_dt, Ey, vy);
-            ke = fmaf(vx0, vx0, fmaf(vy0, vy0, fmaf(vx, vx, fmaf(vy, vy, ke))));
-            px += vx0 + vx;
-            py += vy0 + vy;
-        } else {
-            ke = fmaf(2.f * vx, vx, fmaf(2.f * vy, vy, ke));
-            px = fmaf(2.f, vx, px);
-            py = fmaf(2.f, vy, py);
-        }
-        if (MOVE) {
-            // drift in cell units; carry whole cells into the index (a
-            // non-finite velocity shows in the thread's kinetic-energy sum)
-            ox = fmaf(vx, A.dtdx, ox);
-            oy = fmaf(vy, A.dtdy, oy);
-            float sx = floorf(ox), sy = floorf(oy);
-            ox -= sx;
-            oy -= sy;
-            if (ox >= 1.f) { ox -= 1.f; sx += 1.f; }
-            if (oy >= 1.f) { oy -= 1.f; sy += 1.f; }
-            const int kx = (int)sx, ky = (int)sy;
-            cx += kx;
-            cy += ky;
-            dxl += kx;
-            dyl += ky;
-            if ((unsigned)cx >= (unsigned)nx) { cx %= nx; if (cx < 0) cx += nx; }
-            if ((unsigned)cy >= (unsigned)ny) { cy %= ny; if (cy < 0) cy += ny; }
-        }
-        const int cn = cx | (cy << 16);
-        if (MOVE && A.recount && cn != c) {  // a particle that changed cells
-            atomicAdd(A.recount + push_cell_key(cx, cy, A), 1u);
-            atomicSub(A.recount + push_cell_key(c & 0xFFFF, c >> 16, A), 1u);
-        }
-        cc[j] = cn;
-        xo[j] = ox;
-        yo[j] = oy;
-        xv[j] = vx;
-        yv[j] = vy;
-        if (DEPOSIT) {
-            const unsigned fx = offset_fixed(ox), fy = offset_fixed(oy);
-            const unsigned long long fxy = (unsigned long long)fx * fy;
-            if (gkey < 0) {
-                gkey = cn;
-                gdx = dxl;
-                gdy = dyl;
-            }
-            if (cn == gkey) {
-                ++gcnt;
-                gfx += fx;
-                gfy += fy;
-                gxy += fxy;
-            } else {
-                deposit_group(A, W, cx, cy, dxl, dyl, 1u, fx, fy, fxy);
-            }
-        }
-    }
-    if (DEPOSIT && AGG) {
-        if (warp_group_sum(gcnt ? gkey : -1, gcnt, gfx, gfy, gxy) && gcnt)
-            deposit_group(A, W, gkey & 0xFFFF, gkey >> 16, gdx, gdy, gcnt, gfx, gfy, gxy);
-    } else if (DEPOSIT && gcnt) {
-        deposit_group(A, W, gkey & 0xFFFF, gkey >> 16, gdx, gdy, gcnt, gfx, gfy, gxy);
-    }
-}
-
 // v mod n for a cell coordinate that left [0, n) (0 <= result < n): two
 // float quotients, each off by a few units at most, then one correction.
 __device__ __forceinline__ int wrap_cell(int v, int n)
@@ -471,7 +350,7 @@ __device__ __forceinline__ void push_one(const PushGeo &A, const Window &W, int 
 
 // Four particles with their cells on the grid, each deposited by itself: on
 // row-sorted particles a quad rarely shares a cell, and collecting those that
-// do in registers first, as push_quad does, costs divergent code on every
+// do in registers first, as push_grouped does, costs divergent code on every
 // quad and registers that spill.  2048^2 x 32, sort every 20: 1.094 -> 1.018 ms
 // per step (chunk 16384; with the slow slots out of line and one address per
 // quad and per deposit); collected per quad as before 1.077, with spills up to
@@ -522,6 +401,50 @@ __device__ __forceinline__ void push_slots(const PushGeo &A, const Window &W, in
         cc[j] = c[j];
         xo[j] = p[0][j], yo[j] = p[1][j], xv[j] = p[2][j], yv[j] = p[3][j];
     }
+}
+
+// Four slots, any of them empty or corrupt, for AGG: those that share the first
+// one's new cell are collected in registers and these groups summed across
+// the warp (warp_group_sum) before the deposit, so that a warp whose particles
+// share a cell issues one set of atomics instead of 32 conflicting ones.  Every
+// lane of the warp calls it together.
+template <bool GATHER>
+__device__ __forceinline__ void push_grouped(const PushGeo &A, const Window &W, int (&cc)[4],
+                                             float (&xo)[4], float (&yo)[4], float (&xv)[4],
+                                             float (&yv)[4], float &ke, float &px, float &py, bool &bad)
+{
+    unsigned gcnt = 0u, gfx = 0u, gfy = 0u;
+    unsigned long long gxy = 0ull;
+    int gkey = -1, gdx = 0, gdy = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if (cc[j] < 0) continue;  // empty slot
+        if ((cc[j] & 0xFFFF) >= A.nx || (cc[j] >> 16) >= A.ny) {  // corrupt: flag, leave untouched
+            bad = true;
+            atomicOr(&A.dev->err, (unsigned)PIC_DEVERR_CELL);
+            continue;
+        }
+        push_one<GATHER, true, true, false>(A, W, cc[j], xo[j], yo[j], xv[j], yv[j], ke, px, py,
+                                            [&](int cx, int cy, int dxl, int dyl, unsigned fx, unsigned fy) {
+            const unsigned long long fxy = (unsigned long long)fx * fy;
+            const int cn = cx | (cy << 16);
+            if (gkey < 0) {
+                gkey = cn;
+                gdx = dxl;
+                gdy = dyl;
+            }
+            if (cn == gkey) {
+                ++gcnt;
+                gfx += fx;
+                gfy += fy;
+                gxy += fxy;
+            } else {
+                deposit_group(A, W, cx, cy, dxl, dyl, 1u, fx, fy, fxy);
+            }
+        });
+    }
+    if (warp_group_sum(gcnt ? gkey : -1, gcnt, gfx, gfy, gxy) && gcnt)
+        deposit_group(A, W, gkey & 0xFFFF, gkey >> 16, gdx, gdy, gcnt, gfx, gfy, gxy);
 }
 
 // byte offset `o` into one field's array, whose block starts at the uniform
@@ -658,8 +581,9 @@ __device__ __forceinline__ void push_block(const PushArgs &A, const PushGeo &G, 
                 yv[0] = v4.x, yv[1] = v4.y, yv[2] = v4.z, yv[3] = v4.w;
             }
         }
-        if (AGG) {
-            push_quad<GATHER, DEPOSIT, AGG, MOVE>(G, W, cc, xo, yo, xv, yv, ke, px, py, bad);
+        if constexpr (AGG) {
+            static_assert(DEPOSIT && MOVE && !LATE, "push_grouped");
+            push_grouped<GATHER>(G, W, cc, xo, yo, xv, yv, ke, px, py, bad);
         } else {
             bool whole = true;  // four cells on the grid (-1, an empty slot, is off it)
 #pragma unroll
