@@ -367,7 +367,9 @@ bool plan(int nx, int ny, MixArgs &G, size_t (&smem)[3])
 {
     memset(&G, 0, sizeof G);
     if (nx < 16 || ny < 16 || !plan_dim(nx, G.dx) || !plan_dim(ny, G.dy)) return false;
-    // at most four blocks per SM (two: 700x640 129 us a step, four: 122)
+    // at most four blocks per SM (two: 700x640 129 us a step, four: 122); on 152
+    // SMs that is one row pair and one column a block for every side taken here,
+    // and one row back or two
     const int blocks = 4 * device_sms();
     auto share = [&](int items) { return (items + blocks - 1) / blocks; };
     G.np = share((ny + 1) / 2);
