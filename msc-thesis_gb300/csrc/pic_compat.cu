@@ -27,6 +27,7 @@
 #include <cmath>
 #include <vector>
 
+#include "pic_div_dev.cuh"
 #include "pic_internal.cuh"
 
 namespace pic {
@@ -51,19 +52,6 @@ struct CompatDev {
     const double2 *twx, *twy;  // exp(-2 pi i k / n), n entries each
     double2 *kmode;          // -k^2 and its reciprocal (0, 0 for the zero mode), laid out as fout
 };
-
-// a / b for a divisor known in advance, y = 1/b rounded to nearest: one
-// product, its exact residual and one correction (P. Markstein, "Computation
-// of elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
-// Dev. 34, 1990; N. Brisebarre, J.-M. Muller and S. K. Raina, IEEE Trans.
-// Computers 53(8), 2004).  Three operations on the FP64 pipe, which issues
-// one warp instruction per 16 cycles and SM and bounds the particle pass; the
-// general division takes several times as many.
-__device__ __forceinline__ double div_known(double a, double b, double y)
-{
-    const double q = __dmul_rn(a, y);
-    return __fma_rn(__fma_rn(-b, q, a), y, q);
-}
 
 // (int)(x / d) and its value as a double; positions in range take the
 // integer from the low word of q + 2^52 rounded toward zero
