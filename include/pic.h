@@ -274,7 +274,7 @@ typedef struct pic_dsmc_params {
     double weight;            /* F_N: real atoms per macro-particle             */
     double depth;             /* cell depth for the 2-D cell volume, m          */
     double sigma_g_max0;      /* initial (sigma g)_max per cell, m^3/s          */
-    int every;                /* collide every `every` steps, dt_c = every*dt (0: 1) */
+    int every;                /* not used: a pass follows every step, dt_c = dt     */
     unsigned long long seed;
 } pic_dsmc_params;
 pic_status pic_set_dsmc(pic_handle *h, const pic_dsmc_params *p);

@@ -91,7 +91,8 @@ class MccParams(C.Structure):
 
 class DsmcParams(C.Structure):
     _fields_ = [("species", C.c_int), ("diameter", C.c_double), ("weight", C.c_double),
-                ("depth", C.c_double), ("sigma_g_max0", C.c_double), ("seed", C.c_ulonglong)]
+                ("depth", C.c_double), ("sigma_g_max0", C.c_double), ("every", C.c_int),
+                ("seed", C.c_ulonglong)]
 
 
 class TuneResult(C.Structure):
@@ -425,7 +426,7 @@ class Handle:
         self._c("pic_set_mcc", C.byref(p))
 
     def set_dsmc(self, species, diameter, weight, depth, sigma_g_max0, seed=0):
-        p = DsmcParams(species, diameter, weight, depth, sigma_g_max0, seed)
+        p = DsmcParams(species, diameter, weight, depth, sigma_g_max0, 0, seed)
         self._c("pic_set_dsmc", C.byref(p))
 
     def save(self, path):

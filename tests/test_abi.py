@@ -85,3 +85,26 @@ def test_no_device_is_reported(monkeypatch):
     with pytest.raises(P.PicError) as e:
         P.Handle(c)
     assert e.value.status == 9
+
+
+@pytest.mark.parametrize("struct,ctype", [
+    ("pic_ref_params", P.RefParams), ("pic_species_desc", P.SpeciesDesc), ("pic_config", P.Config),
+    ("pic_init_spec", P.InitSpec), ("pic_diag", P.Diag), ("pic_mcc_params", P.MccParams),
+    ("pic_dsmc_params", P.DsmcParams), ("pic_tune_result", P.TuneResult),
+    ("pic_adjoint_result", P.AdjointResult), ("pic_particles_view", P.ParticlesView)])
+def test_binding_structures_are_laid_out_as_the_header_s(struct, ctype, tmp_path):
+    """Every field of the C structure, in order, at the offset the binding gives it."""
+    import subprocess
+
+    src = re.sub(r"/\*.*?\*/", "", open(os.path.join(ROOT, "include", "pic.h")).read(), flags=re.S)
+    body = re.search(r"typedef struct %s \{(.*?)\} %s;" % (struct, struct), src, re.S)[1]
+    fields = [re.sub(r"\[.*", "", f.strip().lstrip("*").strip()) for d in body.split(";") if d.strip()
+              for f in re.sub(r"^\s*(const\s+)?(unsigned\s+)?(long\s+long|\w+)\s", "", d.strip()).split(",")]
+    assert fields == [f[0] for f in ctype._fields_]
+    c = tmp_path / "layout.c"
+    c.write_text('#include <stddef.h>\n#include <stdio.h>\n#include "pic.h"\nint main(void) {\n' +
+                 "".join(f'printf("%zu ", offsetof({struct}, {f}));\n' for f in fields) +
+                 f'printf("%zu", sizeof({struct}));\nreturn 0;\n}}\n')
+    subprocess.run(["gcc", "-I" + os.path.join(ROOT, "include"), str(c), "-o", str(tmp_path / "layout")], check=True)
+    got = [int(x) for x in subprocess.run([str(tmp_path / "layout")], capture_output=True, check=True).stdout.split()]
+    assert got == [getattr(ctype, f).offset for f in fields] + [C.sizeof(ctype)]
