@@ -25,9 +25,8 @@
 #include <algorithm>
 #include <condition_variable>
 #include <cstring>
-#include <deque>
+#include <exception>
 #include <mutex>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -304,22 +303,26 @@ pic_status adj_plans(pic_ensemble *E)
 {
     if (!E->fork) PIC_CUDA(cudaEventCreateWithFlags(&E->fork, cudaEventDisableTiming));
     for (auto &G : E->groups) {
-        if (G.r2c2) continue;
+        // (each on its own: a call that failed halfway goes on from there)
         if (&G != &E->groups[0]) {
-            PIC_CUDA(cudaStreamCreateWithFlags(&G.side, cudaStreamNonBlocking));
-            PIC_CUDA(cudaEventCreateWithFlags(&G.done, cudaEventDisableTiming));
+            if (!G.side) PIC_CUDA(cudaStreamCreateWithFlags(&G.side, cudaStreamNonBlocking));
+            if (!G.done) PIC_CUDA(cudaEventCreateWithFlags(&G.done, cudaEventDisableTiming));
         }
         cudaStream_t st = G.side ? G.side : E->stream;
         const EnsRun &R = E->runs[G.first];
         int dims[2] = {G.ny, G.nx}, real_emb[2] = {G.ny, G.nx}, cplx_emb[2] = {G.ny, R.nh};
         // gx, gy of every run (stride ncp) -> gx^, gy^ (stride nk)
-        PIC_CUFFT(cufftPlanMany(&G.r2c2, 2, dims, real_emb, 1, (int)R.ncp, cplx_emb, 1, (int)R.nk,
-                                CUFFT_R2C, 2 * G.count));
-        PIC_CUFFT(cufftSetStream(G.r2c2, st));
+        if (!G.r2c2) {
+            PIC_CUFFT(cufftPlanMany(&G.r2c2, 2, dims, real_emb, 1, (int)R.ncp, cplx_emb, 1, (int)R.nk,
+                                    CUFFT_R2C, 2 * G.count));
+            PIC_CUFFT(cufftSetStream(G.r2c2, st));
+        }
         // psi^ (stride 2 nk) -> psi (stride ncp)
-        PIC_CUFFT(cufftPlanMany(&G.c2r1, 2, dims, cplx_emb, 1, (int)(2 * R.nk), real_emb, 1,
-                                (int)R.ncp, CUFFT_C2R, G.count));
-        PIC_CUFFT(cufftSetStream(G.c2r1, st));
+        if (!G.c2r1) {
+            PIC_CUFFT(cufftPlanMany(&G.c2r1, 2, dims, cplx_emb, 1, (int)(2 * R.nk), real_emb, 1,
+                                    (int)R.ncp, CUFFT_C2R, G.count));
+            PIC_CUFFT(cufftSetStream(G.c2r1, st));
+        }
     }
     return PIC_OK;
 }
@@ -353,12 +356,10 @@ public:
     {
         const unsigned cores = std::thread::hardware_concurrency();
         int n = bytes < THREADED ? 0 : (int)std::min(THREADS, cores > 1 ? cores - 1 : 0u);
-        for (; n > 0; --n) {
-            try {
-                workers.emplace_back([this] { work(); });
-            } catch (const std::system_error &) {
-                break;
-            }
+        try {
+            workers.reserve(n);
+            for (; n > 0; --n) workers.emplace_back([this] { work(); });
+        } catch (const std::exception &) {  // no thread, or no memory for one
         }
     }
     ~Export() { close(); }
@@ -379,7 +380,7 @@ public:
             PIC_CUDA(cudaMemcpyAsync(at(slot), src + k, m * sizeof(double), cudaMemcpyDeviceToHost, E->stream));
             PIC_CUDA(cudaEventRecord(E->bounced[slot], E->stream));
             std::lock_guard<std::mutex> lock(mu);
-            queue.push_back(Part{slot, dst + k, m * sizeof(double)});
+            queue[(head + queued++) % SLOTS] = Part{slot, dst + k, m * sizeof(double)};
             changed.notify_one();
         }
         return PIC_OK;
@@ -404,8 +405,9 @@ private:
     // one part out of its slot, the lock released meanwhile
     void copy_one(std::unique_lock<std::mutex> &lock)
     {
-        const Part p = queue.front();
-        queue.pop_front();
+        const Part p = queue[head];
+        head = (head + 1) % SLOTS;
+        --queued;
         lock.unlock();
         const cudaError_t e = cudaEventSynchronize(E->bounced[p.slot]);
         if (e == cudaSuccess) memcpy(p.dst, at(p.slot), p.bytes);
@@ -419,8 +421,8 @@ private:
         cudaSetDevice(E->device);
         std::unique_lock<std::mutex> lock(mu);
         for (;;) {
-            changed.wait(lock, [this] { return closing || !queue.empty(); });
-            if (queue.empty()) return;
+            changed.wait(lock, [this] { return closing || queued; });
+            if (!queued) return;
             copy_one(lock);
         }
     }
@@ -443,7 +445,7 @@ private:
         std::unique_lock<std::mutex> lock(mu);
         closing = true;
         changed.notify_all();
-        while (!queue.empty()) copy_one(lock);
+        while (queued) copy_one(lock);
         lock.unlock();
         for (std::thread &t : workers) t.join();
         workers.clear();
@@ -452,7 +454,8 @@ private:
     pic_ensemble *E;
     std::mutex mu;
     std::condition_variable changed, freed;
-    std::deque<Part> queue;
+    Part queue[SLOTS];  // a ring: a part holds a slot, so there are no more
+    int head = 0, queued = 0;
     unsigned busy = 0;  // slots in use
     bool closing = false;
     cudaError_t failed = cudaSuccess;
