@@ -313,16 +313,20 @@ pic_status adj_plans(pic_ensemble *E)
         int dims[2] = {G.ny, G.nx}, real_emb[2] = {G.ny, G.nx}, cplx_emb[2] = {G.ny, R.nh};
         // gx, gy of every run (stride ncp) -> gx^, gy^ (stride nk)
         if (!G.r2c2) {
-            PIC_CUFFT(cufftPlanMany(&G.r2c2, 2, dims, real_emb, 1, (int)R.ncp, cplx_emb, 1, (int)R.nk,
-                                    CUFFT_R2C, 2 * G.count));
-            PIC_CUFFT(cufftSetStream(G.r2c2, st));
+            cufftHandle p = 0;
+            PIC_CUFFT(cufftPlanMany(&p, 2, dims, real_emb, 1, (int)R.ncp, cplx_emb, 1, (int)R.nk, CUFFT_R2C,
+                                    2 * G.count));
+            G.r2c2 = p;
         }
         // psi^ (stride 2 nk) -> psi (stride ncp)
         if (!G.c2r1) {
-            PIC_CUFFT(cufftPlanMany(&G.c2r1, 2, dims, cplx_emb, 1, (int)(2 * R.nk), real_emb, 1,
-                                    (int)R.ncp, CUFFT_C2R, G.count));
-            PIC_CUFFT(cufftSetStream(G.c2r1, st));
+            cufftHandle p = 0;
+            PIC_CUFFT(cufftPlanMany(&p, 2, dims, cplx_emb, 1, (int)(2 * R.nk), real_emb, 1, (int)R.ncp,
+                                    CUFFT_C2R, G.count));
+            G.c2r1 = p;
         }
+        PIC_CUFFT(cufftSetStream(G.r2c2, st));
+        PIC_CUFFT(cufftSetStream(G.c2r1, st));
     }
     return PIC_OK;
 }
