@@ -34,6 +34,8 @@
 // sums stay at most 2^31 for chunks of at most 32768 particles.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "pic_push_dev.cuh"
 
 namespace pic {
@@ -96,12 +98,16 @@ static size_t push_smem(const Geometry &g)
     return window_bytes(g.wcx, g.wcy) + 32;
 }
 
-// set on every launch: the attribute belongs to the current device, and a
-// process may drive several
+// Set on every launch: the attribute belongs to the current device, and a
+// process may drive several.  Always to the same limit, not to `bytes`: another
+// thread's handle launches the same kernel with another window between this
+// call and the launch.
 pic_status allow_dynamic_smem(const void *kernel, size_t bytes)
 {
+    constexpr size_t LIMIT = 224 * 1024;  // of 227 KB; the rest for static shared memory
     if (bytes > 48 * 1024)
-        PIC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        PIC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)std::max(bytes, LIMIT)));
     return PIC_OK;
 }
 

@@ -144,3 +144,40 @@ def test_default_blocks_of_large_runs_hold_their_tile(nx, ny, ppc):
             h.init_particles(0, P.init_spec(n, vth=(0.1, 0.1, 0.0), seed=4))
             order.append(h.get_particles_raw(0)["cell"])
     np.testing.assert_array_equal(*order)
+
+
+def test_handles_of_two_threads_launch_with_windows_of_different_size():
+    """One handle per host thread: pushes whose windows take 52 and 85 KB of
+    shared memory, launched one by one from two threads at a time."""
+    import threading
+
+    n = NX * NX * 16
+    w = L * L / n
+    p = load(n, 12)
+    results, errors = {}, []
+
+    def work(halo, steps):
+        try:
+            with P.Handle(P.config(NX, NX, L, L, DT, [P.species(n, -w, w, -1)], chunk=4096, tile_w=16, tile_h=16,
+                                   halo=halo)) as h:
+                h.set_particles(0, *p)
+                h.prime_leapfrog()
+                for _ in range(steps):
+                    h.gather_push(True)
+                    h.poisson()
+                results[halo, steps] = h.get_particles(0), h.rho_fixed()
+        except P.PicError as e:
+            errors.append(e)
+
+    for halo in (10, 16):
+        work(halo, 1500)
+    alone = dict(results)
+    for _ in range(3):
+        threads = [threading.Thread(target=work, args=(halo, 1500)) for halo in (10, 16, 10, 16)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert not errors, errors[0]
+        for k in alone:
+            same(results[k], alone[k])
