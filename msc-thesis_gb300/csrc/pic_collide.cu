@@ -509,8 +509,9 @@ pic_status launch_mcc(pic_handle *h)
     A.dev = h->dev;
     mcc_prepare_kernel<<<1, 1, 0, h->stream>>>(h->dev, M.e);
     PIC_CUDA(cudaGetLastError());
-    mcc_kernel<<<grid_for(E.cap, MCC_CHUNK), MCC_THREADS,
-                 4 * M.ntab * sizeof(float) + MCC_CHUNK * sizeof(int), h->stream>>>(A);
+    const size_t smem = 4 * M.ntab * sizeof(float) + MCC_CHUNK * sizeof(int);
+    PIC_TRY(allow_dynamic_smem((const void *)mcc_kernel, smem));
+    mcc_kernel<<<grid_for(E.cap, MCC_CHUNK), MCC_THREADS, smem, h->stream>>>(A);
     PIC_CUDA(cudaGetLastError());
     return PIC_OK;
 }

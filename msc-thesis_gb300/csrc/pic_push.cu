@@ -105,7 +105,7 @@ static size_t push_smem(const Geometry &g)
 pic_status allow_dynamic_smem(const void *kernel, size_t bytes)
 {
     constexpr size_t LIMIT = 224 * 1024;  // of 227 KB; the rest for static shared memory
-    if (bytes > 48 * 1024)
+    if (bytes > 40 * 1024)  // of 48 KB by default, static shared memory included
         PIC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)std::max(bytes, LIMIT)));
     return PIC_OK;

@@ -199,3 +199,18 @@ def test_newborn_particles_are_pushed_beyond_the_loaded_blocks(chunk):
                 old = r["pid"] < d.n[0]  # not those of this step
                 place[k][r["pid"][old]] = np.stack([r["cell"], r["ox"], r["oy"]], 1)[old]
             assert (place["a"] != place["b"]).any(1).all()
+
+
+@pytest.mark.parametrize("ntab", [2, 2560, 4096])
+def test_cross_section_tables_of_every_accepted_length(ntab):
+    """Tables of up to 4096 points, in shared memory beyond the default limit."""
+    from collide_util import NG, TN_EV, mcc_cross_sections
+
+    n, dt = 20_000, 1e-10
+    _, sel, sexc, sion = mcc_cross_sections(ntab)
+    with mcc_handle(n, 20.0, dt) as h:
+        h.set_mcc(0, 1, NG, TN_EV, ME, MI, E_CH, 0.01, 1000.0, sel, sexc, sion, 11.5, 15.8, 3)
+        h.collide(P.COLLIDE_MCC)
+        h.synchronize()
+        c = h.collision_counts()
+        assert h.diagnostics().error_flags == 0 and c[0] > 0
