@@ -237,8 +237,8 @@ struct pic_handle {
     // (rhohat and ehat then hold their column-major intermediates)
     bool spectral = false;
     // other sides that are products of 2, 3, 5 and 7 (pic_spectral_mixed.cu);
-    // library_solve: within a call that hands its results back in 64 bits
-    // (LibrarySolve), whose fields stay those of cuFFT to the last bit
+    // library_solve: within a call whose fields stay those of cuFFT to the last
+    // bit (LibrarySolve)
     bool mixed = false, library_solve = false;
     float2 *tw = nullptr;  // twiddles: nx entries, then ny
     // sort
@@ -306,8 +306,11 @@ pic_status spectral_twiddles(int nx, int ny, float2 **tw);  // cudaMalloc'd tabl
 bool mixed_wanted(int nx, int ny);
 pic_status mixed_twiddles(int nx, int ny, float2 **tw);
 pic_status launch_mixed(pic_handle *h, int adv);
-// pic_run_host and the adjoint: their arrays are doubles, and where the flow is
-// chaotic an adjoint's gradients follow the last bit of the forward fields
+// pic_run_host and the adjoint on those sides: they solved through cuFFT before
+// there were other kernels, and keep its bits.  The adjoint's gradients follow
+// the last bit of the forward fields where the flow is chaotic (a run's were
+// 1.1e-5 apart); the one-call run keeps its results for callers that compare
+// its doubles with earlier ones (its particles are single precision in between).
 struct LibrarySolve {
     pic_handle *h;
     explicit LibrarySolve(pic_handle *h) : h(h) { h->library_solve = true; }

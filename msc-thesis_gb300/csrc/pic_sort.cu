@@ -262,8 +262,9 @@ void sort_sizes_for(double density, int *wk, int *hb)
     *hb = b;
 }
 
-// The DSMC species is sorted by cell (its pass pairs particles per cell);
-// every other species by tile row (keys 0 .. ncell / tw - 1 of the same space).
+// The DSMC species is sorted by cell (the histogram gives its pass the counts
+// per cell that its pushes then keep, and a cell's particles lie together when
+// the pass lists them); every other species by tile row (keys 0 .. ncell / tw - 1 of the same space).
 static int sort_rows(const pic_handle *h, int s) { return h->dsmc.on && s == h->dsmc.s ? 0 : 1; }
 
 // Keys of an import: as the periodic sort's.  (Sorted by cell, a species that
