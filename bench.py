@@ -345,10 +345,11 @@ def ens_fp64_check(P, cfgs, specs, nsteps, max_particles=8_000_000):
 
 # Settings that pic_ensemble_autotune and pic_autotune chose on a GB300 for
 # the 64 two-stream runs (bench.py --workload ensemble, which tunes afresh):
-# the ensemble's push chunk and sort cadence, and per (grid side, particles
+# the ensemble's push chunk (0: these loads set tiles and blocks themselves;
+# with 4096 and 8192 a step takes the same 4.93 ms) and sort cadence, and per (grid side, particles
 # per cell) a single handle's chunk, tile width, tile height and cadence.
 # The default line's ensemble record uses them and so needs no tuning runs.
-ENSEMBLE_TUNED = (4096, 20)
+ENSEMBLE_TUNED = (0, 20)
 PLAIN_TUNED = {
     (512, 256): (16384, 16, 4, 20), (512, 128): (8192, 16, 4, 10), (512, 64): (8192, 16, 8, 10),
     (512, 32): (4096, 16, 8, 10), (512, 16): (4096, 16, 16, 10), (256, 256): (8192, 16, 2, 20),
